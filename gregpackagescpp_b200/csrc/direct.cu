@@ -17,6 +17,8 @@
 #include <mutex>
 #include <tuple>
 
+#include "direct_epilogue.cuh"
+#include "direct_mixed.cuh"
 #include "gtd_internal.cuh"
 #include "gtd_math.cuh"
 
@@ -150,75 +152,12 @@ __global__ void __launch_bounds__(kThreads) force_f64_kernel(ForceKArgs a) {
 // fold provably holds no pair with r^2 < near2 |X_i|^2.  With near2 = (2 / (K - 1))^2 every pair
 // on the fast path keeps its coordinate error below K 2^-24 relative.
 // -------------------------------------------------------------------------------------------
-__device__ __forceinline__ float rsqrt_approx(float x) {
-    float y;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-
-__device__ __forceinline__ void kahan_add(double &sum, double &comp, double v) {
-    const double y = v - comp;
-    const double t = sum + y;
-    comp = (t - sum) - y;
-    sum = t;
-}
-
-// FP64 Kahan accumulators of the I i-bodies of a thread: in registers, or (SMEM) in shared memory,
-// which they only touch once per fold; the latter frees 12 registers per i-body for occupancy.
-template <int I, bool SMEM>
-struct KahanAcc;
-
-template <int I>
-struct KahanAcc<I, false> {
-    double s[3][I], c[3][I];
-    __device__ __forceinline__ void init(int) {
-#pragma unroll
-        for (int d = 0; d < 3; ++d)
-#pragma unroll
-            for (int k = 0; k < I; ++k) s[d][k] = c[d][k] = 0.0;
-    }
-    __device__ __forceinline__ void add(int d, int k, double v) { kahan_add(s[d][k], c[d][k], v); }
-    __device__ __forceinline__ double result(int d, int k) const { return s[d][k] - c[d][k]; }
-};
-
-template <int I>
-struct KahanAcc<I, true> {
-    double (*sm)[I][kThreads];  // [6][I][kThreads]: sums x y z, compensations x y z
-    int t;
-    __device__ __forceinline__ void init(int tid) {
-        t = tid;
-#pragma unroll
-        for (int d = 0; d < 6; ++d)
-#pragma unroll
-            for (int k = 0; k < I; ++k) sm[d][k][t] = 0.0;
-    }
-    __device__ __forceinline__ void add(int d, int k, double v) {
-        double s = sm[d][k][t], c = sm[3 + d][k][t];
-        kahan_add(s, c, v);
-        sm[d][k][t] = s;
-        sm[3 + d][k][t] = c;
-    }
-    __device__ __forceinline__ double result(int d, int k) const { return sm[d][k][t] - sm[3 + d][k][t]; }
-};
-
 // The staged j-tile: FP32 coordinates relative to the row centre (hi), their FP32 remainders (lo,
 // read only on the precise path), G m, and the bounding box of each warp's 32 staged bodies.
 struct MixedTile {
     const float *x, *y, *z, *m, *lx, *ly, *lz;
     const float *box;  // [kThreads / 32][6]: lo xyz, hi xyz
 };
-
-// Order-preserving map of a float onto an unsigned int, so that warp minima and maxima of floats
-// are single REDUX operations (__reduce_min_sync / __reduce_max_sync).
-__device__ __forceinline__ unsigned f2key(float f) {
-    const unsigned b = __float_as_uint(f);
-    return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
-}
-__device__ __forceinline__ float key2f(unsigned k) {
-    return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k);
-}
-__device__ __forceinline__ float warp_minf(float v) { return key2f(__reduce_min_sync(0xffffffffu, f2key(v))); }
-__device__ __forceinline__ float warp_maxf(float v) { return key2f(__reduce_max_sync(0xffffffffu, f2key(v))); }
 
 // The loop over j-pairs [u0, u0 + LEN) of a staged tile.  kPrecise: the coordinate differences are
 // taken from the hi/lo splits, dx = (hi_j - hi_i) + (lo_j - lo_i), which carries only the rounding
@@ -322,44 +261,6 @@ __device__ __forceinline__ void mixed_tile(const MixedTile &T, const float2 (&nx
             acc.add(1, k, (double)fy[k].x + (double)fy[k].y);
             acc.add(2, k, (double)fz[k].x + (double)fz[k].y);
         }
-    }
-}
-
-// One staged body: FP32 hi part of x - c, its FP32 remainder lo, and G m.  Padding bodies are far
-// away and massless, so their terms are exactly 0 on both paths.
-__device__ __forceinline__ void stage_body(bool have, const double4 &q, const double3 &c, double G, int slot,
-                                           float *hx, float *hy, float *hz, float *hm, float *lx, float *ly,
-                                           float *lz) {
-    if (have) {
-        const double ex = q.x - c.x, ey = q.y - c.y, ez = q.z - c.z;
-        const float fx = (float)ex, fy = (float)ey, fz = (float)ez;
-        hx[slot] = fx;
-        hy[slot] = fy;
-        hz[slot] = fz;
-        lx[slot] = (float)(ex - (double)fx);
-        ly[slot] = (float)(ey - (double)fy);
-        lz[slot] = (float)(ez - (double)fz);
-        hm[slot] = (float)(G * q.w);
-    } else {
-        const float kFar = 1e30f;
-        hx[slot] = hy[slot] = hz[slot] = kFar;
-        lx[slot] = ly[slot] = lz[slot] = 0.f;
-        hm[slot] = 0.f;
-    }
-}
-
-// Bounding box of the 32 bodies a warp just staged (padding bodies left out), written by lane 0 to
-// box[warp][6] of the buffer.  Every lane of the warp calls it.
-__device__ __forceinline__ void stage_box(bool have, const float *hx, const float *hy, const float *hz, int slot,
-                                          float *box) {
-    const float kInf = __int_as_float(0x7f800000);
-    const float x = hx[slot], y = hy[slot], z = hz[slot];
-    const float lx = warp_minf(have ? x : kInf), ly = warp_minf(have ? y : kInf), lz = warp_minf(have ? z : kInf);
-    const float ux = warp_maxf(have ? x : -kInf), uy = warp_maxf(have ? y : -kInf), uz = warp_maxf(have ? z : -kInf);
-    if ((threadIdx.x & 31) == 0) {
-        float *b = box + (threadIdx.x >> 5) * 6;
-        b[0] = lx; b[1] = ly; b[2] = lz;
-        b[3] = ux; b[4] = uy; b[5] = uz;
     }
 }
 
@@ -522,32 +423,41 @@ __global__ void __launch_bounds__(kThreads, MINB) force_mixed_kernel(ForceKArgs 
 // Plan and launch
 // -------------------------------------------------------------------------------------------
 // Kernel variants: i-bodies per thread (I) and, for the mixed kernel, the j-bodies summed in FP32
-// between FP64 folds (FOLD).  Index 0 of each table is the default; gtd_system_autotune_direct
-// times them all on the caller's bodies and keeps the fastest.
+// between FP64 folds (FOLD).  gtd_system_autotune_direct times them all on the caller's bodies and
+// keeps the fastest.
 struct VariantInfo {
     int i, fold;
     int bj = kThreads;  // j-bodies per work unit
+    int sym = -1;       // unordered-pair kernel (direct_sym.cu), or -1 for the ordered-pair kernels here
 };
 // mixed: {I, FOLD}; the launch bound (blocks per SM) and where the Kahan sums live are in with_mixed
 static const VariantInfo kMixedVariants[] = {{2, 64}, {4, 128}, {2, 128}, {2, 128}, {1, 64},
-                                             {4, 64}, {2, 64},  {2, 64},  {4, 128}};
-static const VariantInfo kF64Variants[] = {{2, 0}, {1, 0}, {4, 0}, {1, 0, 64}, {1, 0, 32}};
+                                             {4, 64}, {2, 64},  {2, 64},  {4, 128},
+                                             {4, 128, 128, 0}, {4, 64, 64, 1}};
+static const VariantInfo kF64Variants[] = {{2, 0}, {1, 0}, {4, 0}, {1, 0, 64}, {1, 0, 32},
+                                           {4, 0, 64, 0}, {4, 0, 128, 1}};
 constexpr int kNumMixed = sizeof(kMixedVariants) / sizeof(kMixedVariants[0]);
 constexpr int kNumF64 = sizeof(kF64Variants) / sizeof(kF64Variants[0]);
 
 int variant_count(int precision) { return precision == GTD_PREC_MIXED ? kNumMixed : kNumF64; }
 
-// Variant for a handle nobody tuned.  From N ~ 32768 up the mixed kernel is fastest with 4 i-bodies
-// per thread at 1 CTA/SM (<4,128,1,regs,U4>, variant 8: 27.4 ms against 29.1 ms for variant 0 at
-// N = 262144 on B200); below that the 2-per-thread variants keep more CTAs busy.  Small FP64
-// systems take the 32-wide work units so that every SM has work; up to N = 32768 one i-body per
-// thread (0.37 against 0.41 ms per force at N = 16384), above that four (4.50 against 4.64 ms at
-// N = 65536).
+// Variant for a handle nobody tuned: the unordered-pair kernels (direct_sym.cu), per step on B200
+//   mixed   N = 8192 65 us (ordered pairs 75), 16384 162 (192), 65536 1.59 ms (2.32), 262144 21.8 ms (29.3)
+//   FP64    N = 4500 35 us (39), 8192 68 (92), 16384 212 (295), 65536 2.95 ms (4.33)
+// From N = 32768 the mixed kernel folds its FP32 sums half as often: 3 % faster, and its rounding
+// (RMS 3.8e-8 of a body's acceleration at N = 262144 against 3.2e-8) is still that of the ordered
+// kernel's fold of 128 (4.0e-8).  FP64 systems up to kFusedMaxN bodies take the fused kernel instead.
 int default_variant(int precision, int64_t n) {
-    if (precision == GTD_PREC_MIXED) return n >= 32768 ? 8 : 0;
-    if (n <= 4096) return 4;  // FP64: 32-wide units up to N = 4096 (at least 512 units on 148 SMs)
-    return n <= 32768 ? 1 : 2;
+    if (precision == GTD_PREC_MIXED) return n >= 32768 ? 9 : 10;
+    return n <= 32768 ? 5 : 6;
 }
+
+// Variant of gtd_direct_accelerations_noalloc: as for a handle, with the finer folds at every size.
+int noalloc_variant(int precision, int64_t n) {
+    return precision == GTD_PREC_MIXED ? 10 : default_variant(precision, n);
+}
+
+int force_launch_count(const ForcePlan &p) { return p.sym ? sym_launches(p) : 2; }
 
 namespace {
 std::mutex g_tuned_mu;
@@ -622,8 +532,13 @@ ForcePlan make_plan(int64_t n, int precision, int device, int variant) {
     p.rows = (n + p.bi - 1) / p.bi;
     p.tiles = (n + p.bj - 1) / p.bj;
     p.total = p.rows * p.tiles;
+    p.near2 = near2_of(kDefaultNearFactor);
     int sms = 148, per_sm = 1;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    if (vi.sym >= 0) {
+        sym_make_plan(p, precision, vi.sym, sms);
+        return p;
+    }
     if (precision == GTD_PREC_MIXED)
         with_mixed(p.variant, [&](auto k) { cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kThreads, 0); });
     else
@@ -643,7 +558,6 @@ ForcePlan make_plan(int64_t n, int precision, int device, int variant) {
         p.grid = (int)grid;
         p.slots = p.grid + p.rows;
     }
-    p.near2 = near2_of(kDefaultNearFactor);
     return p;
 }
 
@@ -652,9 +566,13 @@ static size_t queue_offset(const ForcePlan &p) {
     return ((size_t)p.slots * 3 * p.bi * sizeof(double) + 255) / 256 * 256;
 }
 
-size_t partial_bytes(const ForcePlan &p) { return queue_offset(p) + (p.segs > 0 ? 256 : 0); }
+size_t partial_bytes(const ForcePlan &p) {
+    if (p.sym) return sym_partial_bytes(p);
+    return queue_offset(p) + (p.segs > 0 ? 256 : 0);
+}
 
 int fit_plan_partials(ForcePlan &p, size_t max_bytes) {
+    if (p.sym) return sym_fit(p, max_bytes);
     if (partial_bytes(p) <= max_bytes) return GTD_OK;
     const size_t per_slot = (size_t)3 * p.bi * sizeof(double);
     const int64_t max_slots = max_bytes > 512 ? (int64_t)((max_bytes - 512) / per_slot) : 0;
@@ -677,6 +595,7 @@ int fit_plan_partials(ForcePlan &p, size_t max_bytes) {
 int launch_force(int precision, const ForcePlan &p, const double4 *src, double G, double *partials,
                  cudaStream_t s) {
     if (p.n == 0) return GTD_OK;
+    if (p.sym) return sym_launch_force(precision, p, src, G, partials, s);
     unsigned *queue = p.segs > 0 ? reinterpret_cast<unsigned *>(reinterpret_cast<char *>(partials) + queue_offset(p))
                                  : nullptr;
     ForceKArgs a{p.n, p.rows, p.tiles, p.total, p.grid, p.bi, src, G, partials, p.near2, p.segs, p.seg_tiles,
@@ -718,70 +637,6 @@ __device__ __forceinline__ void row_slots(const IntArgs &a, int64_t r, int64_t &
     }
 }
 
-// The method's update of body i from its summed force (ax, ay, az), in FP64.
-__device__ __forceinline__ void apply_epilogue(const IntArgs &a, int64_t i, double ax, double ay, double az) {
-    const StepArgs &st = a.st;
-    const double h = st.h, h2 = 0.5 * st.h;
-    if (a.epi == EPI_ACC) {  // the force alone: position and velocity are not read
-        st.acc[i] = make_double4(ax, ay, az, 0.0);
-        return;
-    }
-    const double4 x = st.cur[i];
-    double4 v = st.vel[i];
-    switch (a.epi) {
-        case EPI_KDK: {
-            st.acc[i] = make_double4(ax, ay, az, 0.0);
-            v.x = fma(h2, ax, v.x); v.y = fma(h2, ay, v.y); v.z = fma(h2, az, v.z);
-            if (!st.last) {
-                v.x = fma(h2, ax, v.x); v.y = fma(h2, ay, v.y); v.z = fma(h2, az, v.z);
-                st.dst[i] = make_double4(fma(h, v.x, x.x), fma(h, v.y, x.y), fma(h, v.z, x.z), x.w);
-            }
-            st.vel[i] = v;
-            break;
-        }
-        case EPI_DKD: {
-            st.acc[i] = make_double4(ax, ay, az, 0.0);
-            v.x = fma(h, ax, v.x); v.y = fma(h, ay, v.y); v.z = fma(h, az, v.z);
-            double4 y = make_double4(fma(h2, v.x, x.x), fma(h2, v.y, x.y), fma(h2, v.z, x.z), x.w);
-            if (!st.last) y = make_double4(fma(h2, v.x, y.x), fma(h2, v.y, y.y), fma(h2, v.z, y.z), x.w);
-            st.dst[i] = y;
-            st.vel[i] = v;
-            break;
-        }
-        case EPI_EULER: {
-            st.acc[i] = make_double4(ax, ay, az, 0.0);
-            st.dst[i] = make_double4(fma(h, v.x, x.x), fma(h, v.y, x.y), fma(h, v.z, x.z), x.w);
-            v.x = fma(h, ax, v.x); v.y = fma(h, ay, v.y); v.z = fma(h, az, v.z);
-            st.vel[i] = v;
-            break;
-        }
-        case EPI_PREDICT: {
-            const double hp = st.hp;
-            st.acc[i] = make_double4(ax, ay, az, 0.0);
-            st.pred_pos[i] = make_double4(fma(hp, v.x, x.x), fma(hp, v.y, x.y), fma(hp, v.z, x.z), x.w);
-            st.pred_vel[i] = make_double4(fma(hp, ax, v.x), fma(hp, ay, v.y), fma(hp, az, v.z), 0.0);
-            break;
-        }
-        case EPI_CORR_MEULER: {
-            const double4 pv = st.pred_vel[i], a0 = st.acc[i];
-            st.dst[i] = make_double4(fma(h2, v.x + pv.x, x.x), fma(h2, v.y + pv.y, x.y), fma(h2, v.z + pv.z, x.z),
-                                     x.w);
-            v.x = fma(h2, a0.x + ax, v.x); v.y = fma(h2, a0.y + ay, v.y); v.z = fma(h2, a0.z + az, v.z);
-            st.vel[i] = v;
-            break;
-        }
-        case EPI_CORR_MIDPOINT: {
-            const double4 pv = st.pred_vel[i];
-            st.dst[i] = make_double4(fma(h, pv.x, x.x), fma(h, pv.y, x.y), fma(h, pv.z, x.z), x.w);
-            v.x = fma(h, ax, v.x); v.y = fma(h, ay, v.y); v.z = fma(h, az, v.z);
-            st.vel[i] = v;
-            break;
-        }
-        default:
-            break;
-    }
-}
-
 // Thread per body: the partial sums of body i in CTA order, one after another.
 __global__ void integrate_kernel(IntArgs a) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -797,7 +652,7 @@ __global__ void integrate_kernel(IntArgs a) {
         ay += slot[a.bi + l];
         az += slot[2 * a.bi + l];
     }
-    apply_epilogue(a, i, ax, ay, az);
+    apply_epilogue(a.st, a.epi, i, ax, ay, az);
 }
 
 // Warp per body, for rows spread over many CTAs (small N with narrow work units): the lanes load
@@ -823,7 +678,7 @@ __global__ void integrate_warp_kernel(IntArgs a) {
         ay += __shfl_xor_sync(0xffffffffu, ay, o);
         az += __shfl_xor_sync(0xffffffffu, az, o);
     }
-    if (lane == 0) apply_epilogue(a, i, ax, ay, az);
+    if (lane == 0) apply_epilogue(a.st, a.epi, i, ax, ay, az);
 }
 
 // Small FP64 systems, one launch per force evaluation.  kFusedSlices warps share a body: warp s sums
@@ -875,7 +730,7 @@ __global__ void __launch_bounds__(kFusedBodies * kFusedSlices * 32)
             sy += part[k][bl][1];
             sz += part[k][bl][2];
         }
-        apply_epilogue(a, i, sx, sy, sz);
+        apply_epilogue(a.st, a.epi, i, sx, sy, sz);
     }
 }
 
@@ -890,6 +745,7 @@ int launch_fused_small(int64_t n, const double4 *src, double G, int epi, const S
 
 int launch_integrate(const ForcePlan &p, const double *partials, int epi, const StepArgs &st, cudaStream_t s) {
     if (p.n == 0) return GTD_OK;
+    if (p.sym) return sym_launch_finish(p, partials, epi, st, nullptr, s);
     IntArgs a{p.n, p.tiles, p.total, p.grid, p.bi, epi, partials, st, p.segs};
     const int threads = 256;
     // A row's force spread over more than ~4 slots, with too few bodies for a thread each to keep
@@ -926,6 +782,7 @@ __global__ void sum_partials_kernel(IntArgs a, double *acc3) {
 
 int launch_sum_partials(const ForcePlan &p, const double *partials, double *acc3, cudaStream_t s) {
     if (p.n == 0) return GTD_OK;
+    if (p.sym) return sym_launch_finish(p, partials, EPI_ACC, StepArgs{}, acc3, s);
     IntArgs a{p.n, p.tiles, p.total, p.grid, p.bi, EPI_ACC, partials, StepArgs{}, p.segs};
     sum_partials_kernel<<<(unsigned)((p.n + 255) / 256), 256, 0, s>>>(a, acc3);
     GTD_CHECK_LAUNCH();

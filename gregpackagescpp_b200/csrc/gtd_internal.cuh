@@ -7,6 +7,7 @@
 #include <cstdarg>
 #include <cstdio>
 
+#include "direct_sym_geom.cuh"
 #include "gtd_b200.h"
 
 namespace gtd {
@@ -43,7 +44,19 @@ struct ForcePlan {
     int64_t segs = 0, seg_tiles = 0, units = 0;
     int variant = 0;         // kernel variant (i-bodies per thread, fold length)
     float near2 = 0.f;       // mixed kernel: precise-path threshold, near2_of(near factor)
+    // unordered-pair kernels: their decomposition and the bytes of partial sums a batch may take
+    bool sym = false;
+    int sym_kind = 0;
+    SymGeom sg;
+    size_t sym_bytes = kSymSlotBytes;
 };
+
+int sym_make_plan(ForcePlan &p, int precision, int kind, int sms);
+SymShape sym_shape(int precision, int kind);
+size_t sym_partial_bytes(const ForcePlan &p);
+int sym_fit(ForcePlan &p, size_t max_bytes);
+int sym_launches(const ForcePlan &p);
+int sym_launch_force(int precision, const ForcePlan &p, const double4 *src, double G, double *partials, cudaStream_t s);
 
 // Mixed kernel: a fold that holds a pair closer than 2 |X_i| / (K - 1) to one of its i-bodies (X_i:
 // the body's coordinates in its row's FP32 frame) is recomputed on the precise path, so that the
@@ -63,6 +76,7 @@ enum Epilogue : int {
     EPI_PREDICT = 4,     // acc = a; pred_x = x + hp v; pred_v = v + hp a
     EPI_CORR_MEULER = 5, // x_dst = x + h/2 (v + pred_v); v += h/2 (acc + a)
     EPI_CORR_MIDPOINT = 6,  // x_dst = x + h pred_v; v += h a
+    EPI_ACC3 = 7,        // (double *)acc: a as triples
 };
 
 struct StepArgs {
@@ -84,6 +98,9 @@ int variant_info(int precision, int variant, int *i_per_thread, int *fold);
 // Process-wide autotune results: a handle without a pinned variant takes the variant last tuned on
 // its device for its precision and size class (the bit length of N), else default_variant.
 int default_variant(int precision, int64_t n);
+int noalloc_variant(int precision, int64_t n);
+// Kernels that a force evaluation and its integration launch.
+int force_launch_count(const ForcePlan &p);
 // Up to this many bodies an FP64 force evaluation and its update run as one fused launch.
 constexpr int64_t kFusedMaxN = 4096;
 int launch_fused_small(int64_t n, const double4 *src, double G, int epi, const StepArgs &st, cudaStream_t s);
@@ -104,6 +121,9 @@ int launch_integrate(const ForcePlan &p, const double *partials, int epi, const 
 int launch_kick_drift(int64_t n, const double4 *cur, double4 *dst, double4 *vel, const double4 *acc, double h,
                       cudaStream_t s);
 int launch_half_drift(int64_t n, const double4 *cur, double4 *dst, const double4 *vel, double h, cudaStream_t s);
+
+int sym_launch_finish(const ForcePlan &p, const double *partials, int epi, const StepArgs &st, double *acc3,
+                      cudaStream_t s);
 
 // FP64 diagnostics: out[0]=KE, out[1]=PE, out[2..4]=momentum, out[5..7]=sum m x, out[8]=sum m.
 int launch_energy(int64_t n, const double4 *pm, const double4 *vel, double G, double *scratch, int64_t scratch_n,

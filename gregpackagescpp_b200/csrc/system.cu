@@ -181,7 +181,7 @@ int force_and_integrate(gtd_system *s, const double4 *src, int epi, const StepAr
     if (s->time_force && (rc = timed_event(s))) return rc;
     rc = launch_integrate(s->plan, s->partials, epi, st, s->stream);
     if (rc) return rc;
-    s->launches += 2;
+    s->launches += (uint64_t)force_launch_count(s->plan);
     return GTD_OK;
 }
 
@@ -739,7 +739,7 @@ int gtd_system_direct_plan_info(gtd_system *s, int64_t *units, int64_t *partial_
     DeviceGuard g(s->device);
     int rc = ensure_plan(s);
     if (rc) return rc;
-    if (units) *units = s->plan.segs > 0 ? s->plan.units : s->plan.total;
+    if (units) *units = s->plan.units > 0 ? s->plan.units : s->plan.total;
     if (partial_bytes_out) *partial_bytes_out = (int64_t)partial_bytes(s->plan);
     return GTD_OK;
 }

@@ -317,7 +317,7 @@ GTD_API int gtd_bh_accelerations(gtd_system *sys, double *a3, uint32_t *n_inter)
  * device, stalling other streams inside a running loop.  The caller passes device buffers: pm4 =
  * n x 4 doubles (x, y, z, m), 16-byte aligned; acc3 = n x 3 doubles, written with the accelerations
  * sum_j G m_j (x_j - x_i) / |x_j - x_i|^3 (as gtd_system_accelerations).  The only scratch, the
- * force kernel's partial sums, lives in a fixed 8 MiB device array compiled into the library (every
+ * force kernel's partial sums, lives in a fixed 64 MiB device array compiled into the library (every
  * GPU that loads the library holds it until the process exits); n is limited to 65536 and larger n
  * is rejected with GTD_ERR_CAPACITY.  The first call on a device looks up that array's address
  * (cudaGetSymbolAddress), so make the first call on each device before any stream capture.  All
