@@ -30,13 +30,13 @@ EULER, MODIFIED_EULER, MIDPOINT, LEAPFROG_KDK, LEAPFROG_DKD = 2, 4, 8, 16, 32
 
 def reference_tree() -> str | None:
     """The reference checkout the Makefile reads (GTD_REFERENCE_DIR, else the Makefile's default),
-    or None when it is not present on this machine."""
+    or None when its headers are not present on this machine."""
     try:
         r = subprocess.run(["make", "-s", "-C", HERE, "print-ref"], capture_output=True, text=True, timeout=60)
         path = r.stdout.strip()
     except Exception:
         return None
-    return path if path and os.path.isdir(path) else None
+    return path if path and os.path.isfile(os.path.join(path, "gregsys.hpp")) else None
 
 
 def ensure_built(ref: bool = False) -> None:
