@@ -17,6 +17,8 @@ def _bind(L):
     if getattr(L, "_adj_bound", False):
         return
     L.gtd_adjoint_create.argtypes = [C.POINTER(vp), ip, i64, u64, u64, C.c_double, C.c_double]
+    L.gtd_adjoint_workspace_bytes.argtypes = [ip, i64, u64, u64, C.POINTER(u64)]
+    L.gtd_adjoint_create_in.argtypes = [C.POINTER(vp), ip, i64, u64, u64, C.c_double, C.c_double, vp, u64]
     L.gtd_adjoint_destroy.argtypes = [vp]
     L.gtd_adjoint_forward.argtypes = [vp, vp, vp, vp, vp, vp, vp]
     L.gtd_adjoint_backward.argtypes = [vp, vp, vp, vp, vp, vp, vp]
@@ -25,14 +27,23 @@ def _bind(L):
 
 
 class AdjointRun:
-    """One forward run kept for its reverse sweep (checkpoints every ``checkpoint_every`` steps)."""
+    """One forward run kept for its reverse sweep (checkpoints every ``checkpoint_every`` steps; 0: the
+    library's choice).  ``allocate(bytes)`` gives the device memory it works in (an object with
+    ``data_ptr()``, kept for the life of the run); without it the library allocates its own."""
 
-    def __init__(self, n: int, steps: int, checkpoint_every: int, G: float, dt: float, device: int):
+    def __init__(self, n: int, steps: int, checkpoint_every: int, G: float, dt: float, device: int, allocate=None):
         L = _lib.load()
         _bind(L)
         self._L = L
         h = C.c_void_p()
-        check(L.gtd_adjoint_create(C.byref(h), device, n, steps, checkpoint_every, G, dt))
+        if allocate is None:
+            check(L.gtd_adjoint_create(C.byref(h), device, n, steps, checkpoint_every, G, dt))
+        else:
+            size = C.c_uint64()
+            check(L.gtd_adjoint_workspace_bytes(device, n, steps, checkpoint_every, C.byref(size)))
+            self._mem = allocate(size.value)
+            check(L.gtd_adjoint_create_in(C.byref(h), device, n, steps, checkpoint_every, G, dt, self._mem.data_ptr(),
+                                          size.value))
         self._h = h
 
     def launches(self) -> int:
@@ -51,9 +62,9 @@ class AdjointRun:
 
 def leapfrog_final_state(x0, v0, m, G: float, dt: float, steps: int, checkpoint_every: int | None = None):
     """(x_T, v_T) of `steps` KDK steps from (x0, v0) with masses m (CUDA float64 tensors, shapes
-    (n,3), (n,3), (n,)), differentiable with respect to x0, v0 and m."""
-    import math
-
+    (n,3), (n,3), (n,)), differentiable with respect to x0, v0 and m.  The run's buffers are torch's, on
+    the stream of the call; autograd runs the reverse sweep on the same stream.  checkpoint_every bounds
+    their size; by default every position is kept while they fit 1.25 GiB."""
     import torch
 
     class _LeapfrogAdjoint(torch.autograd.Function):
@@ -64,8 +75,8 @@ def leapfrog_final_state(x0, v0, m, G: float, dt: float, steps: int, checkpoint_
                     raise TypeError("x0, v0, m must be CUDA float64 tensors")
             x0c, v0c, mc = x0_.contiguous(), v0_.contiguous(), m_.contiguous()
             n = mc.numel()
-            every = checkpoint_every or max(1, int(round(math.sqrt(steps))))
-            run = AdjointRun(n, steps, every, G, dt, x0c.device.index or 0)
+            run = AdjointRun(n, steps, checkpoint_every or 0, G, dt, x0c.device.index or 0,
+                             lambda size: torch.empty(size, dtype=torch.uint8, device=x0c.device))
             xT = torch.empty_like(x0c)
             vT = torch.empty_like(v0c)
             stream = torch.cuda.current_stream(x0c.device).cuda_stream

@@ -70,6 +70,13 @@ __device__ __forceinline__ void apply_epilogue(const StepArgs &st, int epi, int6
             st.vel[i] = v;
             break;
         }
+        case EPI_KICK_DRIFT: {
+            const double c = st.hp;
+            v.x = fma(c, ax, v.x); v.y = fma(c, ay, v.y); v.z = fma(c, az, v.z);
+            st.vel[i] = v;
+            if (!st.last) st.dst[i] = make_double4(fma(h, v.x, x.x), fma(h, v.y, x.y), fma(h, v.z, x.z), x.w);
+            break;
+        }
         default:
             break;
     }

@@ -24,9 +24,11 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "direct_epilogue.cuh"
 #include "direct_mixed.cuh"
+#include "direct_sym_reduce.cuh"
 #include "gtd_internal.cuh"
 #include "gtd_math.cuh"
 
@@ -42,19 +44,6 @@ struct SymKArgs {
     float near2;
     unsigned *queue;            // zeroed before the launch
 };
-
-// term(0) + .. + term(N - 1), added as a balanced tree (short dependent chains, fixed order).
-template <int N, typename F>
-__device__ __forceinline__ double sym_tree(F &&term) {
-    double v[N];
-#pragma unroll
-    for (int k = 0; k < N; ++k) v[k] = term(k);
-#pragma unroll
-    for (int h = N / 2; h > 0; h >>= 1)
-#pragma unroll
-        for (int k = 0; k < h; ++k) v[k] += v[k + h];
-    return v[0];
-}
 
 // -------------------------------------------------------------------------------------------
 // FP64
@@ -111,6 +100,9 @@ __global__ void __launch_bounds__(T, MINB) force_f64_sym_kernel(SymKArgs a) {
         }
         const int64_t own_end = (r / a.g.s + 1) * a.g.kw;  // tiles below are ordered pairs
         const int64_t coff = sym_col_off(a.g, r) - a.col0 - own_end;
+        // Coincident bodies: selected away within the row block's group and in the last, incomplete 256
+        // bodies, where the ordered-pair kernel does so too.
+        const int64_t tail = a.g.n / 256 * (256 / TC);
         if (c0 < c1)
             for (int c = t; c < TC; c += T) stage(0, c, fetch(c0 * TC + c));
         __syncthreads();
@@ -127,13 +119,14 @@ __global__ void __launch_bounds__(T, MINB) force_f64_sym_kernel(SymKArgs a) {
                 for (int ch = 0; ch < kChunks; ++ch) {
                     const double2 *XY = sxy[cur] + ch * 64 + lane, *ZM = szm[cur] + ch * 64 + lane;
                     double cx = 0.0, cy = 0.0, cz = 0.0;
-#pragma unroll 4
-                    for (int s = 0; s < 32; ++s) {
+                    auto step = [&](auto guard, int s) {
                         const double2 xy = XY[s], zm = ZM[s];
 #pragma unroll
                         for (int k = 0; k < I; ++k) {
                             const double dx = xy.x - xi[k], dy = xy.y - yi[k], dz = zm.x - zi[k];
-                            const double w = inv_r3(fma(dz, dz, fma(dy, dy, dx * dx)));
+                            const double r2 = fma(dz, dz, fma(dy, dy, dx * dx));
+                            double w = inv_r3(r2);
+                            if (decltype(guard)::value) w = r2 > 0.0 ? w : 0.0;
                             const double sj = zm.y * w, si = mi[k] * w;
                             ax[k] = fma(sj, dx, ax[k]);
                             ay[k] = fma(sj, dy, ay[k]);
@@ -145,6 +138,13 @@ __global__ void __launch_bounds__(T, MINB) force_f64_sym_kernel(SymKArgs a) {
                         cx = __shfl_sync(0xffffffffu, cx, lane + 1);
                         cy = __shfl_sync(0xffffffffu, cy, lane + 1);
                         cz = __shfl_sync(0xffffffffu, cz, lane + 1);
+                    };
+                    if (jt >= tail) {
+#pragma unroll 1
+                        for (int s = 0; s < 32; ++s) step(std::true_type{}, s);
+                    } else {
+#pragma unroll 4
+                        for (int s = 0; s < 32; ++s) step(std::false_type{}, s);
                     }
                     col[cur][warp][0][ch * 32 + lane] = cx;
                     col[cur][warp][1][ch * 32 + lane] = cy;
@@ -523,73 +523,25 @@ __global__ void __launch_bounds__(T, MINB) force_mixed_sym_kernel(SymKArgs a) {
 // The sum of a body's row and column slots
 // -------------------------------------------------------------------------------------------
 struct SymReduceArgs {
-    SymGeom g;
-    const double *rowpart, *colpart;
-    int64_t unit0, col0;
-    int64_t Pa, Pb;       // super-groups of the batch
-    const double *base;   // sums of the earlier batches (3 n), or NULL
-    double *out3;         // mode 0: base to write (3 arrays of n); mode 2: triples
-    int mode;             // 0 running sum, 1 epilogue, 2 triples
+    SymSlots slots;
+    double *out3;  // mode 0: the running sum to write (3 arrays of n); mode 2: triples
+    int mode;      // 0 running sum, 1 epilogue, 2 triples
     StepArgs st;
     int epi;
 };
 
-// 32 bodies per CTA; warp w takes every kRedWarps-th slot of each body (consecutive bodies read
-// consecutive words), compensated; the warps' sums are added in warp order.
-constexpr int kRedWarps = 8;
-
 __global__ void __launch_bounds__(kRedWarps * 32) sym_reduce_kernel(SymReduceArgs a) {
-    __shared__ double part[kRedWarps][3][32];
-    const SymGeom &g = a.g;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int64_t i0 = (int64_t)blockIdx.x * 32, i = i0 + lane;
-    // B, TC and W are multiples of 32: the CTA's bodies share a row block, a tile and a group
-    const int64_t b = i0 / g.B, R = i0 / g.W, P = R / g.L, tile = i0 / g.TC;
-    const int l = (int)(i0 - b * g.B) + lane, cl = (int)(i0 - tile * g.TC) + lane;
-    double s[3] = {0.0, 0.0, 0.0}, k[3] = {0.0, 0.0, 0.0};
-    if (i < g.n) {
-        int64_t rows = 0;  // row slots of the body in this batch
-        if (P >= a.Pa && P < a.Pb) rows = (g.Gs - P) * g.q;
-        const int64_t per = sym_block_units(g);
-        const int64_t u0 = sym_tri(g, P) * per + (b - P * g.L * g.s) * g.q - a.unit0;
-#pragma unroll 2
-        for (int64_t e = warp; e < rows; e += kRedWarps) {
-            const int64_t Q = e / g.q, sub = e - Q * g.q;
-            const double *slot = a.rowpart + (size_t)(u0 + Q * per + sub) * 3 * g.B + l;
+    sym_reduce<3>(a.slots, [&](int64_t i, const double (&v)[3]) {
+        if (a.mode == 1) {
+            apply_epilogue(a.st, a.epi, i, v[0], v[1], v[2]);
+        } else if (a.mode == 0) {
 #pragma unroll
-            for (int d = 0; d < 3; ++d) kahan_add(s[d], k[d], slot[d * g.B]);
+            for (int d = 0; d < 3; ++d) a.out3[(size_t)d * a.slots.g.n + i] = v[d];
+        } else {
+#pragma unroll
+            for (int d = 0; d < 3; ++d) a.out3[3 * i + d] = v[d];
         }
-        const int64_t r0 = a.Pa * g.L * g.s, r1 = min(a.Pb * g.L, R) * g.s;
-#pragma unroll 4
-        for (int64_t r = r0 + warp; r < r1; r += kRedWarps) {
-            const int64_t at = sym_col_off(g, r) - a.col0 + tile - (r / g.s + 1) * g.kw;
-            const double *slot = a.colpart + (size_t)at * 3 * g.TC + cl;
-#pragma unroll
-            for (int d = 0; d < 3; ++d) kahan_add(s[d], k[d], slot[d * g.TC]);
-        }
-    }
-#pragma unroll
-    for (int d = 0; d < 3; ++d) part[warp][d][lane] = s[d] - k[d];
-    __syncthreads();
-    if (warp != 0 || i >= g.n) return;
-    double v[3];
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        double sum = 0.0, comp = 0.0;
-        if (a.base) sum = a.base[(size_t)d * g.n + i];
-#pragma unroll
-        for (int w = 0; w < kRedWarps; ++w) kahan_add(sum, comp, part[w][d][lane]);
-        v[d] = sum - comp;
-    }
-    if (a.mode == 1) {
-        apply_epilogue(a.st, a.epi, i, v[0], v[1], v[2]);
-    } else if (a.mode == 0) {
-#pragma unroll
-        for (int d = 0; d < 3; ++d) a.out3[(size_t)d * g.n + i] = v[d];
-    } else {
-#pragma unroll
-        for (int d = 0; d < 3; ++d) a.out3[3 * i + d] = v[d];
-    }
+    });
 }
 
 // -------------------------------------------------------------------------------------------
@@ -615,28 +567,7 @@ static void with_sym(int precision, int kind, F &&f) {
     }
 }
 
-// Partials buffer: a queue counter per batch | the running sum (where there are several batches) | slots.
-struct SymLayout {
-    int64_t batches = 0;
-    size_t base = 0, slots = 0, bytes = 0;
-};
-static SymLayout sym_layout(const ForcePlan &p) {
-    const SymGeom &g = p.sg;
-    SymLayout o;
-    size_t most = 0;
-    for (int64_t P = 0; P < g.Gs;) {
-        const int64_t e = sym_batch_end(g, P, p.sym_bytes);
-        most = std::max(most, sym_slot_bytes(g, P, e));
-        ++o.batches;
-        P = e;
-    }
-    o.base = ((size_t)o.batches * sizeof(unsigned) + 255) / 256 * 256;
-    o.slots = o.base + (o.batches > 1 ? ((size_t)3 * g.n * sizeof(double) + 255) / 256 * 256 : 0);
-    o.bytes = o.slots + most;
-    return o;
-}
-
-size_t sym_partial_bytes(const ForcePlan &p) { return sym_layout(p).bytes; }
+size_t sym_partial_bytes(const ForcePlan &p) { return sym_layout(p.sg, p.sym_bytes, 3).bytes; }
 
 int sym_make_plan(ForcePlan &p, int precision, int kind, int sms) {
     const SymShape sh = sym_shape(precision, kind);
@@ -677,40 +608,25 @@ int sym_fit(ForcePlan &p, size_t max_bytes) {
     return GTD_OK;
 }
 
-static SymReduceArgs sym_reduce_args(const ForcePlan &p, const SymLayout &lay, const double *partials, int64_t Pa,
-                                     int64_t Pb) {
-    const SymGeom &g = p.sg;
-    const char *base = reinterpret_cast<const char *>(partials);
-    SymReduceArgs r{};
-    r.g = g;
-    r.unit0 = sym_tri(g, Pa) * sym_block_units(g);
-    r.col0 = sym_col_off(g, Pa * g.L * g.s);
-    r.rowpart = reinterpret_cast<const double *>(base + lay.slots);
-    r.colpart = r.rowpart + (size_t)((sym_tri(g, Pb) - sym_tri(g, Pa)) * sym_block_units(g)) * 3 * g.B;
-    r.Pa = Pa;
-    r.Pb = Pb;
-    r.base = Pa > 0 ? reinterpret_cast<const double *>(base + lay.base) : nullptr;
-    return r;
-}
-
 int sym_launch_force(int precision, const ForcePlan &p, const double4 *src, double G, double *partials, cudaStream_t s) {
     const SymGeom &g = p.sg;
-    const SymLayout lay = sym_layout(p);
+    const SymLayout lay = sym_layout(g, p.sym_bytes, 3);
     char *mem = reinterpret_cast<char *>(partials);
     GTD_CUDA(cudaMemsetAsync(mem, 0, (size_t)lay.batches * sizeof(unsigned), s));
     int64_t batch = 0;
     for (int64_t Pa = 0; Pa < g.Gs; ++batch) {
         const int64_t Pb = sym_batch_end(g, Pa, p.sym_bytes);
-        SymReduceArgs r = sym_reduce_args(p, lay, partials, Pa, Pb);
+        SymReduceArgs r{};
+        r.slots = sym_slots(g, lay, mem, Pa, Pb, 3);
         SymKArgs a{};
         a.g = g;
         a.src = src;
         a.G = G;
-        a.rowpart = const_cast<double *>(r.rowpart);
-        a.colpart = const_cast<double *>(r.colpart);
-        a.unit0 = r.unit0;
+        a.rowpart = const_cast<double *>(r.slots.rowpart);
+        a.colpart = const_cast<double *>(r.slots.colpart);
+        a.unit0 = r.slots.unit0;
         a.unit1 = sym_tri(g, Pb) * sym_block_units(g);
-        a.col0 = r.col0;
+        a.col0 = r.slots.col0;
         a.near2 = p.near2;
         a.queue = reinterpret_cast<unsigned *>(mem) + batch;
         const int grid = (int)std::min<int64_t>(p.grid, a.unit1 - a.unit0);
@@ -732,19 +648,17 @@ int sym_launch_force(int precision, const ForcePlan &p, const double4 *src, doub
     return GTD_OK;
 }
 
-int sym_launches(const ForcePlan &p) { return 2 * (int)sym_layout(p).batches; }
+int sym_launches(const ForcePlan &p) { return 2 * (int)sym_layout(p.sg, p.sym_bytes, 3).batches; }
 
 // The last batch's sums, with the earlier ones', into the epilogue (acc3 == NULL) or acc3.
 int sym_launch_finish(const ForcePlan &p, const double *partials, int epi, const StepArgs &st, double *acc3,
                       cudaStream_t s) {
     const SymGeom &g = p.sg;
-    const SymLayout lay = sym_layout(p);
+    const SymLayout lay = sym_layout(g, p.sym_bytes, 3);
     int64_t Pa = 0, Pb = sym_batch_end(g, 0, p.sym_bytes);
-    while (Pb < g.Gs) {
-        Pa = Pb;
-        Pb = sym_batch_end(g, Pa, p.sym_bytes);
-    }
-    SymReduceArgs r = sym_reduce_args(p, lay, partials, Pa, Pb);
+    for (; Pb < g.Gs; Pb = sym_batch_end(g, Pa, p.sym_bytes)) Pa = Pb;
+    SymReduceArgs r{};
+    r.slots = sym_slots(g, lay, reinterpret_cast<const char *>(partials), Pa, Pb, 3);
     r.mode = acc3 ? 2 : 1;
     r.out3 = acc3;
     r.st = st;

@@ -57,17 +57,17 @@ __host__ __device__ __forceinline__ SymUnit sym_unit(const SymGeom &g, int64_t u
     return o;
 }
 
-// Bytes of the slots of super-groups [Pa, Pb).
-inline size_t sym_slot_bytes(const SymGeom &g, int64_t Pa, int64_t Pb) {
+// Bytes of the slots of super-groups [Pa, Pb), D words per body.
+inline size_t sym_slot_bytes(const SymGeom &g, int64_t Pa, int64_t Pb, int D = 3) {
     const int64_t units = (sym_tri(g, Pb) - sym_tri(g, Pa)) * sym_block_units(g);
     const int64_t cols = sym_col_off(g, std::min(Pb * g.L, g.G - 1) * g.s) - sym_col_off(g, std::min(Pa * g.L, g.G - 1) * g.s);
-    return ((size_t)units * g.B + (size_t)cols * g.TC) * 3 * sizeof(double);
+    return ((size_t)units * g.B + (size_t)cols * g.TC) * D * sizeof(double);
 }
 
 // The end of the batch that starts at super-group Pa: as many as fit `bytes` (at least one).
-inline int64_t sym_batch_end(const SymGeom &g, int64_t Pa, size_t bytes) {
+inline int64_t sym_batch_end(const SymGeom &g, int64_t Pa, size_t bytes, int D = 3) {
     int64_t Pb = Pa + 1;
-    while (Pb < g.Gs && sym_slot_bytes(g, Pa, Pb + 1) <= bytes) ++Pb;
+    while (Pb < g.Gs && sym_slot_bytes(g, Pa, Pb + 1, D) <= bytes) ++Pb;
     return Pb;
 }
 
@@ -88,7 +88,7 @@ inline SymGeom sym_geometry(int64_t n, const SymShape &sh, int sms, int per_sm) 
     // tiles plus about a tenth of a 64-column tile, an SM runs per_sm units side by side (fewer leave
     // its pipe partly idle), and the SM with the most units sets the time.
     double best = 0.0;
-    for (int q = 1; q <= g.kw; q *= 2) {
+    for (int q = 1; g.kw % q == 0; q *= 2) {
         const double each = (double)((blocks * q + sms - 1) / sms);
         const double side = std::min<double>(each, per_sm);
         const double cost = each * ((double)(g.kw / q) * g.TC / 64 + 0.1) * (side + per_sm) / (2.0 * side);

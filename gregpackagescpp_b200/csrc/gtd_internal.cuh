@@ -77,6 +77,7 @@ enum Epilogue : int {
     EPI_CORR_MEULER = 5, // x_dst = x + h/2 (v + pred_v); v += h/2 (acc + a)
     EPI_CORR_MIDPOINT = 6,  // x_dst = x + h pred_v; v += h a
     EPI_ACC3 = 7,        // (double *)acc: a as triples
+    EPI_KICK_DRIFT = 8,  // v += hp a; if !last: x_dst = x + h v
 };
 
 struct StepArgs {

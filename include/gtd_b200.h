@@ -368,12 +368,21 @@ GTD_API int gtd_ensemble_autotune(gtd_ensemble *ens, int *best_threads, double *
 /* ---- adjoint of the FP64 leapfrog KDK evolve (no counterpart in the reference) ---------------
  * Gradients of a loss on the final state of evolve(leapfrog_kdk) (gregsys.hpp:2946-2990) with
  * respect to the initial positions, velocities and masses, by a hand-written reverse sweep with
- * checkpoints every `checkpoint_every` steps and recomputation in between.  All arrays are DEVICE
- * pointers (n x 3 or n doubles, row-major); `stream` is a cudaStream_t or NULL. */
+ * checkpoints every `checkpoint_every` steps and recomputation in between; with checkpoint_every = 0
+ * every position is kept (32 bytes per body and step) while they fit 1.25 GiB, and checkpoints are about
+ * sqrt(steps) apart beyond.  All arrays are DEVICE pointers (n x 3 or n doubles, row-major); `stream` is
+ * a cudaStream_t or NULL. */
 typedef struct gtd_adjoint gtd_adjoint;
 
 GTD_API int gtd_adjoint_create(gtd_adjoint **out, int device, int64_t n, uint64_t steps, uint64_t checkpoint_every,
                                double G, double dt);
+/* The same with the caller's device memory: gtd_adjoint_workspace_bytes gives its size for the same
+ * arguments, `workspace` is 256-byte aligned and stays the caller's, who keeps it until the handle is
+ * destroyed and its work has run.  Nothing is allocated and destroy does not synchronise. */
+GTD_API int gtd_adjoint_workspace_bytes(int device, int64_t n, uint64_t steps, uint64_t checkpoint_every,
+                                        uint64_t *bytes);
+GTD_API int gtd_adjoint_create_in(gtd_adjoint **out, int device, int64_t n, uint64_t steps, uint64_t checkpoint_every,
+                                  double G, double dt, void *workspace, uint64_t bytes);
 GTD_API int gtd_adjoint_destroy(gtd_adjoint *adj);
 GTD_API int gtd_adjoint_forward(gtd_adjoint *adj, const double *x0, const double *v0, const double *m, double *xT,
                                 double *vT, void *stream);
