@@ -5,11 +5,13 @@
 // This is the device form of the reference drivers' ensemble pattern - one gtd::system per
 // std::thread (bdsim.cpp:82-113) - with FP64 state and FP32 pair forces.
 //
-// Work decomposition: one CTA owns one system at a time.  Systems are handed out largest first
-// from an atomic work counter (longest-processing-time order), so the spread in per-system work
-// (N = 3 .. 2048: 4.7e5x in pairs) balances across the persistent grid.  A system's bodies are staged once per
-// step in shared memory as FP32 coordinates relative to the system's mean position, with G m and
-// the radius; the rows are spread over the CTA in passes of IB rows per thread (IB = 1, 2 or 4),
+// Work decomposition: a CTA takes one item, a chunk of IB rows per thread of one system, and the items
+// start largest system first, so the spread in per-system work (N = 3 .. 2048: 4.7e5x in pairs) balances
+// across the GPU; with a CTA per system the largest alone set the step time (512 systems of up to 2048
+// bodies: 0.60 ms a step, 0.38 with items).  The CTA that finishes a system's last chunk (a count of
+// arrivals, no waiting) also takes its merges and the next step's kick and drift, so a step stays one
+// launch.  Each CTA stages the whole system in shared memory as FP32 coordinates relative to the
+// system's mean position, with G m; its rows are spread over the threads, IB (1, 2 or 4) each,
 // and each thread sums its rows' forces two j-bodies per packed FP32x2 instruction, folding every
 // 64 j-bodies into FP64.  Alongside the force it keeps the smallest separation to any other body (a
 // 3-input float minimum; the one fold holding the row's own body excludes the self pair by its bit
@@ -26,25 +28,37 @@
 
 #include "gtd_internal.cuh"
 
+namespace gtd {
+struct EnsCand;
+struct EnsInfo;
+}
+
 struct gtd_ensemble {
     int device = 0;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     double G = 6.6743e-11, dt = 1.0;
     int merge = 1;
-    int threads = 256;   // CTA size (autotuned)
-    int ib = 1;          // bodies per thread in the force loop (autotuned; 2 and 4 need threads <= 256)
-    int blocks_per_sm = 0;
+    int threads = 256;   // CTA size
+    int ib = 1;          // bodies per thread in the force loop (2 and 4 need threads <= 256)
+    bool configured = false;  // both set by the caller or the autotuner; else ens_default chooses at upload
     int64_t n_sys = 0, n_bodies = 0;
     int max_n = 0;
     std::vector<int64_t> off_h;       // [n_sys+1]
+    std::vector<int32_t> order_h;     // systems, largest first
     int64_t *off = nullptr;           // [n_sys+1]
     int32_t *cnt = nullptr;           // live bodies per system
     int32_t *order = nullptr;         // systems, largest first
     double4 *pos = nullptr, *vel = nullptr, *acc = nullptr;
     double *rad = nullptr, *rest = nullptr;
     int32_t *ids = nullptr;
-    unsigned *work = nullptr;         // [2]: work counter, merges this launch
+    unsigned *work = nullptr;         // [2]: unused, merges so far
+    gtd::EnsCand *cand = nullptr;     // [n_sys] rows the separation test flagged
+    gtd::EnsInfo *info = nullptr;     // [n_sys] frame of the staged coordinates
+    int *arrived = nullptr;           // [n_sys] chunks finished in this launch
+    int2 *items = nullptr;            // (system, first row), largest system first
+    int64_t n_items = 0;
+    int items_for = 0;                // the (threads, ib) the items were made for
     int *status = nullptr;
     bool begun = false;
     uint64_t launches = 0;
@@ -58,20 +72,39 @@ namespace gtd {
 constexpr int kEnsMaxN = 8192;
 constexpr int kEnsFold = 64;
 
+constexpr int kEnsCand = 256;  // candidate rows a system's scan tracks before it falls back to the full scan
+
+struct EnsCand {
+    int n;                 // candidates listed (may exceed kEnsCand: then the list is incomplete)
+    int o, num, next;      // scan state: current row, rows, the partner found (-1: none, -2: done)
+    int restarted;
+    int row[kEnsCand];
+};
+
+// Frame of a system's staged coordinates and what its separation test needs.
+struct EnsInfo {
+    double cx, cy, cz;  // mean position
+    float rmax, floor2, slack;
+};
+
 struct EnsArgs {
-    int n_sys;
     const int64_t *off;
     int32_t *cnt;
-    const int32_t *order;
+    const int32_t *order;  // systems, largest first
+    const int2 *items;
     double4 *pos, *vel, *acc;
     double *rad, *rest;
     int32_t *ids;
+    EnsCand *cand;
+    EnsInfo *info;
+    int *arrived;
     double G, h;
-    int kdk;     // 0: force only (initial acceleration); 1: kick-drift, force, kick
+    int kick;    // close the step with a half kick (0: the initial force)
+    int pre;     // then open the next one: half kick and drift
     int merge;
+    int chunk;   // rows per item
     int stride;  // floats per staged coordinate array (largest system, rounded up to even)
     unsigned *work;
-    int *status;
 };
 
 __device__ __forceinline__ float ens_rsqrt(float x) {
@@ -177,15 +210,6 @@ __device__ __noinline__ int ens_merge_scan(int n, int o0, bool restarted0, doubl
     __syncthreads();
     return out;
 }
-
-constexpr int kEnsCand = 256;  // candidate rows a system's scan tracks before it falls back to the full scan
-
-struct EnsCand {
-    int n;                 // candidates listed (may exceed kEnsCand: then the list is incomplete)
-    int o, num, next;      // scan state: current row, rows, the partner found (-1: none, -2: done)
-    int restarted;
-    int row[kEnsCand];
-};
 
 // One step of the candidate scan, by one thread: sorts and de-duplicates the list, finds the next
 // (row, partner) pair in scan order from the state in c and merges the partner into the row
@@ -357,7 +381,7 @@ template <int IB>
 __device__ __forceinline__ int ens_force_rows(int r0, int s, int nc, int npad, const float *sx, const float *sy,
                                               const float *sz, const float *sm, double4 *pos, double4 *vel,
                                               double4 *acc, const double *rad, float rmx, float slack, bool kick,
-                                              double h2, float floor2, EnsCand &cand) {
+                                              double h2, float floor2, EnsCand *cand) {
     const float2 *X2 = reinterpret_cast<const float2 *>(sx);
     const float2 *Y2 = reinterpret_cast<const float2 *>(sy);
     const float2 *Z2 = reinterpret_cast<const float2 *>(sz);
@@ -412,8 +436,10 @@ __device__ __forceinline__ int ens_force_rows(int r0, int s, int nc, int npad, c
             const float reach = ((float)rad[i] + rmx) * 1.00001f + slack;
             if (mind2 < reach * reach * 1.0001f + floor2) {
                 flagged = 1;
-                const int k = atomicAdd(&cand.n, 1);
-                if (k < kEnsCand) cand.row[k] = i;
+                if (cand) {
+                    const int k = atomicAdd(&cand->n, 1);
+                    if (k < kEnsCand) cand->row[k] = i;
+                }
             }
         }
         if (kick) {
@@ -426,8 +452,112 @@ __device__ __forceinline__ int ens_force_rows(int r0, int s, int nc, int npad, c
     return flagged;
 }
 
-// One launch = one KDK step (or the initial force) for every system.  IB bodies per thread (1, 2 or 4;
-// each staged j pair feeds IB bodies, dividing the shared-memory reads per interaction by IB).
+__device__ __forceinline__ double4 ens_ldcg(const double4 *p) {  // past the L1: another CTA may have written it
+    const double2 a = __ldcg(reinterpret_cast<const double2 *>(p)), b = __ldcg(reinterpret_cast<const double2 *>(p) + 1);
+    return make_double4(a.x, a.y, b.x, b.y);
+}
+
+// Half kick and drift of a system's n rows (with pre), then its frame, by one CTA.  The frame is left in
+// shared memory (o) and in *out.
+struct EnsBeginSmem {
+    double red[3][32];
+    float redr[32], redg[32];
+    EnsInfo o;
+    int xmax_bits;  // largest staged |coordinate| (non-negative float bits)
+};
+__device__ __noinline__ void ens_begin(int n, double G, double h, int pre, double4 *pos, double4 *vel, const double4 *acc,
+                                       const double *rad, EnsInfo *out, EnsBeginSmem &S) {
+    const int t = threadIdx.x, T = blockDim.x, lane = t & 31, warp = t >> 5, nw = (T + 31) >> 5;
+    const double h2 = 0.5 * h;
+    double cx = 0.0, cy = 0.0, cz = 0.0;
+    float rmax = 0.f, gmax = 0.f;
+    for (int i = t; i < n; i += T) {
+        double4 p = ens_ldcg(&pos[i]);
+        if (pre) {
+            double4 v = ens_ldcg(&vel[i]);
+            const double4 ac = ens_ldcg(&acc[i]);
+            v.x = fma(h2, ac.x, v.x); v.y = fma(h2, ac.y, v.y); v.z = fma(h2, ac.z, v.z);
+            p.x = fma(h, v.x, p.x); p.y = fma(h, v.y, p.y); p.z = fma(h, v.z, p.z);
+            vel[i] = v;
+            pos[i] = p;
+        }
+        cx += p.x; cy += p.y; cz += p.z;
+        rmax = fmaxf(rmax, (float)__ldcg(&rad[i]));
+        gmax = fmaxf(gmax, (float)(G * p.w));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        cx += __shfl_xor_sync(0xffffffffu, cx, o);
+        cy += __shfl_xor_sync(0xffffffffu, cy, o);
+        cz += __shfl_xor_sync(0xffffffffu, cz, o);
+        rmax = fmaxf(rmax, __shfl_xor_sync(0xffffffffu, rmax, o));
+        gmax = fmaxf(gmax, __shfl_xor_sync(0xffffffffu, gmax, o));
+    }
+    if (lane == 0) {
+        S.red[0][warp] = cx; S.red[1][warp] = cy; S.red[2][warp] = cz;
+        S.redr[warp] = rmax;
+        S.redg[warp] = gmax;
+    }
+    __syncthreads();
+    if (t == 0) {
+        double X = 0, Y = 0, Z = 0;
+        float R = 0.f, Gm = 0.f;
+        for (int w = 0; w < nw; ++w) {
+            X += S.red[0][w]; Y += S.red[1][w]; Z += S.red[2][w];
+            R = fmaxf(R, S.redr[w]);
+            Gm = fmaxf(Gm, S.redg[w]);
+        }
+        S.o.cx = X / n; S.o.cy = Y / n; S.o.cz = Z / n;
+        S.o.rmax = R;
+        S.o.floor2 = ens_r2_floor(Gm);
+        S.xmax_bits = 0;
+    }
+    __syncthreads();
+    float xm = 0.f;
+    for (int i = t; i < n; i += T) {  // the thread's own rows, as it wrote them
+        const double4 p = pos[i];
+        xm = fmaxf(xm, fmaxf(fabsf((float)(p.x - S.o.cx)), fmaxf(fabsf((float)(p.y - S.o.cy)), fabsf((float)(p.z - S.o.cz)))));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) xm = fmaxf(xm, __shfl_xor_sync(0xffffffffu, xm, o));
+    if (lane == 0) atomicMax(&S.xmax_bits, __float_as_int(xm));
+    __syncthreads();
+    if (t == 0) {
+        // Bound on the FP32 error of a staged separation: each staged coordinate is within
+        // 2^-24 |X| of its FP64 value, so a separation is off by at most sqrt(3) 2^-23 xmax
+        // (plus its own relative rounding, covered by the factor on the reach); 2^-21 xmax
+        // keeps a factor 2 of room.  Every pair the FP64 overlap test would merge is flagged.
+        S.o.slack = __int_as_float(S.xmax_bits) * 0x1p-21f;
+        *out = S.o;
+    }
+    __syncthreads();
+}
+
+// Stages a system: FP32 relative positions and G m (padded to an even count, far and massless).
+__device__ __forceinline__ void ens_stage(int n, double G, const EnsInfo &f, const double4 *pos, float *sx, float *sy,
+                                          float *sz, float *sm) {
+    for (int i = threadIdx.x; i < ((n + 1) & ~1); i += blockDim.x) {
+        if (i < n) {
+            const double4 p = pos[i];
+            sx[i] = (float)(p.x - f.cx); sy[i] = (float)(p.y - f.cy); sz[i] = (float)(p.z - f.cz);
+            sm[i] = (float)(G * p.w);
+        } else {
+            sx[i] = 1e30f; sy[i] = 1e30f; sz[i] = 1e30f; sm[i] = 0.f;
+        }
+    }
+}
+
+// The opening half kick and drift (with pre) and the frame of every system.
+__global__ void ens_begin_kernel(EnsArgs a) {
+    __shared__ EnsBeginSmem S;
+    const int s = a.order[blockIdx.x];
+    const int64_t b0 = a.off[s];
+    ens_begin(a.cnt[s], a.G, a.h, a.pre, a.pos + b0, a.vel + b0, a.acc + b0, a.rad + b0, a.info + s, S);
+}
+
+// One launch = the force and closing half kick of one KDK step (or the initial force alone) for every
+// system, its merges and, with pre, the next step's opening half kick and drift.  IB bodies per thread
+// (1, 2 or 4; each staged j pair feeds IB bodies, dividing the shared-memory reads per interaction by IB).
 template <int IB>
 __global__ void __launch_bounds__(IB == 1 ? 512 : 256) ensemble_step_kernel(EnsArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -435,127 +565,70 @@ __global__ void __launch_bounds__(IB == 1 ? 512 : 256) ensemble_step_kernel(EnsA
     float *sy = sx + a.stride;
     float *sz = sy + a.stride;
     float *sm = sz + a.stride;
-    __shared__ double red[3][32];
-    __shared__ double cen[3];
-    __shared__ float redr[32], redg[32];
-    __shared__ int sh[8];
-    __shared__ float rmax_s, floor_s;
-    __shared__ int xmax_bits;  // largest staged |coordinate| (non-negative float bits)
-    __shared__ EnsCand cand;   // rows the separation test flagged
-    const int t = threadIdx.x, T = blockDim.x, lane = t & 31, warp = t >> 5, nw = (T + 31) >> 5;
-    const double h = a.h, h2 = 0.5 * a.h;
-    while (true) {
-        if (t == 0) sh[3] = (int)atomicAdd(&a.work[0], 1u);
+    __shared__ int sh[8], last_s;
+    __shared__ EnsCand cand;
+    __shared__ EnsBeginSmem S;
+    const int t = threadIdx.x, T = blockDim.x;
+    const double h2 = 0.5 * a.h;
+    const int2 item = a.items[blockIdx.x];
+    const int s = item.x;
+    const int64_t b0 = a.off[s];
+    double4 *pos = a.pos + b0, *vel = a.vel + b0, *acc = a.acc + b0;
+    double *rad = a.rad + b0;
+    int n = a.cnt[s];
+    // the rows of [row0, row1): each of the first sw threads (sw the smallest multiple of 32 with
+    // IB sw >= rows) takes t, t + sw, ...: threads hold IB valid rows except in the last warp, and whole
+    // warps past sw sit out
+    auto rows = [&](int row0, int row1, const EnsInfo &f, bool kick, EnsCand *list) {
+        const int sw = ((row1 - row0 + IB - 1) / IB + 31) & ~31;
+        if (t < sw)
+            ens_force_rows<IB>(row0 + t, sw, row1, (n + 1) & ~1, sx, sy, sz, sm, pos, vel, acc, rad, f.rmax, f.slack, kick,
+                               h2, f.floor2, list);
+    };
+    if (item.y < n) {
+        const EnsInfo f = a.info[s];
+        ens_stage(n, a.G, f, pos, sx, sy, sz, sm);
         __syncthreads();
-        const int item = sh[3];
+        rows(item.y, min(item.y + a.chunk, n), f, a.kick != 0, a.merge ? a.cand + s : nullptr);
+    }
+    // The last chunk of the system to get here finishes the step: everything the others wrote is visible
+    // to it (their fence and count, its count and fence).
+    __threadfence();
+    __syncthreads();
+    if (t == 0) {
+        const int chunks = (int)((a.off[s + 1] - b0 + a.chunk - 1) / a.chunk);
+        last_s = atomicAdd(&a.arrived[s], 1) == chunks - 1;
+    }
+    __syncthreads();
+    if (!last_s) return;
+    __threadfence();
+    if (t == 0) a.arrived[s] = 0;
+    const int listed = a.merge ? __ldcg(&a.cand[s].n) : 0;
+    if (listed) {
+        for (int k = t; k < min(listed, kEnsCand); k += T) cand.row[k] = __ldcg(&a.cand[s].row[k]);
+        if (t == 0) cand.n = listed;
         __syncthreads();
-        if (item >= a.n_sys) break;
-        const int s = a.order[item];
-        const int64_t b0 = a.off[s];
-        const int n = a.cnt[s];
-        double4 *pos = a.pos + b0, *vel = a.vel + b0, *acc = a.acc + b0;
-        double *rad = a.rad + b0;
-        // pass 0: kick-drift, force, kick, merge check; pass 1 (only after merges): the force at the
-        // merged state, so the next step's first half kick uses a(x) of the bodies that remain
-        int nc = n;
-        for (int pass = 0; pass < 2; ++pass) {
-            const bool first = pass == 0;
-            double cx = 0.0, cy = 0.0, cz = 0.0;
-            float rmax = 0.f, gmax = 0.f;
-            for (int i = t; i < nc; i += T) {
-                double4 p = pos[i];
-                if (a.kdk && first) {
-                    double4 v = vel[i];
-                    const double4 ac = acc[i];
-                    v.x = fma(h2, ac.x, v.x); v.y = fma(h2, ac.y, v.y); v.z = fma(h2, ac.z, v.z);
-                    p.x = fma(h, v.x, p.x); p.y = fma(h, v.y, p.y); p.z = fma(h, v.z, p.z);
-                    vel[i] = v;
-                    pos[i] = p;
-                }
-                cx += p.x; cy += p.y; cz += p.z;
-                rmax = fmaxf(rmax, (float)rad[i]);
-                gmax = fmaxf(gmax, (float)(a.G * p.w));
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                cx += __shfl_xor_sync(0xffffffffu, cx, o);
-                cy += __shfl_xor_sync(0xffffffffu, cy, o);
-                cz += __shfl_xor_sync(0xffffffffu, cz, o);
-                rmax = fmaxf(rmax, __shfl_xor_sync(0xffffffffu, rmax, o));
-                gmax = fmaxf(gmax, __shfl_xor_sync(0xffffffffu, gmax, o));
-            }
-            if (lane == 0) {
-                red[0][warp] = cx; red[1][warp] = cy; red[2][warp] = cz;
-                redr[warp] = rmax;
-                redg[warp] = gmax;
-            }
-            __syncthreads();
+        if (t == 0) a.cand[s].n = 0;
+        const int left = listed <= kEnsCand
+                             ? ens_merge_scan_cand(n, pos, vel, acc, rad, a.rest + b0, a.ids + b0, cand, sh)
+                             : ens_merge_scan(n, 0, false, pos, vel, acc, rad, a.rest + b0, a.ids + b0, sh);
+        if (left != n) {
             if (t == 0) {
-                double X = 0, Y = 0, Z = 0;
-                float R = 0.f, Gm = 0.f;
-                for (int w = 0; w < nw; ++w) {
-                    X += red[0][w]; Y += red[1][w]; Z += red[2][w];
-                    R = fmaxf(R, redr[w]);
-                    Gm = fmaxf(Gm, redg[w]);
-                }
-                cen[0] = X / nc; cen[1] = Y / nc; cen[2] = Z / nc;
-                rmax_s = R;
-                floor_s = ens_r2_floor(Gm);
-                xmax_bits = 0;
-                cand.n = 0;
+                a.cnt[s] = left;
+                atomicAdd(&a.work[1], (unsigned)(n - left));
             }
+            n = left;
+            // the force at the merged state, so the next step's first half kick uses a(x) of the bodies
+            // that remain
+            ens_begin(n, a.G, a.h, 0, pos, vel, acc, rad, a.info + s, S);
+            ens_stage(n, a.G, S.o, pos, sx, sy, sz, sm);
             __syncthreads();
-            const double mx = cen[0], my = cen[1], mz = cen[2];
-            const float rmx = rmax_s, floor2 = floor_s;
-            // stage the system: FP32 relative positions and G m (pad to an even count, far and massless)
-            const int npad = (nc + 1) & ~1;
-            float xm = 0.f;
-            for (int i = t; i < npad; i += T) {
-                if (i < nc) {
-                    const double4 p = pos[i];
-                    const float X = (float)(p.x - mx), Y = (float)(p.y - my), Z = (float)(p.z - mz);
-                    sx[i] = X; sy[i] = Y; sz[i] = Z;
-                    sm[i] = (float)(a.G * p.w);
-                    xm = fmaxf(xm, fmaxf(fabsf(X), fmaxf(fabsf(Y), fabsf(Z))));
-                } else {
-                    sx[i] = 1e30f; sy[i] = 1e30f; sz[i] = 1e30f; sm[i] = 0.f;
-                }
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) xm = fmaxf(xm, __shfl_xor_sync(0xffffffffu, xm, o));
-            if (lane == 0) atomicMax(&xmax_bits, __float_as_int(xm));
-            __syncthreads();
-            // Bound on the FP32 error of a staged separation: each staged coordinate is within
-            // 2^-24 |X| of its FP64 value, so a separation is off by at most sqrt(3) 2^-23 xmax
-            // (plus its own relative rounding, covered by the factor on the reach); 2^-21 xmax
-            // keeps a factor 2 of room.  Every pair the FP64 overlap test would merge is flagged.
-            const float slack = __int_as_float(xmax_bits) * 0x1p-21f;
-            // rows in passes of up to IB*T; a pass of c rows gives each of its first s threads (s the
-            // smallest multiple of 32 with IB*s >= c) the rows t, t + s, ...: threads hold IB valid
-            // rows except in the last warp, and whole warps past s sit the pass out
-            int flagged = 0;
-            for (int base = 0; base < nc; base += IB * T) {
-                const int c = min(IB * T, nc - base);
-                const int sw = ((c + IB - 1) / IB + 31) & ~31;
-                if (t < sw)
-                    flagged |= ens_force_rows<IB>(base + t, sw, nc, npad, sx, sy, sz, sm, pos, vel, acc, rad, rmx,
-                                                  slack, a.kdk && first, h2, floor2, cand);
-            }
-            flagged = __syncthreads_or(flagged);
-            if (!first || !flagged || !a.merge) break;
-            const int nn = cand.n <= kEnsCand
-                               ? ens_merge_scan_cand(nc, pos, vel, acc, rad, a.rest + b0, a.ids + b0, cand, sh)
-                               : ens_merge_scan(nc, 0, false, pos, vel, acc, rad, a.rest + b0, a.ids + b0, sh);
-            if (nn == nc) break;
-            if (t == 0) {
-                a.cnt[s] = nn;
-                atomicAdd(&a.work[1], (unsigned)(nc - nn));
-            }
-            nc = nn;
+            for (int base = 0; base < n; base += IB * T) rows(base, min(base + IB * T, n), S.o, false, nullptr);
+            __threadfence_block();
             __syncthreads();
         }
-        __syncthreads();
     }
+    if (a.pre) ens_begin(n, a.G, a.h, 1, pos, vel, acc, rad, a.info + s, S);
 }
 
 // The kernel for ib bodies per thread (1, 2 or 4).
@@ -573,43 +646,92 @@ int ens_smem_bytes(int max_n) { return 4 * ens_stride(max_n) * (int)sizeof(float
 
 using namespace gtd;
 
+static void ens_release_graph(gtd_ensemble *e);
+
 static void ens_release(gtd_ensemble *e) {
-    if (e->graph) cudaGraphExecDestroy(e->graph);
-    e->graph = nullptr;
+    ens_release_graph(e);
+    cudaFree(e->items); cudaFree(e->cand); cudaFree(e->info); cudaFree(e->arrived);
+    e->items = nullptr; e->cand = nullptr; e->info = nullptr; e->arrived = nullptr;
+    e->items_for = 0;
     cudaFree(e->off); cudaFree(e->cnt); cudaFree(e->order); cudaFree(e->pos); cudaFree(e->vel); cudaFree(e->acc);
     cudaFree(e->rad); cudaFree(e->rest); cudaFree(e->ids); cudaFree(e->work); cudaFree(e->status);
     e->off = nullptr; e->cnt = nullptr; e->order = nullptr; e->pos = e->vel = e->acc = nullptr;
     e->rad = e->rest = nullptr; e->ids = nullptr; e->work = nullptr; e->status = nullptr;
 }
 
-static int ens_launch(gtd_ensemble *e, int kdk) {
-    EnsArgs a{(int)e->n_sys, e->off, e->cnt, e->order, e->pos, e->vel, e->acc, e->rad, e->rest, e->ids,
-              e->G, e->dt, kdk, e->merge, ens_stride(e->max_n), e->work, e->status};
-    const int smem = ens_smem_bytes(e->max_n);
-    int dev_sms = 148;
-    cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, e->device);
-    int per_sm = 1;
-    with_ens_kernel(e->ib, [&](auto k) { cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, e->threads, smem); });
-    if (per_sm < 1) per_sm = 1;
-    const int grid = (int)std::min<int64_t>((int64_t)dev_sms * per_sm, std::max<int64_t>(e->n_sys, 1));
-    GTD_CUDA(cudaMemsetAsync(e->work, 0, sizeof(unsigned), e->stream));
-    with_ens_kernel(e->ib, [&](auto k) { k<<<grid, e->threads, smem, e->stream>>>(a); });
+static EnsArgs ens_args(const gtd_ensemble *e, int kick, int pre) {
+    return EnsArgs{e->off, e->cnt, e->order, e->items, e->pos, e->vel, e->acc, e->rad, e->rest, e->ids, e->cand, e->info,
+                   e->arrived, e->G, e->dt, kick, pre, e->merge, e->threads * e->ib, ens_stride(e->max_n), e->work};
+}
+
+static void ens_release_graph(gtd_ensemble *e) {
+    if (e->graph) cudaGraphExecDestroy(e->graph);
+    e->graph = nullptr;
+}
+
+// CTA size and bodies per thread for an ensemble nobody configured.  128 threads: the smallest items,
+// for balance and latency, unless systems are so large that staging them for 128 or 256 rows shows.  Two
+// bodies per thread (fewer shared-memory reads) once that still leaves two rounds of CTAs, 4 per SM.
+// Steps in us on B200, 128 x 1 / 128 x 2 / 256 x 1: 4096 systems of up to 2048 bodies 3012 / 2763 / 3106,
+// 512 of them 395 / 376 / 402, 128 of them 125 / 140 / 127, 512 of up to 256 19 / 22 / 22, 8 of up to 8192
+// 446 / 395 / 350.
+static void ens_default(gtd_ensemble *e) {
+    e->threads = e->max_n > 4096 ? 256 : 128;
+    int64_t items = 0;
+    for (int64_t s = 0; s < e->n_sys; ++s) {
+        const int64_t n = e->off_h[(size_t)s + 1] - e->off_h[(size_t)s];
+        items += (n + 2 * e->threads - 1) / (2 * e->threads);
+    }
+    e->ib = items >= 8 * 148 ? 2 : 1;
+}
+
+// The items for the present CTA size and bodies per thread.
+static int ens_prepare(gtd_ensemble *e) {
+    const int key = e->threads * 4 + e->ib;
+    if (e->items_for == key) return GTD_OK;
+    ens_release_graph(e);
+    const int chunk = e->threads * e->ib;
+    std::vector<int2> items;
+    for (int32_t s : e->order_h)
+        for (int64_t r = 0; r < e->off_h[(size_t)s + 1] - e->off_h[(size_t)s]; r += chunk)
+            items.push_back(make_int2(s, (int)r));
+    GTD_CUDA(cudaStreamSynchronize(e->stream));  // no launch reads the old items any more
+    cudaFree(e->items);
+    e->items = nullptr;
+    e->items_for = 0;
+    GTD_CUDA(cudaMalloc(&e->items, sizeof(int2) * std::max<size_t>(items.size(), 1)));
+    GTD_CUDA(cudaMemcpy(e->items, items.data(), sizeof(int2) * items.size(), cudaMemcpyHostToDevice));
+    e->n_items = (int64_t)items.size();
+    e->items_for = key;
+    return GTD_OK;
+}
+
+static int ens_open(gtd_ensemble *e, int pre) {
+    ens_begin_kernel<<<(unsigned)e->n_sys, 256, 0, e->stream>>>(ens_args(e, 0, pre));
     GTD_CHECK_LAUNCH();
+    return GTD_OK;
+}
+
+static int ens_launch(gtd_ensemble *e, int kick, int pre) {
+    if (e->n_items > 0) {
+        const EnsArgs a = ens_args(e, kick, pre);
+        with_ens_kernel(e->ib, [&](auto k) {
+            k<<<(unsigned)e->n_items, e->threads, ens_smem_bytes(e->max_n), e->stream>>>(a);
+        });
+        GTD_CHECK_LAUNCH();
+    }
     e->launches += 1;
     return GTD_OK;
 }
 
-// Captures `steps` KDK steps (a memset and one persistent launch each) into a CUDA graph.
+// Captures `steps` KDK steps, each opening the next, into a CUDA graph.
 static int ens_build_graph(gtd_ensemble *e, int steps) {
-    if (e->graph) {
-        cudaGraphExecDestroy(e->graph);
-        e->graph = nullptr;
-    }
+    ens_release_graph(e);
     cudaGraph_t g;
     GTD_CUDA(cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal));
     int rc = GTD_OK;
     const uint64_t before = e->launches;
-    for (int k = 0; k < steps && !rc; ++k) rc = ens_launch(e, 1);
+    for (int k = 0; k < steps && !rc; ++k) rc = ens_launch(e, 1, 1);
     cudaError_t ce = cudaStreamEndCapture(e->stream, &g);
     e->launches = before;  // captured, not launched
     if (rc) return rc;
@@ -623,25 +745,30 @@ static int ens_build_graph(gtd_ensemble *e, int steps) {
 }
 
 static int ens_steps(gtd_ensemble *e, uint64_t steps) {
+    int rc = ens_prepare(e);
+    if (rc) return rc;
     if (!e->begun) {
-        int rc = ens_launch(e, 0);  // initial accelerations (and add-time merges)
+        rc = ens_open(e, 0);
+        if (!rc) rc = ens_launch(e, 0, 1);  // initial accelerations (and add-time merges)
         if (rc) return rc;
         e->begun = true;
+    } else if ((rc = ens_open(e, 1))) {
+        return rc;
     }
     const int chunk = 16;
-    if (steps >= (uint64_t)chunk) {
+    if (steps > (uint64_t)chunk) {  // the last step does not open another
         if (!e->graph || e->graph_steps != chunk || e->graph_threads != e->threads * 4 + e->ib) {
-            int rc = ens_build_graph(e, chunk);
+            rc = ens_build_graph(e, chunk);
             if (rc) return rc;
         }
-        while (steps >= (uint64_t)chunk) {
+        while (steps > (uint64_t)chunk) {
             GTD_CUDA(cudaGraphLaunch(e->graph, e->stream));
             e->launches += chunk;
             steps -= chunk;
         }
     }
     for (uint64_t k = 0; k < steps; ++k) {
-        int rc = ens_launch(e, 1);
+        rc = ens_launch(e, 1, k + 1 < steps ? 1 : 0);
         if (rc) return rc;
     }
     return GTD_OK;
@@ -694,10 +821,7 @@ int gtd_ensemble_set_params(gtd_ensemble *e, double G, double dt, int merge) {
     e->G = G;
     e->dt = dt;
     e->merge = merge ? 1 : 0;
-    if (e->graph) {
-        cudaGraphExecDestroy(e->graph);
-        e->graph = nullptr;
-    }
+    ens_release_graph(e);
     return GTD_OK;
 }
 
@@ -713,7 +837,9 @@ int gtd_ensemble_upload(gtd_ensemble *e, int64_t n_systems, const int64_t *offse
     const int64_t nb = n_systems ? offsets[n_systems] : 0;
     e->n_bodies = nb;
     e->max_n = 0;
-    std::vector<int32_t> cnt((size_t)n_systems), order((size_t)n_systems);
+    std::vector<int32_t> cnt((size_t)n_systems);
+    std::vector<int32_t> &order = e->order_h;
+    order.assign((size_t)n_systems, 0);
     for (int64_t s = 0; s < n_systems; ++s) {
         const int64_t k = offsets[s + 1] - offsets[s];
         if (k < 0 || offsets[s] < 0) return fail(GTD_ERR_INVALID_ARGUMENT, "offsets must be non-decreasing from 0");
@@ -748,6 +874,12 @@ int gtd_ensemble_upload(gtd_ensemble *e, int64_t n_systems, const int64_t *offse
     GTD_CUDA(cudaMalloc(&e->ids, sizeof(int32_t) * (size_t)std::max<int64_t>(nb, 1)));
     GTD_CUDA(cudaMalloc(&e->work, 4 * sizeof(unsigned)));
     GTD_CUDA(cudaMalloc(&e->status, sizeof(int)));
+    const size_t ns = (size_t)std::max<int64_t>(n_systems, 1);
+    GTD_CUDA(cudaMalloc(&e->cand, sizeof(EnsCand) * ns));
+    GTD_CUDA(cudaMalloc(&e->info, sizeof(EnsInfo) * ns));
+    GTD_CUDA(cudaMalloc(&e->arrived, sizeof(int) * ns));
+    GTD_CUDA(cudaMemset(e->cand, 0, sizeof(EnsCand) * ns));
+    GTD_CUDA(cudaMemset(e->arrived, 0, sizeof(int) * ns));
     GTD_CUDA(cudaMemcpy(e->off, offsets, sizeof(int64_t) * (size_t)(n_systems + 1), cudaMemcpyHostToDevice));
     if (n_systems) {
         GTD_CUDA(cudaMemcpy(e->cnt, cnt.data(), sizeof(int32_t) * cnt.size(), cudaMemcpyHostToDevice));
@@ -764,6 +896,7 @@ int gtd_ensemble_upload(gtd_ensemble *e, int64_t n_systems, const int64_t *offse
     GTD_CUDA(cudaMemset(e->work, 0, 4 * sizeof(unsigned)));
     GTD_CUDA(cudaMemset(e->status, 0, sizeof(int)));
     e->begun = false;
+    if (!e->configured) ens_default(e);
     return GTD_OK;
 }
 
@@ -830,8 +963,9 @@ int gtd_ensemble_set_threads(gtd_ensemble *e, int threads) {
     if (!e) return fail(GTD_ERR_INVALID_ARGUMENT, "ensemble is NULL");
     if (threads != 64 && threads != 128 && threads != 256 && threads != 512)
         return fail(GTD_ERR_INVALID_ARGUMENT, "threads must be 64, 128, 256 or 512");
-    if (e->ib > 1 && threads > 256) e->ib = 1;
+    if (!e->configured || (e->ib > 1 && threads > 256)) e->ib = 1;
     e->threads = threads;
+    e->configured = true;
     return GTD_OK;
 }
 
@@ -841,7 +975,9 @@ int gtd_ensemble_set_bodies_per_thread(gtd_ensemble *e, int bodies) {
         return fail(GTD_ERR_INVALID_ARGUMENT, "bodies per thread must be 1, 2 or 4");
     if (bodies > 1 && e->threads > 256)
         return fail(GTD_ERR_INVALID_ARGUMENT, "%d bodies per thread need a CTA of at most 256 threads", bodies);
+    if (!e->configured) e->threads = 256;
     e->ib = bodies;
+    e->configured = true;
     return GTD_OK;
 }
 
@@ -904,8 +1040,10 @@ int gtd_ensemble_autotune(gtd_ensemble *e, int *best_threads, double *best_ms) {
         for (int k = 0; k < kCands && !rc; ++k) {
             e->threads = cands[k][0];
             e->ib = cands[k][1];
+            if ((rc = ens_prepare(e))) break;
             if ((rc = cudaEventRecord(e->ev0, e->stream) ? GTD_ERR_CUDA : GTD_OK)) break;
-            for (int q = 0; q < kTuneSteps && !rc; ++q) rc = ens_launch(e, 1);
+            rc = ens_open(e, 1);
+            for (int q = 0; q < kTuneSteps && !rc; ++q) rc = ens_launch(e, 1, q + 1 < kTuneSteps ? 1 : 0);
             if (rc) break;
             cudaEventRecord(e->ev1, e->stream);
             cudaEventSynchronize(e->ev1);
@@ -932,6 +1070,7 @@ int gtd_ensemble_autotune(gtd_ensemble *e, int *best_threads, double *best_ms) {
         }
     e->threads = best;
     e->ib = best_ib;
+    e->configured = true;
     e->begun = was_begun;
     GTD_CUDA(cudaStreamSynchronize(e->stream));
     GTD_CUDA(cudaMemset(e->work, 0, 4 * sizeof(unsigned)));

@@ -350,7 +350,8 @@ GTD_API int gtd_ensemble_upload(gtd_ensemble *ens, int64_t n_systems, const int6
                                 const double *r, const double *rest, const double *x3, const double *v3);
 /* Advances every system `steps` KDK steps; *elapsed_ns is the device time (CUDA events). */
 GTD_API int gtd_ensemble_evolve(gtd_ensemble *ens, uint64_t steps, int64_t *elapsed_ns);
-/* Live bodies per system (counts[n_systems]), merges so far, kernel launches so far. */
+/* Live bodies per system (counts[n_systems]), merges so far, step-kernel launches so far (one per step and
+ * one for the initial force). */
 GTD_API int gtd_ensemble_counts(gtd_ensemble *ens, int64_t *counts, uint64_t *merges, uint64_t *launches);
 /* State at the upload offsets: system s's survivors occupy the first counts[s] rows of its range,
  * in upload order. */
