@@ -444,11 +444,14 @@ int variant_count(int precision) { return precision == GTD_PREC_MIXED ? kNumMixe
 // Variant for a handle nobody tuned: the unordered-pair kernels (direct_sym.cu), per step on B200
 //   mixed   N = 8192 65 us (ordered pairs 75), 16384 162 (192), 65536 1.59 ms (2.32), 262144 21.8 ms (29.3)
 //   FP64    N = 4500 35 us (39), 8192 68 (92), 16384 212 (295), 65536 2.95 ms (4.33)
+// but FP64 systems of up to 17 rows and tiles of 256 bodies, whose 289 ordered tiles all run at once, one
+// per CTA: N = 4200 29 us against 35.
 // From N = 32768 the mixed kernel folds its FP32 sums half as often: 3 % faster, and its rounding
 // (RMS 3.8e-8 of a body's acceleration at N = 262144 against 3.2e-8) is still that of the ordered
 // kernel's fold of 128 (4.0e-8).  FP64 systems up to kFusedMaxN bodies take the fused kernel instead.
 int default_variant(int precision, int64_t n) {
     if (precision == GTD_PREC_MIXED) return n >= 32768 ? 9 : 10;
+    if (n <= 17 * 256) return 1;
     return n <= 32768 ? 5 : 6;
 }
 
@@ -681,64 +684,105 @@ __global__ void integrate_warp_kernel(IntArgs a) {
     if (lane == 0) apply_epilogue(a.st, a.epi, i, ax, ay, az);
 }
 
-// Small FP64 systems, one launch per force evaluation.  kFusedSlices warps share a body: warp s sums
+// Small FP64 systems, one launch per force evaluation.  kFusedSlices warps share I bodies: warp s sums
 // the j in the 32-wide chunks s, s + S, s + 2S, ... (loads straight from the L1/L2-resident
-// positions, several in flight), reduces with shuffles, and the body's first warp adds the slices
+// positions, several in flight), reduces with shuffles, and the bodies' first warp adds the slices
 // in order and applies the method's update.  No partial sums in memory, no second kernel; the short
-// per-warp loops keep the latency of a step low when there are few bodies.
-constexpr int kFusedBodies = 4;  // bodies per CTA
-constexpr int kFusedSlices = 4;  // warps per body
+// per-warp loops keep the latency of a step low when there are few bodies.  The update is a template
+// argument: as a switch in the kernel its registers slowed every method by 4 to 13 %.
+// I, the bodies a warp shares its loads between, grows with the system: at one body a chunk's loads take as
+// many L1 cycles as its arithmetic takes FP64 cycles (8 each), and the CTAs should fit the GPU at once -
+// past that the step takes the time of two rounds.  Shapes {bodies per warp, groups per CTA, CTAs per SM}
+// and the bodies a round holds on 148 SMs: {1, 2, 4} 1184, {2, 1, 5} 1480, {2, 1, 8} 2368, {4, 2, 3} 3552;
+// larger systems take {2, 1, 8} again, whose rounds are short.  Microseconds a step on B200, with
+// one body per warp and four groups per CTA throughout / with these:
+//   N = 150 2.72 / 2.47, 592 3.37 / 3.37, 727 4.39 / 3.9, 1024 5.04 / 4.77, 1300 7.75 / 5.62, 2000 12.7 / 8.8,
+//   3000 24.0 / 18.0, 4096 35.2 / 25.3
+constexpr int kFusedSlices = 4;  // warps per group
 
-__global__ void __launch_bounds__(kFusedBodies * kFusedSlices * 32)
-    fused_small_kernel(IntArgs a, const double4 *__restrict__ src, double G) {
-    __shared__ double part[kFusedSlices][kFusedBodies][3];
+template <int EPI, int I, int kFusedGroups, int MINB>
+__global__ void __launch_bounds__(kFusedGroups * kFusedSlices * 32, MINB)
+    fused_small_kernel(StepArgs st, const double4 *__restrict__ src, double G) {
+    __shared__ double part[kFusedSlices][kFusedGroups][I][3];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int bl = w % kFusedBodies, slice = w / kFusedBodies;
-    const int64_t i = (int64_t)blockIdx.x * kFusedBodies + bl;
-    double ax = 0.0, ay = 0.0, az = 0.0;
-    if (i < a.n) {
-        const double4 p = src[i];
+    const int bl = w % kFusedGroups, slice = w / kFusedGroups;
+    const int64_t i0 = ((int64_t)blockIdx.x * kFusedGroups + bl) * I;
+    double4 p[I];
+    double ax[I], ay[I], az[I];
+#pragma unroll
+    for (int k = 0; k < I; ++k) {  // a missing body stands at the origin; its sums are dropped
+        p[k] = i0 + k < st.n ? src[i0 + k] : make_double4(0.0, 0.0, 0.0, 0.0);
+        ax[k] = ay[k] = az[k] = 0.0;
+    }
+    if (i0 < st.n) {
 #pragma unroll 4
-        for (int64_t j = (int64_t)slice * 32 + lane; j < a.n; j += 32 * kFusedSlices) {
+        for (int64_t j = (int64_t)slice * 32 + lane; j < st.n; j += 32 * kFusedSlices) {
             const double4 q = src[j];
             const double gm = q.w * G;
-            const double dx = q.x - p.x, dy = q.y - p.y, dz = q.z - p.z;
-            const double r2 = fma(dz, dz, fma(dy, dy, dx * dx));
-            const double sc = r2 > 0.0 ? gm * inv_r3(r2) : 0.0;
-            ax = fma(sc, dx, ax);
-            ay = fma(sc, dy, ay);
-            az = fma(sc, dz, az);
+#pragma unroll
+            for (int k = 0; k < I; ++k) {
+                const double dx = q.x - p[k].x, dy = q.y - p[k].y, dz = q.z - p[k].z;
+                const double r2 = fma(dz, dz, fma(dy, dy, dx * dx));
+                const double sc = r2 > 0.0 ? gm * inv_r3(r2) : 0.0;
+                ax[k] = fma(sc, dx, ax[k]);
+                ay[k] = fma(sc, dy, ay[k]);
+                az[k] = fma(sc, dz, az[k]);
+            }
         }
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        ax += __shfl_xor_sync(0xffffffffu, ax, o);
-        ay += __shfl_xor_sync(0xffffffffu, ay, o);
-        az += __shfl_xor_sync(0xffffffffu, az, o);
-    }
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int k = 0; k < I; ++k) {
+            ax[k] += __shfl_xor_sync(0xffffffffu, ax[k], o);
+            ay[k] += __shfl_xor_sync(0xffffffffu, ay[k], o);
+            az[k] += __shfl_xor_sync(0xffffffffu, az[k], o);
+        }
     if (lane == 0) {
-        part[slice][bl][0] = ax;
-        part[slice][bl][1] = ay;
-        part[slice][bl][2] = az;
+#pragma unroll
+        for (int k = 0; k < I; ++k) {
+            part[slice][bl][k][0] = ax[k];
+            part[slice][bl][k][1] = ay[k];
+            part[slice][bl][k][2] = az[k];
+        }
     }
     __syncthreads();
-    if (slice == 0 && lane == 0 && i < a.n) {
-        double sx = part[0][bl][0], sy = part[0][bl][1], sz = part[0][bl][2];
+    if (slice == 0 && lane < I && i0 + lane < st.n) {
+        double s[3];
 #pragma unroll
-        for (int k = 1; k < kFusedSlices; ++k) {
-            sx += part[k][bl][0];
-            sy += part[k][bl][1];
-            sz += part[k][bl][2];
+        for (int d = 0; d < 3; ++d) {
+            s[d] = part[0][bl][lane][d];
+#pragma unroll
+            for (int k = 1; k < kFusedSlices; ++k) s[d] += part[k][bl][lane][d];
         }
-        apply_epilogue(a.st, a.epi, i, sx, sy, sz);
+        apply_epilogue(st, EPI, i0 + lane, s[0], s[1], s[2]);
+    }
+}
+
+template <int I, int GROUPS, int MINB>
+static void launch_fused(int64_t n, const double4 *src, double G, int epi, const StepArgs &st, cudaStream_t s) {
+    const unsigned grid = (unsigned)((n + GROUPS * I - 1) / (GROUPS * I));
+    auto go = [&](auto k) { k<<<grid, GROUPS * kFusedSlices * 32, 0, s>>>(st, src, G); };
+    switch (epi) {
+        case EPI_ACC: go(fused_small_kernel<EPI_ACC, I, GROUPS, MINB>); break;
+        case EPI_KDK: go(fused_small_kernel<EPI_KDK, I, GROUPS, MINB>); break;
+        case EPI_DKD: go(fused_small_kernel<EPI_DKD, I, GROUPS, MINB>); break;
+        case EPI_EULER: go(fused_small_kernel<EPI_EULER, I, GROUPS, MINB>); break;
+        case EPI_PREDICT: go(fused_small_kernel<EPI_PREDICT, I, GROUPS, MINB>); break;
+        case EPI_CORR_MEULER: go(fused_small_kernel<EPI_CORR_MEULER, I, GROUPS, MINB>); break;
+        case EPI_CORR_MIDPOINT: go(fused_small_kernel<EPI_CORR_MIDPOINT, I, GROUPS, MINB>); break;
+        case EPI_ACC3: go(fused_small_kernel<EPI_ACC3, I, GROUPS, MINB>); break;
+        default: go(fused_small_kernel<EPI_KICK_DRIFT, I, GROUPS, MINB>); break;
     }
 }
 
 int launch_fused_small(int64_t n, const double4 *src, double G, int epi, const StepArgs &st, cudaStream_t s) {
     if (n == 0) return GTD_OK;
-    IntArgs a{n, 0, 0, 0, 0, epi, nullptr, st, 0};
-    fused_small_kernel<<<(unsigned)((n + kFusedBodies - 1) / kFusedBodies), kFusedBodies * kFusedSlices * 32, 0, s>>>(
-        a, src, G);
+    if (n <= 900) launch_fused<1, 2, 4>(n, src, G, epi, st, s);
+    else if (n <= 5 * 148 * 2) launch_fused<2, 1, 5>(n, src, G, epi, st, s);
+    else if (n <= 8 * 148 * 2) launch_fused<2, 1, 8>(n, src, G, epi, st, s);
+    else if (n <= 3 * 148 * 8) launch_fused<4, 2, 3>(n, src, G, epi, st, s);
+    else launch_fused<2, 1, 8>(n, src, G, epi, st, s);
     GTD_CHECK_LAUNCH();
     return GTD_OK;
 }

@@ -81,3 +81,20 @@ def test_noalloc_paths(gpu, n, precision):
         assert rel.max() < 1e-12, rel.max()
     else:
         assert np.sqrt((rel ** 2).mean()) < 1e-6, rel.max()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [2, 3, 900, 901, 1480, 1481, 2368, 2369, 3551, 3552, 3553, 4095])
+def test_fused_shapes(gpu, n):
+    """Every launch shape of the fused FP64 kernel at its boundary, odd counts included, under a two-stage
+    method: the positions and velocities of one modified Euler step from host sums (FP64, 1e-12)."""
+    m, x, v = plummer(n, n)
+    x[n - 1] = x[0]  # coincident: no pair
+    h = 3600.0
+    a, _ = _host_acc(m, x)
+    xp, vp = x + h * v, v + h * a
+    ap, _ = _host_acc(m, xp)
+    s = System(m, x, v, timestep=h, num_iterations=1, units_format=UNITS_G6674)
+    s.evolve(System.modified_euler)
+    for got, want in ((s.x, x + 0.5 * h * (v + vp)), (s.v, v + 0.5 * h * (a + ap)), (s.a, a)):
+        assert np.abs(got - want).max() <= 1e-12 * np.abs(want).max()
