@@ -246,49 +246,68 @@ struct VjpUpdate {
 // Small systems: VJP and update in one launch, as fused_small_kernel (direct.cu) does force and step.
 // kVjpSlices warps share a body, their lanes take the ordered pairs of every 32 kVjpSlices-th partner
 // straight from L1 / L2, and the body's first warp adds the slices in order.
-constexpr int kVjpBodies = 4, kVjpSlices = 4;
+constexpr int kVjpSlices = 4;
 
-__global__ void __launch_bounds__(kVjpBodies * kVjpSlices * 32)
+template <int I, int GROUPS, int MINB>
+__global__ void __launch_bounds__(GROUPS * kVjpSlices * 32, MINB)
     vjp_small_kernel(int64_t n, const double4 *__restrict__ x, const double4 *__restrict__ w, VjpUpdate up) {
-    __shared__ double part[kVjpSlices][kVjpBodies][4];
+    __shared__ double part[kVjpSlices][GROUPS][I][4];
     const int wp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int bl = wp % kVjpBodies, slice = wp / kVjpBodies;
-    const int64_t i = (int64_t)blockIdx.x * kVjpBodies + bl;
-    VjpSums s, none;
-    s.clear();
-    if (i < n) {
-        const double4 xk = x[i], wk = w[i];
-        const double m3 = 3.0 * xk.w;
+    const int bl = wp % GROUPS, slice = wp / GROUPS;
+    const int64_t i0 = ((int64_t)blockIdx.x * GROUPS + bl) * I;
+    double4 xk[I], wk[I];
+    VjpSums s[I], none;
+#pragma unroll
+    for (int k = 0; k < I; ++k) {
+        xk[k] = i0 + k < n ? x[i0 + k] : make_double4(0.0, 0.0, 0.0, 0.0);
+        wk[k] = i0 + k < n ? w[i0 + k] : make_double4(0.0, 0.0, 0.0, 0.0);
+        s[k].clear();
+    }
+    if (i0 < n) {
 #pragma unroll 2
         for (int64_t j = (int64_t)slice * 32 + lane; j < n; j += 32 * kVjpSlices) {
             const double4 xj = x[j], wj = w[j];
-            vjp_pair<false, true>(xk, wk, m3, xj.x, xj.y, xj.z, xj.w, wj.x, wj.y, wj.z, 3.0 * xj.w, s, none);
+#pragma unroll
+            for (int k = 0; k < I; ++k)
+                vjp_pair<false, true>(xk[k], wk[k], 3.0 * xk[k].w, xj.x, xj.y, xj.z, xj.w, wj.x, wj.y, wj.z, 3.0 * xj.w, s[k],
+                                      none);
         }
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
-        s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
-        s.z += __shfl_xor_sync(0xffffffffu, s.z, o);
-        s.m += __shfl_xor_sync(0xffffffffu, s.m, o);
-    }
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int k = 0; k < I; ++k) {
+            s[k].x += __shfl_xor_sync(0xffffffffu, s[k].x, o);
+            s[k].y += __shfl_xor_sync(0xffffffffu, s[k].y, o);
+            s[k].z += __shfl_xor_sync(0xffffffffu, s[k].z, o);
+            s[k].m += __shfl_xor_sync(0xffffffffu, s[k].m, o);
+        }
     if (lane == 0) {
-        part[slice][bl][0] = s.x;
-        part[slice][bl][1] = s.y;
-        part[slice][bl][2] = s.z;
-        part[slice][bl][3] = s.m;
+#pragma unroll
+        for (int k = 0; k < I; ++k) {
+            part[slice][bl][k][0] = s[k].x;
+            part[slice][bl][k][1] = s[k].y;
+            part[slice][bl][k][2] = s[k].z;
+            part[slice][bl][k][3] = s[k].m;
+        }
     }
     __syncthreads();
-    if (slice == 0 && lane == 0 && i < n) {
+    if (slice == 0 && lane < I && i0 + lane < n) {
         double v[4];
 #pragma unroll
         for (int d = 0; d < 4; ++d) {
-            v[d] = part[0][bl][d];
+            v[d] = part[0][bl][lane][d];
 #pragma unroll
-            for (int k = 1; k < kVjpSlices; ++k) v[d] += part[k][bl][d];
+            for (int k = 1; k < kVjpSlices; ++k) v[d] += part[k][bl][lane][d];
         }
-        up.apply(i, v[0], v[1], v[2], v[3]);
+        up.apply(i0 + lane, v[0], v[1], v[2], v[3]);
     }
+}
+
+template <int I, int GROUPS, int MINB>
+static void launch_vjp_small(int64_t n, const double4 *x, const double4 *w, const VjpUpdate &up, cudaStream_t st) {
+    vjp_small_kernel<I, GROUPS, MINB><<<(unsigned)((n + GROUPS * I - 1) / (GROUPS * I)), GROUPS * kVjpSlices * 32, 0, st>>>(
+        n, x, w, up);
 }
 
 __global__ void __launch_bounds__(kRedWarps * 32) vjp_reduce_kernel(SymSlots s, double *base_out, VjpUpdate up) {
@@ -366,9 +385,9 @@ static unsigned g1(int64_t n) { return (unsigned)((n + 255) / 256); }
 
 // Bytes of positions that the forward keeps rather than recompute them: 16384 bodies over 2000 steps.
 constexpr size_t kKeepBytes = (size_t)5 << 28;
-// Up to this many bodies a VJP and its update run as one launch: per step 25 us at N = 2048 (31 in the
-// blocked form), 33 at 2500 (33), 46 at 3000 (40).
-constexpr int64_t kVjpSmallMaxN = 2048;
+// Up to this many bodies a VJP and its update run as one launch: 17 us a step at N = 2048 (31 in the
+// blocked form), 31 at 3000 (40), 39 at 3500 (41).
+constexpr int64_t kVjpSmallMaxN = 3400;
 
 // Fills the plan and lays the buffers out from `base` (sizes only where base is NULL); the bytes they take.
 static size_t adj_layout(gtd_adjoint *A, char *base) {
@@ -452,8 +471,10 @@ static int adj_vjp(gtd_adjoint *A, const double4 *x, uint64_t k, int &cur, cudaS
     const double4 *w = A->w[cur];
     cur ^= 1;
     if (A->small_vjp) {
-        vjp_small_kernel<<<(unsigned)((A->n + kVjpBodies - 1) / kVjpBodies), kVjpBodies * kVjpSlices * 32, 0, st>>>(
-            A->n, x, w, up);
+        // bodies per warp, groups per CTA and CTAs per SM as in launch_fused_small
+        if (A->n <= 1000) launch_vjp_small<1, 1, 8>(A->n, x, w, up, st);
+        else if (A->n <= 5 * 148 * 2) launch_vjp_small<2, 1, 5>(A->n, x, w, up, st);
+        else launch_vjp_small<2, 1, 4>(A->n, x, w, up, st);
         GTD_CHECK_LAUNCH();
         A->launches += 1;
         return GTD_OK;
