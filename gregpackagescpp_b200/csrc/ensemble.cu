@@ -27,6 +27,7 @@
 #include <vector>
 
 #include "gtd_internal.cuh"
+#include "host_copy.cuh"
 
 namespace gtd {
 struct EnsCand;
@@ -60,6 +61,8 @@ struct gtd_ensemble {
     int64_t n_items = 0;
     int items_for = 0;                // the (threads, ib) the items were made for
     int *status = nullptr;
+    double *io = nullptr;             // host arrays on the device: x3 | v3 | a3 | m | r | rest
+    gtd::HostRing host_ring;
     bool begun = false;
     uint64_t launches = 0;
     cudaGraphExec_t graph = nullptr;
@@ -631,6 +634,35 @@ __global__ void __launch_bounds__(IB == 1 ? 512 : 256) ensemble_step_kernel(EnsA
     if (a.pre) ens_begin(n, a.G, a.h, 1, pos, vel, acc, rad, a.info + s, S);
 }
 
+// Host layout (x3 | v3 | a3 | m | r | rest, nb bodies) to the device arrays and back.
+__global__ void ens_pack_kernel(const int64_t *off, int64_t nb, const double *io, int has_v, int has_r, int has_rest,
+                                double4 *pos, double4 *vel, double4 *acc, double *rad, double *rest, int32_t *ids) {
+    const double *x3 = io, *v3 = io + 3 * nb, *m = io + 9 * nb, *r = io + 10 * nb, *e = io + 11 * nb;
+    const int64_t b = off[blockIdx.x];
+    for (int64_t i = b + threadIdx.x; i < off[blockIdx.x + 1]; i += blockDim.x) {
+        pos[i] = make_double4(x3[3 * i], x3[3 * i + 1], x3[3 * i + 2], m[i]);
+        vel[i] = has_v ? make_double4(v3[3 * i], v3[3 * i + 1], v3[3 * i + 2], 0.0) : make_double4(0, 0, 0, 0);
+        acc[i] = make_double4(0, 0, 0, 0);
+        rad[i] = has_r ? r[i] : 0.0;
+        rest[i] = has_rest ? e[i] : 1.0;
+        ids[i] = (int32_t)(i - b);
+    }
+}
+
+__global__ void ens_unpack_kernel(int64_t nb, const double4 *pos, const double4 *vel, const double4 *acc, const double *rad,
+                                  const double *rest, double *io) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= nb) return;
+    double *x3 = io, *v3 = io + 3 * nb, *a3 = io + 6 * nb;
+    const double4 p = pos[i], v = vel[i], a = acc[i];
+    x3[3 * i] = p.x; x3[3 * i + 1] = p.y; x3[3 * i + 2] = p.z;
+    v3[3 * i] = v.x; v3[3 * i + 1] = v.y; v3[3 * i + 2] = v.z;
+    a3[3 * i] = a.x; a3[3 * i + 1] = a.y; a3[3 * i + 2] = a.z;
+    io[9 * nb + i] = p.w;
+    io[10 * nb + i] = rad[i];
+    io[11 * nb + i] = rest[i];
+}
+
 // The kernel for ib bodies per thread (1, 2 or 4).
 template <typename F>
 void with_ens_kernel(int ib, F &&f) {
@@ -646,6 +678,22 @@ int ens_smem_bytes(int max_n) { return 4 * ens_stride(max_n) * (int)sizeof(float
 
 using namespace gtd;
 
+static std::vector<HostSpan> ens_spans(const gtd_ensemble *e, const double *m, const double *r, const double *rest,
+                                       const double *x3, const double *v3, const double *a3) {
+    std::vector<HostSpan> o;
+    const int64_t nb = e->n_bodies;
+    auto add = [&](const double *host, int64_t at, int64_t words) {
+        if (host) o.push_back({const_cast<double *>(host), e->io + at * nb, sizeof(double) * (size_t)(words * nb)});
+    };
+    add(x3, 0, 3);
+    add(v3, 3, 3);
+    add(a3, 6, 3);
+    add(m, 9, 1);
+    add(r, 10, 1);
+    add(rest, 11, 1);
+    return o;
+}
+
 static void ens_release_graph(gtd_ensemble *e);
 
 static void ens_release(gtd_ensemble *e) {
@@ -653,6 +701,8 @@ static void ens_release(gtd_ensemble *e) {
     cudaFree(e->items); cudaFree(e->cand); cudaFree(e->info); cudaFree(e->arrived);
     e->items = nullptr; e->cand = nullptr; e->info = nullptr; e->arrived = nullptr;
     e->items_for = 0;
+    cudaFree(e->io);
+    e->io = nullptr;
     cudaFree(e->off); cudaFree(e->cnt); cudaFree(e->order); cudaFree(e->pos); cudaFree(e->vel); cudaFree(e->acc);
     cudaFree(e->rad); cudaFree(e->rest); cudaFree(e->ids); cudaFree(e->work); cudaFree(e->status);
     e->off = nullptr; e->cnt = nullptr; e->order = nullptr; e->pos = e->vel = e->acc = nullptr;
@@ -700,7 +750,8 @@ static int ens_prepare(gtd_ensemble *e) {
     e->items = nullptr;
     e->items_for = 0;
     GTD_CUDA(cudaMalloc(&e->items, sizeof(int2) * std::max<size_t>(items.size(), 1)));
-    GTD_CUDA(cudaMemcpy(e->items, items.data(), sizeof(int2) * items.size(), cudaMemcpyHostToDevice));
+    GTD_CUDA(cudaMemcpyAsync(e->items, items.data(), sizeof(int2) * items.size(), cudaMemcpyHostToDevice, e->stream));
+    GTD_CUDA(cudaStreamSynchronize(e->stream));
     e->n_items = (int64_t)items.size();
     e->items_for = key;
     return GTD_OK;
@@ -808,6 +859,7 @@ int gtd_ensemble_destroy(gtd_ensemble *e) {
     cudaSetDevice(e->device);
     cudaStreamSynchronize(e->stream);
     ens_release(e);
+    release_host_ring(e->host_ring);
     cudaEventDestroy(e->ev0);
     cudaEventDestroy(e->ev1);
     cudaStreamDestroy(e->stream);
@@ -850,18 +902,9 @@ int gtd_ensemble_upload(gtd_ensemble *e, int64_t n_systems, const int64_t *offse
     }
     std::iota(order.begin(), order.end(), 0);
     std::stable_sort(order.begin(), order.end(), [&](int32_t a, int32_t b) { return cnt[a] > cnt[b]; });
-    std::vector<double4> hp((size_t)nb), hv((size_t)nb);
-    std::vector<double> hr((size_t)nb), he((size_t)nb);
-    std::vector<int32_t> hid((size_t)nb);
-    for (int64_t s = 0; s < n_systems; ++s)
-        for (int64_t i = offsets[s]; i < offsets[s + 1]; ++i) {
-            if (m[i] < 0) return fail(GTD_ERR_INVALID_ARGUMENT, "negative mass at body %lld", (long long)i);
-            hp[(size_t)i] = make_double4(x3[3 * i], x3[3 * i + 1], x3[3 * i + 2], m[i]);
-            hv[(size_t)i] = v3 ? make_double4(v3[3 * i], v3[3 * i + 1], v3[3 * i + 2], 0.0) : make_double4(0, 0, 0, 0);
-            hr[(size_t)i] = r ? r[i] : 0.0;
-            he[(size_t)i] = rest ? rest[i] : 1.0;
-            hid[(size_t)i] = (int32_t)(i - offsets[s]);
-        }
+    const int64_t first = n_systems ? offsets[0] : 0;  // rows before it belong to no system and read as zero
+    for (int64_t i = first; i < nb; ++i)
+        if (m[i] < 0) return fail(GTD_ERR_INVALID_ARGUMENT, "negative mass at body %lld", (long long)i);
     const size_t b4 = sizeof(double4) * (size_t)std::max<int64_t>(nb, 1);
     GTD_CUDA(cudaMalloc(&e->off, sizeof(int64_t) * (size_t)(n_systems + 1)));
     GTD_CUDA(cudaMalloc(&e->cnt, sizeof(int32_t) * (size_t)std::max<int64_t>(n_systems, 1)));
@@ -878,23 +921,33 @@ int gtd_ensemble_upload(gtd_ensemble *e, int64_t n_systems, const int64_t *offse
     GTD_CUDA(cudaMalloc(&e->cand, sizeof(EnsCand) * ns));
     GTD_CUDA(cudaMalloc(&e->info, sizeof(EnsInfo) * ns));
     GTD_CUDA(cudaMalloc(&e->arrived, sizeof(int) * ns));
-    GTD_CUDA(cudaMemset(e->cand, 0, sizeof(EnsCand) * ns));
-    GTD_CUDA(cudaMemset(e->arrived, 0, sizeof(int) * ns));
-    GTD_CUDA(cudaMemcpy(e->off, offsets, sizeof(int64_t) * (size_t)(n_systems + 1), cudaMemcpyHostToDevice));
+    cudaStream_t st = e->stream;
+    GTD_CUDA(cudaMemsetAsync(e->cand, 0, sizeof(EnsCand) * ns, st));
+    GTD_CUDA(cudaMemsetAsync(e->arrived, 0, sizeof(int) * ns, st));
+    GTD_CUDA(cudaMemcpyAsync(e->off, offsets, sizeof(int64_t) * (size_t)(n_systems + 1), cudaMemcpyHostToDevice, st));
     if (n_systems) {
-        GTD_CUDA(cudaMemcpy(e->cnt, cnt.data(), sizeof(int32_t) * cnt.size(), cudaMemcpyHostToDevice));
-        GTD_CUDA(cudaMemcpy(e->order, order.data(), sizeof(int32_t) * order.size(), cudaMemcpyHostToDevice));
+        GTD_CUDA(cudaMemcpyAsync(e->cnt, cnt.data(), sizeof(int32_t) * cnt.size(), cudaMemcpyHostToDevice, st));
+        GTD_CUDA(cudaMemcpyAsync(e->order, order.data(), sizeof(int32_t) * order.size(), cudaMemcpyHostToDevice, st));
     }
     if (nb) {
-        GTD_CUDA(cudaMemcpy(e->pos, hp.data(), b4, cudaMemcpyHostToDevice));
-        GTD_CUDA(cudaMemcpy(e->vel, hv.data(), b4, cudaMemcpyHostToDevice));
-        GTD_CUDA(cudaMemset(e->acc, 0, b4));
-        GTD_CUDA(cudaMemcpy(e->rad, hr.data(), sizeof(double) * (size_t)nb, cudaMemcpyHostToDevice));
-        GTD_CUDA(cudaMemcpy(e->rest, he.data(), sizeof(double) * (size_t)nb, cudaMemcpyHostToDevice));
-        GTD_CUDA(cudaMemcpy(e->ids, hid.data(), sizeof(int32_t) * (size_t)nb, cudaMemcpyHostToDevice));
+        GTD_CUDA(cudaMalloc(&e->io, 12 * sizeof(double) * (size_t)nb));
+        int rc = copy_to_device(e->host_ring, e->device, e->stream, ens_spans(e, m, r, rest, x3, v3, nullptr));
+        if (rc) return rc;
+        ens_pack_kernel<<<(unsigned)n_systems, 256, 0, e->stream>>>(e->off, nb, e->io, v3 != nullptr, r != nullptr,
+                                                                    rest != nullptr, e->pos, e->vel, e->acc, e->rad,
+                                                                    e->rest, e->ids);
+        GTD_CHECK_LAUNCH();
+        if (first > 0) {
+            GTD_CUDA(cudaMemsetAsync(e->pos, 0, sizeof(double4) * (size_t)first, st));
+            GTD_CUDA(cudaMemsetAsync(e->vel, 0, sizeof(double4) * (size_t)first, st));
+            GTD_CUDA(cudaMemsetAsync(e->acc, 0, sizeof(double4) * (size_t)first, st));
+            GTD_CUDA(cudaMemsetAsync(e->rad, 0, sizeof(double) * (size_t)first, st));
+            GTD_CUDA(cudaMemsetAsync(e->rest, 0, sizeof(double) * (size_t)first, st));
+        }
     }
-    GTD_CUDA(cudaMemset(e->work, 0, 4 * sizeof(unsigned)));
-    GTD_CUDA(cudaMemset(e->status, 0, sizeof(int)));
+    GTD_CUDA(cudaMemsetAsync(e->work, 0, 4 * sizeof(unsigned), st));
+    GTD_CUDA(cudaMemsetAsync(e->status, 0, sizeof(int), st));
+    GTD_CUDA(cudaStreamSynchronize(st));
     e->begun = false;
     if (!e->configured) ens_default(e);
     return GTD_OK;
@@ -941,22 +994,10 @@ int gtd_ensemble_download(gtd_ensemble *e, double *m, double *r, double *rest, d
     GTD_CUDA(cudaStreamSynchronize(e->stream));
     const int64_t nb = e->n_bodies;
     if (!nb) return GTD_OK;
-    std::vector<double4> hp((size_t)nb), hv((size_t)nb), ha((size_t)nb);
-    std::vector<double> hr((size_t)nb), he((size_t)nb);
-    GTD_CUDA(cudaMemcpy(hp.data(), e->pos, sizeof(double4) * (size_t)nb, cudaMemcpyDeviceToHost));
-    GTD_CUDA(cudaMemcpy(hv.data(), e->vel, sizeof(double4) * (size_t)nb, cudaMemcpyDeviceToHost));
-    GTD_CUDA(cudaMemcpy(ha.data(), e->acc, sizeof(double4) * (size_t)nb, cudaMemcpyDeviceToHost));
-    GTD_CUDA(cudaMemcpy(hr.data(), e->rad, sizeof(double) * (size_t)nb, cudaMemcpyDeviceToHost));
-    GTD_CUDA(cudaMemcpy(he.data(), e->rest, sizeof(double) * (size_t)nb, cudaMemcpyDeviceToHost));
-    for (int64_t i = 0; i < nb; ++i) {
-        if (m) m[i] = hp[(size_t)i].w;
-        if (x3) { x3[3 * i] = hp[(size_t)i].x; x3[3 * i + 1] = hp[(size_t)i].y; x3[3 * i + 2] = hp[(size_t)i].z; }
-        if (v3) { v3[3 * i] = hv[(size_t)i].x; v3[3 * i + 1] = hv[(size_t)i].y; v3[3 * i + 2] = hv[(size_t)i].z; }
-        if (a3) { a3[3 * i] = ha[(size_t)i].x; a3[3 * i + 1] = ha[(size_t)i].y; a3[3 * i + 2] = ha[(size_t)i].z; }
-        if (r) r[i] = hr[(size_t)i];
-        if (rest) rest[i] = he[(size_t)i];
-    }
-    return GTD_OK;
+    ens_unpack_kernel<<<(unsigned)((nb + 255) / 256), 256, 0, e->stream>>>(nb, e->pos, e->vel, e->acc, e->rad, e->rest,
+                                                                          e->io);
+    GTD_CHECK_LAUNCH();
+    return copy_to_host(e->host_ring, e->device, e->stream, ens_spans(e, m, r, rest, x3, v3, a3));
 }
 
 int gtd_ensemble_set_threads(gtd_ensemble *e, int threads) {

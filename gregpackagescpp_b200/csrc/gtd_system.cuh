@@ -9,6 +9,7 @@
 #include <vector>
 
 #include "gtd_internal.cuh"
+#include "host_copy.cuh"
 
 // What a captured step graph depends on.
 struct GraphKey {
@@ -46,7 +47,8 @@ struct gtd_system {
     double4 *pred_pos = nullptr, *pred_vel = nullptr;
     double *rad = nullptr, *rest = nullptr;
     int32_t *ids = nullptr;  // upload index of the body in each slot
-    double4 *stage = nullptr;  // pinned host staging (4 double4 per body)
+    void *stage = nullptr;     // pinned host scratch (ensure_stage)
+    size_t stage_bytes = 0;
 
     // direct summation
     gtd::ForcePlan plan;
@@ -142,6 +144,7 @@ struct gtd_system {
     // host-array staging on the device (io.cu)
     void *io_dev = nullptr;
     size_t io_bytes = 0;
+    gtd::HostRing host_ring;
 
     // evolve callbacks (callbacks.cu).  Host: a hook called inside every step of evolve_steps at
     // for_all_bods' place.  Device: continue_ev_if / for_each_bod / for_all_bods as GPU work.
@@ -229,6 +232,7 @@ int device_upload(gtd_system *s, int64_t n, const double *m, const double *r, co
 int device_download(gtd_system *s, double *m, double *r, double *rest, double *x3, double *v3, double *a3);
 int record_frame(gtd_system *s, uint64_t state);
 int ensure_body_capacity(gtd_system *s, int64_t n);
+int ensure_stage(gtd_system *s, size_t bytes);
 int set_loaded_bodies(gtd_system *s, int64_t n);
 int ensure_plan(gtd_system *s);
 int force_and_integrate(gtd_system *s, const double4 *src, int epi, const gtd::StepArgs &st);

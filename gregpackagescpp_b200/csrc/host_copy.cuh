@@ -1,0 +1,33 @@
+// Copies between a caller's pageable arrays and device memory.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <cstddef>
+#include <vector>
+
+namespace gtd {
+
+struct HostSpan {
+    void *host;
+    void *dev;
+    size_t bytes;
+};
+
+// A handle's pinned staging ring, made on the first large copy and freed with the handle.
+struct HostRing {
+    char *mem = nullptr;
+    std::vector<cudaEvent_t> events;  // one per slot
+};
+void release_host_ring(HostRing &ring);
+
+// Copies the spans behind what `stream` has queued.  copy_to_host returns when every byte has arrived;
+// after copy_to_device the caller's arrays may change once the stream has been synchronised.  Small
+// copies, and arrays that are pinned already, go through the driver; large ones are cut into chunks that
+// a few threads move between the caller's arrays and pinned slots while the copy engine moves the slots:
+// one thread copies, and takes the page faults of a fresh array, at 5 to 15 GB/s (88 bytes of each of 2^20
+// bodies to fresh arrays: 17.7 ms, 4.8 with the threads).
+int copy_to_host(HostRing &ring, int device, cudaStream_t stream, const std::vector<HostSpan> &spans);
+int copy_to_device(HostRing &ring, int device, cudaStream_t stream, const std::vector<HostSpan> &spans);
+
+}  // namespace gtd

@@ -4,13 +4,14 @@
 // double per body for m, r, rest), in upload order.  The device keeps double4 records, possibly in a
 // spatial order.  The conversion runs on the GPU: each requested array crosses PCIe once, as is,
 // into (or out of) a device staging area, and a kernel packs (or unpacks and reorders) it, so the
-// host does no per-body work.
+// host does no per-body work beyond the copy (host_copy.cuh).
 #include <cuda_runtime.h>
 
 #include <vector>
 
 #include "gtd_internal.cuh"
 #include "gtd_system.cuh"
+#include "host_copy.cuh"
 
 namespace gtd {
 
@@ -32,6 +33,23 @@ static IoView io_view(double *base, int64_t n) {
     v.rest = base + 11 * n;
     v.rows = reinterpret_cast<int32_t *>(base + 12 * n);
     return v;
+}
+
+// The caller's arrays beside their staging areas (NULL: not given).
+static std::vector<HostSpan> io_spans(const IoView &io, int64_t n, const double *m, const double *r, const double *rest,
+                                      const double *x3, const double *v3, const double *a3) {
+    std::vector<HostSpan> o;
+    const size_t b = sizeof(double) * (size_t)n;
+    auto add = [&](const double *host, double *dev, size_t bytes) {
+        if (host) o.push_back({const_cast<double *>(host), dev, bytes});
+    };
+    add(x3, io.x3, 3 * b);
+    add(v3, io.v3, 3 * b);
+    add(a3, io.a3, 3 * b);
+    add(m, io.m, b);
+    add(r, io.r, b);
+    add(rest, io.rest, b);
+    return o;
 }
 
 static int ensure_io(gtd_system *s, int64_t n) {
@@ -111,6 +129,7 @@ __global__ void update_bodies_kernel(int64_t n, double4 *pm, double4 *vel, doubl
 using namespace gtd;
 
 void release_io(gtd_system *s) {
+    release_host_ring(s->host_ring);
     cudaFree(s->io_dev);
     s->io_dev = nullptr;
     s->io_bytes = 0;
@@ -123,12 +142,8 @@ int device_upload(gtd_system *s, int64_t n, const double *m, const double *r, co
     if (rc) return rc;
     IoView io = io_view(static_cast<double *>(s->io_dev), n);
     cudaStream_t st = s->stream;
-    const size_t d = sizeof(double);
-    GTD_CUDA(cudaMemcpyAsync(io.x3, x3, 3 * d * (size_t)n, cudaMemcpyHostToDevice, st));
-    GTD_CUDA(cudaMemcpyAsync(io.m, m, d * (size_t)n, cudaMemcpyHostToDevice, st));
-    if (v3) GTD_CUDA(cudaMemcpyAsync(io.v3, v3, 3 * d * (size_t)n, cudaMemcpyHostToDevice, st));
-    if (r) GTD_CUDA(cudaMemcpyAsync(io.r, r, d * (size_t)n, cudaMemcpyHostToDevice, st));
-    if (rest) GTD_CUDA(cudaMemcpyAsync(io.rest, rest, d * (size_t)n, cudaMemcpyHostToDevice, st));
+    rc = copy_to_device(s->host_ring, s->device, st, io_spans(io, n, m, r, rest, x3, v3, nullptr));
+    if (rc) return rc;
     int *bad = reinterpret_cast<int *>(io.rows);  // two ints of scratch, before the rows are needed
     const int init[2] = {INT32_MAX, INT32_MAX};
     GTD_CUDA(cudaMemcpyAsync(bad, init, sizeof init, cudaMemcpyHostToDevice, st));
@@ -181,15 +196,7 @@ int device_download(gtd_system *s, double *m, double *r, double *rest, double *x
                                                                         s->rest, map, io, want);
     GTD_CHECK_LAUNCH();
     s->launches += 1;
-    const size_t d = sizeof(double);
-    if (x3) GTD_CUDA(cudaMemcpyAsync(x3, io.x3, 3 * d * (size_t)n, cudaMemcpyDeviceToHost, st));
-    if (v3) GTD_CUDA(cudaMemcpyAsync(v3, io.v3, 3 * d * (size_t)n, cudaMemcpyDeviceToHost, st));
-    if (a3) GTD_CUDA(cudaMemcpyAsync(a3, io.a3, 3 * d * (size_t)n, cudaMemcpyDeviceToHost, st));
-    if (m) GTD_CUDA(cudaMemcpyAsync(m, io.m, d * (size_t)n, cudaMemcpyDeviceToHost, st));
-    if (r) GTD_CUDA(cudaMemcpyAsync(r, io.r, d * (size_t)n, cudaMemcpyDeviceToHost, st));
-    if (rest) GTD_CUDA(cudaMemcpyAsync(rest, io.rest, d * (size_t)n, cudaMemcpyDeviceToHost, st));
-    GTD_CUDA(cudaStreamSynchronize(st));
-    return GTD_OK;
+    return copy_to_host(s->host_ring, s->device, st, io_spans(io, n, m, r, rest, x3, v3, a3));
 }
 
 // Overwrites the given arrays (any may be NULL) of the live bodies, in download order, leaving the
@@ -206,12 +213,8 @@ int device_update(gtd_system *s, const double *m, const double *r, const double 
     const int32_t *map = nullptr;
     rc = row_map(s, io, &map);
     if (rc) return rc;
-    const size_t d = sizeof(double);
-    if (x3) GTD_CUDA(cudaMemcpyAsync(io.x3, x3, 3 * d * (size_t)n, cudaMemcpyHostToDevice, st));
-    if (v3) GTD_CUDA(cudaMemcpyAsync(io.v3, v3, 3 * d * (size_t)n, cudaMemcpyHostToDevice, st));
-    if (m) GTD_CUDA(cudaMemcpyAsync(io.m, m, d * (size_t)n, cudaMemcpyHostToDevice, st));
-    if (r) GTD_CUDA(cudaMemcpyAsync(io.r, r, d * (size_t)n, cudaMemcpyHostToDevice, st));
-    if (rest) GTD_CUDA(cudaMemcpyAsync(io.rest, rest, d * (size_t)n, cudaMemcpyHostToDevice, st));
+    rc = copy_to_device(s->host_ring, s->device, st, io_spans(io, n, m, r, rest, x3, v3, nullptr));
+    if (rc) return rc;
     update_bodies_kernel<<<(unsigned)((n + kIT - 1) / kIT), kIT, 0, st>>>(n, s->pm[s->cur], s->vel, s->rad, s->rest,
                                                                         map, io, have);
     GTD_CHECK_LAUNCH();

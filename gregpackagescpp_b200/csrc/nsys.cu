@@ -556,7 +556,9 @@ int gtd_system_load_nsys(gtd_system *s, const char *path, int check_nan_inf, int
             return fail(GTD_ERR_NSYS_LOAD, "Error reading .nsys file. Could not load data.\n");
         rc = ensure_body_capacity(s, n);
         if (rc) return rc;
-        unsigned long long *bad = reinterpret_cast<unsigned long long *>(s->stage);  // pinned, >= 8 bytes
+        rc = ensure_stage(s, sizeof(unsigned long long));
+        if (rc) return rc;
+        unsigned long long *bad = static_cast<unsigned long long *>(s->stage);
         GTD_CUDA(cudaMemcpyAsync(s->nsys_dev, s->nsys_host, bytes, cudaMemcpyHostToDevice, s->stream));
         unsigned long long *bad_dev = reinterpret_cast<unsigned long long *>(s->acc);  // scratch until zeroed
         GTD_CUDA(cudaMemsetAsync(bad_dev, 0xff, sizeof(unsigned long long), s->stream));

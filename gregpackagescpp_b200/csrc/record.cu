@@ -93,11 +93,12 @@ int record_frame(gtd_system *s, uint64_t state) {
     frame_kernel<<<blocks, kRT, 0, s->stream>>>(n, s->pm[s->cur], s->vel, s->ids, s->G, s->rec_dev);
     GTD_CHECK_LAUNCH();
     s->launches += 1;
-    // the pinned staging area holds 16 doubles per body
+    const int rc = ensure_stage(s, sizeof(double) * 8 * (size_t)n);
+    if (rc) return rc;
     GTD_CUDA(cudaMemcpyAsync(s->stage, s->rec_dev, sizeof(double) * 8 * (size_t)n, cudaMemcpyDeviceToHost,
                              s->stream));
     GTD_CUDA(cudaStreamSynchronize(s->stream));
-    const double *h = reinterpret_cast<const double *>(s->stage);
+    const double *h = static_cast<const double *>(s->stage);
     s->rec_frames.insert(s->rec_frames.end(), h, h + 8 * (size_t)n);
     s->rec_states.push_back((int64_t)state);
     s->rec_n = n;

@@ -56,8 +56,18 @@ static int ensure_capacity(gtd_system *s, int64_t n) {
     GTD_CUDA(cudaMalloc(&s->rad, sizeof(double) * (size_t)n));
     GTD_CUDA(cudaMalloc(&s->rest, sizeof(double) * (size_t)n));
     GTD_CUDA(cudaMalloc(&s->ids, sizeof(int32_t) * (size_t)n));
-    GTD_CUDA(cudaMallocHost(&s->stage, 4 * b4));
     s->cap = n;
+    return GTD_OK;
+}
+
+// Pinned host scratch of at least `bytes`.
+int ensure_stage(gtd_system *s, size_t bytes) {
+    if (bytes <= s->stage_bytes) return GTD_OK;
+    cudaFreeHost(s->stage);
+    s->stage = nullptr;
+    s->stage_bytes = 0;
+    GTD_CUDA(cudaMallocHost(&s->stage, bytes));
+    s->stage_bytes = bytes;
     return GTD_OK;
 }
 
@@ -103,6 +113,7 @@ void release_bodies(gtd_system *s) {
     s->partials = nullptr;
     s->escratch = nullptr;
     s->stage = nullptr;
+    s->stage_bytes = 0;
     s->part_bytes = 0;
     s->escratch_n = 0;
     s->cap = 0;

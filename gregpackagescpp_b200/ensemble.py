@@ -67,8 +67,8 @@ class Ensemble:
     def state(self):
         """Per-system survivors: list of dicts with m, r, rest, x, v, a (upload order)."""
         nb = int(self.offsets[-1])
-        m, r, rest = np.zeros(nb), np.zeros(nb), np.zeros(nb)
-        x, v, a = np.zeros((nb, 3)), np.zeros((nb, 3)), np.zeros((nb, 3))
+        m, r, rest = np.empty(nb), np.empty(nb), np.empty(nb)
+        x, v, a = np.empty((nb, 3)), np.empty((nb, 3)), np.empty((nb, 3))
         check(self._L.gtd_ensemble_download(self._h, ptr(m), ptr(r), ptr(rest), ptr(x), ptr(v), ptr(a)))
         c, _, _ = self.counts()
         out = []

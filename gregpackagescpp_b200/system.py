@@ -288,8 +288,8 @@ class System:
         L = self._L
         check(L.gtd_system_num_bodies(self._h, C.byref(n)))
         k = n.value
-        m, r, rest = np.zeros(k), np.zeros(k), np.zeros(k)
-        x, v, a = np.zeros((k, 3)), np.zeros((k, 3)), np.zeros((k, 3))
+        m, r, rest = np.empty(k), np.empty(k), np.empty(k)
+        x, v, a = np.empty((k, 3)), np.empty((k, 3)), np.empty((k, 3))
         check(L.gtd_system_download(self._h, C.byref(n), ptr(m), ptr(r), ptr(rest), ptr(x), ptr(v), ptr(a)))
         self.m, self.r, self.rest, self.x, self.v, self.a = m, r, rest, x, v, a
         if len(getattr(self, "curr_ke", ())) != k:
@@ -313,14 +313,13 @@ class System:
             return self._evolve_device(integration_method, continue_ev_if, for_each_bod, for_all_bods, max_steps)
         self._push()
         ns = C.c_int64()
+        x0, v0 = self._start_state()
         if not cbs:
-            x0, v0 = self.x.copy(), self.v.copy()
             check(self._L.gtd_system_evolve(self._h, integration_method, C.byref(ns)))
             self._pull()
             self._recordings_from(x0, v0, integration_method)
             self.time_elapsed = self.iterations * self.dt
             return ns.value
-        x0, v0 = self.x.copy(), self.v.copy()
         if (integration_method & System.barnes_hut) == System.barnes_hut:
             # the Barnes-Hut branch calls no callback (gregsys.hpp:2893-2945)
             check(self._L.gtd_system_evolve(self._h, integration_method, C.byref(ns)))
@@ -381,7 +380,7 @@ class System:
 
     def _evolve_device(self, method, cont, each, all_, max_steps) -> int:
         L, h = self._L, self._h
-        x0, v0 = self.x.copy(), self.v.copy()
+        x0, v0 = self._start_state()
         self._push()
         hooks = []
         for cb in (cont, each, all_):
@@ -432,6 +431,10 @@ class System:
         self.pe = np.zeros((0, n))
         self.energies = np.zeros((0, n))
         self.tot_pe, self.tot_ke, self.tot_e = np.zeros(0), np.zeros(0), np.zeros(0)
+
+    def _start_state(self) -> tuple:
+        """The state an evolve starts from, for its records (None where it keeps none)."""
+        return (self.x.copy(), self.v.copy()) if self.mem_freq else (None, None)
 
     def _recordings_from(self, x0, v0, method: int) -> None:
         """The last evolve's records, its first frame the state (x0, v0) it started from."""
