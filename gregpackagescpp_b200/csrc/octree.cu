@@ -619,7 +619,7 @@ __global__ void __launch_bounds__(kTT, sizeof(T) == 4 ? 6 : 1) walk_kernel(int64
     }
 }
 
-// ---- list walk (float trees) ------------------------------------------------------------------
+// ---- list walk ------------------------------------------------------------------
 // The same per-body cell sets as walk_kernel, computed in two phases per warp of 32 consecutive
 // slots.  Traversal: the warp pops up to 32 (sibling chain, lane mask) entries from a stack in
 // shared memory - one node per lane - and classifies each node for all lanes of its mask at once
@@ -636,12 +636,19 @@ __global__ void __launch_bounds__(kTT, sizeof(T) == 4 ? 6 : 1) walk_kernel(int64
 // Resident warps hide the traversal's dependent loads: 4 warps per CTA with 6.25 KB of shared
 // memory each and at most 64 registers give 8 CTAs (32 warps) per SM (13.1 ms per walk at
 // N = 4194304, against 15.2 ms with a 512-entry stack at 24 warps per SM).
+// Double trees: the same traversal in FP64 (the bounds hold at any precision), entries of 32 bytes evaluated
+// by 17 FP64 operations each: 0.88 ms per walk at N = 131072, 3.17 at 524288, against 1.92 and 5.19 for
+// walk_kernel.
 constexpr int kLwWarps = 4;      // warps per CTA
 constexpr int kLwStack = 320;    // stack entries per warp (a walk of 2M bodies peaks near 220)
 constexpr int kLwDfs = kLwStack - 64;  // above this many entries the warp pops one entry at a time
 constexpr int kLwList = 128;     // list entries per warp before an evaluation pass
 
-struct LwWarp {
+template <typename T>
+struct LwWarp;
+
+template <>
+struct LwWarp<float> {
     int st[kLwStack], en[kLwStack];  // sibling chain: nodes st, skip[st], ... below en
     unsigned mk[kLwStack];           // lanes still walking below the chain's parent
     // accepted node: centre of mass and G M (or a bucket leaf's body), stored by pairs of entries:
@@ -652,8 +659,16 @@ struct LwWarp {
 };
 static_assert(kLwList % 2 == 0 && (3 * kLwStack * sizeof(int)) % 16 == 0, "float4 pairs of list entries");
 
+template <>
+struct LwWarp<double> {
+    int st[kLwStack], en[kLwStack];
+    unsigned mk[kLwStack];
+    double2 xy[kLwList], zw[kLwList];
+    unsigned lm[kLwList];
+};
+
 // writes list entry `at`
-__device__ __forceinline__ void lw_put(LwWarp &W, int at, float x, float y, float z, float w, unsigned m) {
+__device__ __forceinline__ void lw_put(LwWarp<float> &W, int at, float x, float y, float z, float w, unsigned m) {
     float *a = reinterpret_cast<float *>(&W.pxy[at >> 1]) + (at & 1);
     float *b = reinterpret_cast<float *>(&W.pzw[at >> 1]) + (at & 1);
     a[0] = x;
@@ -662,25 +677,33 @@ __device__ __forceinline__ void lw_put(LwWarp &W, int at, float x, float y, floa
     b[2] = w;
     W.lm[at] = m;
 }
-constexpr size_t kLwSmem = sizeof(LwWarp) * kLwWarps;
+__device__ __forceinline__ void lw_put(LwWarp<double> &W, int at, double x, double y, double z, double w, unsigned m) {
+    W.xy[at] = make_double2(x, y);
+    W.zw[at] = make_double2(z, w);
+    W.lm[at] = m;
+}
+template <typename T>
+constexpr size_t kLwSmem = sizeof(LwWarp<T>) * kLwWarps;
 
-__device__ __forceinline__ float lw_r2(float dx, float dy, float dz) {
-    return __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
+template <typename T>
+__device__ __forceinline__ T lw_r2(T dx, T dy, T dz) {
+    return fma_t(dz, dz, fma_t(dy, dy, mul_t(dx, dx)));
 }
 
 // distance from a box [lo, hi] to c along one axis: nearest and farthest offsets as the lanes
 // round them (c - hi <= fl(c - p) <= c - lo for every lane p in the box)
-__device__ __forceinline__ void lw_axis(float c, float lo, float hi, float &dmin, float &dmax) {
-    const float a = __fsub_rn(c, hi), b = __fsub_rn(c, lo);
-    dmin = a > 0.f ? a : (b < 0.f ? -b : 0.f);
-    dmax = fmaxf(fabsf(a), fabsf(b));
+template <typename T>
+__device__ __forceinline__ void lw_axis(T c, T lo, T hi, T &dmin, T &dmax) {
+    const T a = sub_t(c, hi), b = sub_t(c, lo);
+    dmin = a > (T)0 ? a : (b < (T)0 ? -b : (T)0);
+    dmax = max(abs(a), abs(b));
 }
 
 // Evaluation pass over the list: two entries per step in packed FP32x2 arithmetic (per lane of the
 // pair the same correctly rounded operations as the scalar walk: x + (-p) = x - p exactly as
 // rounded), summed in two partial sums.
 template <bool SOFT, bool COUNT>
-__device__ __forceinline__ void lw_eval(const LwWarp &W, int len, unsigned lane, float4 p, float eps2, float &ax,
+__device__ __forceinline__ void lw_eval(const LwWarp<float> &W, int len, unsigned lane, float4 p, float eps2, float &ax,
                                         float &ay, float &az, uint32_t &cnt) {
     const float2 npx = make_float2(-p.x, -p.x), npy = make_float2(-p.y, -p.y), npz = make_float2(-p.z, -p.z);
     const float2 zero = make_float2(0.f, 0.f);
@@ -736,12 +759,52 @@ __device__ __forceinline__ void lw_eval(const LwWarp &W, int len, unsigned lane,
     az += fz.x + fz.y;
 }
 
+// FP64: two entries per step, summed apart; terms as in walk_kernel.
 template <bool SOFT, bool COUNT>
-__global__ void __launch_bounds__(kLwWarps * 32, 8) list_walk_kernel(int64_t n, int64_t n_nodes, const float4 *rec,
-                                                                  const float4 *bodies, float th2, float eps2,
-                                                                  float4 *slot_acc, uint32_t *slot_cnt, int *status) {
+__device__ __forceinline__ void lw_eval(const LwWarp<double> &W, int len, unsigned lane, double4 p, double eps2, double &ax,
+                                        double &ay, double &az, uint32_t &cnt) {
+    const unsigned lbit = 1u << lane;
+    double f[2][3] = {};
+    auto term = [&](int e, double (&o)[3]) {
+        const double2 xy = W.xy[e], zw = W.zw[e];
+        const bool bit = (W.lm[e] & lbit) != 0u;
+        const double dx = sub_t(xy.x, p.x), dy = sub_t(xy.y, p.y), dz = sub_t(zw.x, p.z);
+        const double r2 = lw_r2(dx, dy, dz);
+        const double inv = rsqrt_t(SOFT ? r2 + eps2 : r2);
+        double sc = mul_t(mul_t(mul_t(zw.y, inv), inv), inv);
+        sc = bit ? sc : 0.0;
+        o[0] = fma_t(sc, dx, o[0]);
+        o[1] = fma_t(sc, dy, o[1]);
+        o[2] = fma_t(sc, dz, o[2]);
+        if constexpr (COUNT) cnt += bit ? 1u : 0u;
+    };
+    int e = 0;
+    for (; e + 1 < len; e += 2) {
+        term(e, f[0]);
+        term(e + 1, f[1]);
+    }
+    if (e < len) term(e, f[0]);
+    ax += f[0][0] + f[1][0];
+    ay += f[0][1] + f[1][1];
+    az += f[0][2] + f[1][2];
+}
+
+// The nodes' walk records: float trees A and B interleaved in rec, double trees in three arrays.
+struct LwNodes {
+    const void *rec;
+    const int4 *rec_b;
+    const double *w2;
+};
+
+template <typename T, bool SOFT, bool COUNT>
+__global__ void __launch_bounds__(kLwWarps * 32, sizeof(T) == 4 ? 8 : 4)
+    list_walk_kernel(int64_t n, int64_t n_nodes, LwNodes nodes, const void *bodies_v, T th2, T eps2, void *slot_acc_v,
+                     uint32_t *slot_cnt, int *status) {
+    using V = typename V4<T>::type;
+    const V *bodies = reinterpret_cast<const V *>(bodies_v);
+    V *slot_acc = reinterpret_cast<V *>(slot_acc_v);
     extern __shared__ __align__(16) unsigned char lw_smem[];
-    LwWarp &W = reinterpret_cast<LwWarp *>(lw_smem)[threadIdx.x >> 5];
+    LwWarp<T> &W = reinterpret_cast<LwWarp<T> *>(lw_smem)[threadIdx.x >> 5];
     const unsigned lane = threadIdx.x & 31u;
     const unsigned lt = (1u << lane) - 1u;  // lanes below this one
     const int64_t base = ((int64_t)blockIdx.x * kLwWarps + (threadIdx.x >> 5)) * 32;
@@ -749,19 +812,18 @@ __global__ void __launch_bounds__(kLwWarps * 32, 8) list_walk_kernel(int64_t n, 
     const int64_t s = base + lane;
     const bool active = s < n;
     const unsigned full = __ballot_sync(0xffffffffu, active);
-    float4 p = bodies[active ? s : base];  // lanes past n stand on lane 0's body (in no mask)
-    float lox = p.x, hix = p.x, loy = p.y, hiy = p.y, loz = p.z, hiz = p.z;
+    const V p = bodies[active ? s : base];  // lanes past n stand on lane 0's body (in no mask)
+    T lox = p.x, hix = p.x, loy = p.y, hiy = p.y, loz = p.z, hiz = p.z;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
-        lox = fminf(lox, __shfl_xor_sync(0xffffffffu, lox, o));
-        hix = fmaxf(hix, __shfl_xor_sync(0xffffffffu, hix, o));
-        loy = fminf(loy, __shfl_xor_sync(0xffffffffu, loy, o));
-        hiy = fmaxf(hiy, __shfl_xor_sync(0xffffffffu, hiy, o));
-        loz = fminf(loz, __shfl_xor_sync(0xffffffffu, loz, o));
-        hiz = fmaxf(hiz, __shfl_xor_sync(0xffffffffu, hiz, o));
+        lox = min(lox, __shfl_xor_sync(0xffffffffu, lox, o));
+        hix = max(hix, __shfl_xor_sync(0xffffffffu, hix, o));
+        loy = min(loy, __shfl_xor_sync(0xffffffffu, loy, o));
+        hiy = max(hiy, __shfl_xor_sync(0xffffffffu, hiy, o));
+        loz = min(loz, __shfl_xor_sync(0xffffffffu, loz, o));
+        hiz = max(hiz, __shfl_xor_sync(0xffffffffu, hiz, o));
     }
-    const int4 *recb = reinterpret_cast<const int4 *>(rec);
-    float ax = 0.f, ay = 0.f, az = 0.f;
+    T ax = (T)0, ay = (T)0, az = (T)0;
     uint32_t cnt = 0;
     int top = 0, len = 0;  // warp-uniform stack and list sizes
     const int nn = (int)n_nodes;
@@ -807,23 +869,31 @@ __global__ void __launch_bounds__(kLwWarps * 32, 8) list_walk_kernel(int64_t n, 
         }
         top -= k;
         __syncwarp();
-        float4 A = make_float4(0.f, 0.f, 0.f, 0.f);
+        V A;
+        A.x = A.y = A.z = A.w = (T)0;
         int4 B = make_int4(0, 0, 0, 0);
+        T w2 = (T)0;
         if (have) {
-            A = rec[2 * (size_t)st];
-            B = recb[2 * (size_t)st + 1];
+            if constexpr (sizeof(T) == 4) {
+                A = reinterpret_cast<const V *>(nodes.rec)[2 * (size_t)st];
+                B = reinterpret_cast<const int4 *>(nodes.rec)[2 * (size_t)st + 1];
+                w2 = __int_as_float(B.w);
+            } else {
+                A = reinterpret_cast<const V *>(nodes.rec)[st];
+                B = nodes.rec_b[st];
+                w2 = nodes.w2[st];
+            }
         }
         const bool leaf = have && B.z < 0;
         const int count = B.z & 0x7fffffff;
-        const float w2 = __int_as_float(B.w);
         bool far = false, near = false, mixed = false;
         if (have && !leaf) {
-            float nx, fx, ny, fy, nz, fz;
+            T nx, fx, ny, fy, nz, fz;
             lw_axis(A.x, lox, hix, nx, fx);
             lw_axis(A.y, loy, hiy, ny, fy);
             lw_axis(A.z, loz, hiz, nz, fz);
-            far = w2 < __fmul_rn(th2, lw_r2(nx, ny, nz));
-            near = !far && !(w2 < __fmul_rn(th2, lw_r2(fx, fy, fz)));
+            far = w2 < mul_t(th2, lw_r2(nx, ny, nz));
+            near = !far && !(w2 < mul_t(th2, lw_r2(fx, fy, fz)));
             mixed = !far && !near;
         }
         // the in-between nodes: each lane of the node's mask applies walk_kernel's test
@@ -832,11 +902,11 @@ __global__ void __launch_bounds__(kLwWarps * 32, 8) list_walk_kernel(int64_t n, 
         while (mm) {
             const int j = __ffs(mm) - 1;
             mm &= mm - 1;
-            const float cx = __shfl_sync(0xffffffffu, A.x, j), cy = __shfl_sync(0xffffffffu, A.y, j);
-            const float cz = __shfl_sync(0xffffffffu, A.z, j), cw = __shfl_sync(0xffffffffu, w2, j);
-            const float dx = __fsub_rn(cx, p.x), dy = __fsub_rn(cy, p.y), dz = __fsub_rn(cz, p.z);
+            const T cx = __shfl_sync(0xffffffffu, A.x, j), cy = __shfl_sync(0xffffffffu, A.y, j);
+            const T cz = __shfl_sync(0xffffffffu, A.z, j), cw = __shfl_sync(0xffffffffu, w2, j);
+            const T dx = sub_t(cx, p.x), dy = sub_t(cy, p.y), dz = sub_t(cz, p.z);
             // every lane tests; lane j keeps the answers of the lanes in its node's mask
-            const unsigned a = __ballot_sync(0xffffffffu, cw < __fmul_rn(th2, lw_r2(dx, dy, dz)));
+            const unsigned a = __ballot_sync(0xffffffffu, cw < mul_t(th2, lw_r2(dx, dy, dz)));
             if ((int)lane == j) acc = a & mk;
         }
         unsigned em = 0;
@@ -891,7 +961,7 @@ __global__ void __launch_bounds__(kLwWarps * 32, 8) list_walk_kernel(int64_t n, 
                 const bool ap = q0 + (int)lane < c && m1 != 0u;
                 const unsigned b2 = __ballot_sync(0xffffffffu, ap);
                 if (ap) {
-                    const float4 Q = bodies[q];
+                    const V Q = bodies[q];
                     lw_put(W, len + __popc(b2 & lt), Q.x, Q.y, Q.z, Q.w, m1);
                 }
                 len += __popc(b2);
@@ -902,7 +972,9 @@ __global__ void __launch_bounds__(kLwWarps * 32, 8) list_walk_kernel(int64_t n, 
     __syncwarp();
     lw_eval<SOFT, COUNT>(W, len, lane, p, eps2, ax, ay, az, cnt);
     if (active) {
-        slot_acc[s] = make_float4(ax, ay, az, 0.f);
+        V o;
+        o.x = ax; o.y = ay; o.z = az; o.w = (T)0;
+        slot_acc[s] = o;
         if constexpr (COUNT) slot_cnt[s] = cnt;
     }
 }
@@ -961,7 +1033,7 @@ static unsigned blocks_for(int64_t n, int t = kTT) { return (unsigned)((n + t - 
 
 // Float walk: 0 = walk_kernel with A and B in separate arrays, 1 = walk_kernel with interleaved
 // records, 2 = list_walk_kernel (interleaved records; the default: 13.1 ms against 21.0 ms for 1 at
-// N = 4194304, theta = 0.5).  Double trees take walk_kernel.
+// N = 4194304, theta = 0.5).  Double trees: 2, and walk_kernel for 0 and 1.
 constexpr int kDefaultWalkVariant = 2;
 constexpr int kNumWalkVariants = 3;
 static int walk_variant_of(const gtd_system *s) { return s->walk_variant < 0 ? kDefaultWalkVariant : s->walk_variant; }
@@ -1201,25 +1273,26 @@ static void launch_walk(gtd_system *s, T th2, T e2, bool count) {
     }
 }
 
-// The list walk (float trees, interleaved records); errors go to status[1].
-static int launch_list_walk(gtd_system *s, float th2, float e2, bool count) {
+// The list walk (float trees with interleaved records, double trees); errors go to status[1].
+template <typename T>
+static int launch_list_walk(gtd_system *s, T th2, T e2, bool count) {
     const int64_t n = s->n;
-    const bool soft = e2 != 0.f;
+    const bool soft = e2 != (T)0;
     const unsigned blocks = (unsigned)((n + kLwWarps * 32 - 1) / (kLwWarps * 32));
+    const LwNodes nodes{s->nwalk_a, s->nwalk_b, s->nwalk_w2};
     cudaError_t ce = cudaSuccess;
     auto go = [&](auto kern) {
-        ce = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLwSmem);
+        ce = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLwSmem<T>);
         if (ce != cudaSuccess) return;
-        kern<<<blocks, kLwWarps * 32, kLwSmem, s->stream>>>(
-            n, s->n_nodes, reinterpret_cast<const float4 *>(s->nwalk_a), reinterpret_cast<const float4 *>(s->slot_pos),
-            th2, e2, reinterpret_cast<float4 *>(s->slot_acc), s->slot_cnt, s->status + 1);
+        kern<<<blocks, kLwWarps * 32, kLwSmem<T>, s->stream>>>(n, s->n_nodes, nodes, s->slot_pos, th2, e2, s->slot_acc,
+                                                               s->slot_cnt, s->status + 1);
     };
     if (soft) {
-        if (count) go(list_walk_kernel<true, true>);
-        else go(list_walk_kernel<true, false>);
+        if (count) go(list_walk_kernel<T, true, true>);
+        else go(list_walk_kernel<T, true, false>);
     } else {
-        if (count) go(list_walk_kernel<false, true>);
-        else go(list_walk_kernel<false, false>);
+        if (count) go(list_walk_kernel<T, false, true>);
+        else go(list_walk_kernel<T, false, false>);
     }
     GTD_CUDA(ce);
     return GTD_OK;
@@ -1246,7 +1319,7 @@ static int bh_walk_impl(gtd_system *s, double kick, bool do_kick, bool count) {
     if (s->tree_float) {
         const float th2 = (float)(s->theta * s->theta), e2 = (float)(s->eps * s->eps);
         if (s->walk_interleaved && walk_variant_of(s) == 2) {
-            int rc = launch_list_walk(s, th2, e2, count);
+            int rc = launch_list_walk<float>(s, th2, e2, count);
             if (rc) return rc;
         } else if (s->walk_interleaved) {
             launch_walk<float, true>(s, th2, e2, count);
@@ -1258,7 +1331,12 @@ static int bh_walk_impl(gtd_system *s, double kick, bool do_kick, bool count) {
                                                                  ninter, do_kick ? s->vel : nullptr, kick);
     } else {
         const double th2 = s->theta * s->theta, e2 = s->eps * s->eps;
-        launch_walk<double, false>(s, th2, e2, count);
+        if (walk_variant_of(s) == 2) {
+            int rc = launch_list_walk<double>(s, th2, e2, count);
+            if (rc) return rc;
+        } else {
+            launch_walk<double, false>(s, th2, e2, count);
+        }
         GTD_CHECK_LAUNCH();
         scatter_acc_kernel<double><<<blocks_for(n), kTT, 0, st>>>(n, s->perm, s->slot_acc, s->slot_cnt, s->acc,
                                                                   ninter, do_kick ? s->vel : nullptr, kick);

@@ -524,7 +524,7 @@ class System:
         return a, cnt
 
     def set_bh_walk_variant(self, variant: int) -> None:
-        """Float-tree walk (-1 default = 2, 0 per-lane walk with separate node arrays, 1 per-lane
+        """Tree walk (-1 default = 2, 0 per-lane walk with separate node arrays, 1 per-lane
         walk with interleaved 32-byte records, 2 list walk); all take the same interactions per
         body, 0 and 1 in the same order, 2 summed in another order."""
         if variant < -1 or variant > 2:
