@@ -7,7 +7,8 @@
 // device work: the built-ins of random_comet (gregsys.hpp:1935-1984) or hooks that enqueue the
 // caller's own kernels.  The predicate's verdict stays on the device: the loop is a CUDA graph whose
 // WHILE node runs up to kChunkSteps steps, each behind IF nodes that the predicate kernel opens or
-// closes, so the host waits once per chunk.  Cases the graph cannot hold (merging collisions, the
+// closes, so the host waits once per chunk.  Small FP64 leapfrog systems with overlap collisions and
+// built-in callbacks run their steps as two kernels each (build_paired_graph).  Cases the graph cannot hold (merging collisions, the
 // periodic spatial reorder of the mixed path, force timing, memFreq recording) run the same kernels
 // eagerly with one 64-byte read of the verdict per step; the bodies never cross PCIe in either form
 // (a recorded frame is read back when it is made, every memFreq-th step).
@@ -100,7 +101,7 @@ constexpr int64_t kForAllOneBlock = 16384;
 __global__ void __launch_bounds__(kCbThreads) cb_for_all_kernel(int64_t n, const double4 *pm, double *rest, CbCtl *c,
                                                                 int weighted, int set_rest, double min_cor,
                                                                 double max_cor, double scale, double n_exp) {
-    __shared__ double sh[32];
+    __shared__ double sh[96];
     __shared__ double com[3];
     cb_for_all_block(n, pm, rest, c, weighted, set_rest, min_cor, max_cor, scale, n_exp, sh, com);
 }
@@ -357,6 +358,62 @@ static int build_loop_graph(gtd_system *s, const int *coll_status, cudaGraphExec
     return GTD_OK;
 }
 
+// Whether the loop's steps can run as two kernels each (collide.cu): FP64 leapfrog KDK of a size the fused
+// force kernel takes, overlap collisions, and callbacks that are built in.
+static bool paired_steps(const gtd_system *s, int branch) {
+    return branch == GTD_LEAPFROG_KDK && s->precision == GTD_PREC_F64 && s->coll == GTD_OVERLAP_COLL && s->n >= 2 &&
+           s->n <= kFusedMaxN && s->cb.cont_kind != 1 && s->cb.all_kind != 1 && !s->cb.each_fn;
+}
+
+// The loop graph of paired steps:
+//   open (verdict, kick-drift) -> WHILE(hw) { step A; step B }
+// where a step is the force kernel (with the closing kick and the detection of overlaps) and the
+// resolving kernel (for_all, resolution, the next verdict and kick-drift).  A step after a false verdict
+// does nothing; step B's resolving kernel ends the loop on one, and on a full chunk.
+static int build_paired_graph(gtd_system *s, cudaGraphExec_t *exec) {
+    *exec = nullptr;
+    cudaGraph_t G = nullptr;
+    GTD_CUDA(cudaGraphCreate(&G, 0));
+    cudaStream_t st = s->stream;
+    PassHooks hk;
+    hk.ctl = ctl_of(s);
+    if (s->cb.all_kind == 2) {
+        hk.for_all = 1;
+        hk.weighted = s->cb.mass_weighted;
+        hk.min_cor = s->cb.min_cor;
+        hk.max_cor = s->cb.max_cor;
+        hk.scale = s->cb.scale_factor;
+        hk.n_exp = s->cb.n_exp;
+    }
+    hk.decide = 1;
+    hk.mode = s->cb.cont_kind;
+    hk.bound = s->cb.min_max_cor;
+    hk.probing = s->cb.probing_iters;
+    const int rc = [&]() -> int {
+        GTD_CUDA(cudaGraphConditionalHandleCreate(&hk.handle, G, 1, cudaGraphCondAssignDefault));
+        cudaGraph_t body = nullptr;
+        int r = capture_into(st, G, [&]() -> int {
+            const int q = enqueue_paired_open(s, hk);
+            return q ? q : add_conditional(st, hk.handle, cudaGraphCondTypeWhile, &body);
+        });
+        if (r) return r;
+        r = capture_into(st, body, [&]() -> int {
+            const int q = enqueue_paired_step(s, s->cur ^ 1, hk, false);
+            return q ? q : enqueue_paired_step(s, s->cur, hk, true);
+        });
+        if (r) return r;
+        GTD_CUDA(cudaGraphInstantiate(exec, G, 0));
+        return GTD_OK;
+    }();
+    cudaGraphDestroy(G);
+    if (rc) {
+        if (*exec) cudaGraphExecDestroy(*exec);
+        *exec = nullptr;
+        cudaGetLastError();
+    }
+    return rc;
+}
+
 static int read_ctl(gtd_system *s, CbCtl *h) {
     GTD_CUDA(cudaMemcpyAsync(s->cb_host, s->cb_ctl, sizeof(CbCtl), cudaMemcpyDeviceToHost, s->stream));
     GTD_CUDA(cudaStreamSynchronize(s->stream));
@@ -387,6 +444,8 @@ static int eager_loop(gtd_system *s, uint64_t *waits) {
     }
 }
 
+constexpr int kPaired = 3;
+
 static int graph_loop(gtd_system *s, cudaGraphExec_t exec, int flips, uint64_t per_step, int verdicts_apart,
                       uint64_t *waits) {
     const int cur0 = s->cur;
@@ -396,9 +455,12 @@ static int graph_loop(gtd_system *s, cudaGraphExec_t exec, int flips, uint64_t p
         int rc = read_ctl(s, &h);
         if (rc) return rc;
         *waits += 1;
-        // reset, first nodes, steps, and the verdicts that run as kernels of their own
-        s->launches += 1 + h.iter + h.chunk * per_step +
-                       (verdicts_apart == 2 ? h.chunk + 1 : verdicts_apart == 1 ? (h.chunk + 1) / 2 : 0);
+        // reset, first nodes, steps, and the verdicts that run as kernels of their own; paired steps: the
+        // opening kernel and both steps of each iteration
+        s->launches += verdicts_apart == kPaired
+                           ? 1 + (h.chunk + 1) / 2 * 2 * per_step
+                           : 1 + h.iter + h.chunk * per_step +
+                                 (verdicts_apart == 2 ? h.chunk + 1 : verdicts_apart == 1 ? (h.chunk + 1) / 2 : 0);
         if (h.status) return status_error(h.status);
         if (h.done || h.capped) break;
         if (h.chunk < kChunkSteps) return fail(GTD_ERR_CUDA, "callback loop chunk ended early (%llu steps)", h.chunk);
@@ -525,8 +587,14 @@ int gtd_system_evolve_callbacks(gtd_system *s, int method, uint64_t max_steps, u
         if (s->coll != GTD_NO_COLL) rc = prepare_collisions(s, &coll_status);
         if (!rc) rc = cb_prepare_steps(s);
         if (rc) return rc;
-        if (build_loop_graph(s, coll_status, &exec, &flips, &per_step, &verdicts_apart) != GTD_OK)
+        if (paired_steps(s, branch)) {
+            flips = 1;
+            per_step = 2;
+            verdicts_apart = kPaired;
+            if (build_paired_graph(s, &exec) != GTD_OK) exec = nullptr;
+        } else if (build_loop_graph(s, coll_status, &exec, &flips, &per_step, &verdicts_apart) != GTD_OK) {
             exec = nullptr;  // eager below
+        }
     }
     if (exec) {
         s->cb_graph = true;

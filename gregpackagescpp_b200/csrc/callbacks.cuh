@@ -48,6 +48,27 @@ __device__ __forceinline__ double cb_block_sum(double v, double *sh) {
     return r;
 }
 
+// Three sums at once: per value cb_block_sum's additions in its order.  sh: 96 doubles.
+__device__ __forceinline__ void cb_block_sum3(double (&v)[3], double *sh) {
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5, nw = blockDim.x >> 5;
+    for (int d = 16; d > 0; d >>= 1)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) v[k] += __shfl_down_sync(0xffffffffu, v[k], d);
+    if (lane == 0)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) sh[32 * k + w] = v[k];
+    __syncthreads();
+    if (w < 3) {  // warp k: sum k
+        double s = lane < nw ? sh[32 * w + lane] : 0.0;
+        for (int d = 16; d > 0; d >>= 1) s += __shfl_down_sync(0xffffffffu, s, d);
+        if (lane == 0) sh[32 * w] = s;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 3; ++k) v[k] = sh[32 * k];
+    __syncthreads();
+}
+
 __device__ __forceinline__ double cb_block_min(double v, double *sh) {
     const int t = threadIdx.x, lane = t & 31, w = t >> 5, nw = blockDim.x >> 5;
     for (int d = 16; d > 0; d >>= 1) v = fmin(v, __shfl_down_sync(0xffffffffu, v, d));
@@ -116,38 +137,41 @@ __device__ __forceinline__ double cb_rest_from_distance(const double4 &p, const 
 // the sum, so it carries: com = (com + sum x) / N, or (com + sum m x) / M with GREGSYS_MERGERS;
 // then, with set_rest, every body takes its restitution from the distance to it.  The sum is
 // strided over kForAllLanes threads whatever the block size (512 or more), so every caller gets the
-// same bits.  sh: 32 doubles, com: 3 doubles of shared memory.
+// same bits.  sh: 96 doubles, com: 3 doubles of shared memory.  With set_rest, returns the smallest
+// restitution the thread set (INFINITY for none).
 constexpr int kForAllLanes = 512;
 
-__device__ __forceinline__ void cb_for_all_block(int64_t n, const double4 *pm, double *rest, CbCtl *c, int weighted,
+__device__ __forceinline__ double cb_for_all_block(int64_t n, const double4 *pm, double *rest, CbCtl *c, int weighted,
                                                  int set_rest, double min_cor, double max_cor, double scale,
                                                  double n_exp, double *sh, double *com) {
-    double sx = 0.0, sy = 0.0, sz = 0.0;
+    double s[3] = {0.0, 0.0, 0.0};
     for (int64_t i = threadIdx.x; threadIdx.x < kForAllLanes && i < n; i += kForAllLanes) {
         const double4 p = pm[i];
         if (weighted) {
-            sx += p.w * p.x;
-            sy += p.w * p.y;
-            sz += p.w * p.z;
+            s[0] += p.w * p.x;
+            s[1] += p.w * p.y;
+            s[2] += p.w * p.z;
         } else {
-            sx += p.x;
-            sy += p.y;
-            sz += p.z;
+            s[0] += p.x;
+            s[1] += p.y;
+            s[2] += p.z;
         }
     }
-    sx = cb_block_sum(sx, sh);
-    sy = cb_block_sum(sy, sh);
-    sz = cb_block_sum(sz, sh);
-    if (threadIdx.x == 0) {
-        com[0] = c->com[0] = (c->com[0] + sx) / c->divisor;
-        com[1] = c->com[1] = (c->com[1] + sy) / c->divisor;
-        com[2] = c->com[2] = (c->com[2] + sz) / c->divisor;
+    cb_block_sum3(s, sh);
+    if (threadIdx.x < 3) {
+        const int k = threadIdx.x;
+        com[k] = c->com[k] = (c->com[k] + (k == 0 ? s[0] : k == 1 ? s[1] : s[2])) / c->divisor;
     }
     __syncthreads();
-    if (!set_rest) return;
-    for (int64_t i = threadIdx.x; i < n; i += blockDim.x)
-        rest[i] = cb_rest_from_distance(pm[i], com, min_cor, max_cor, scale, n_exp);
+    double lo = INFINITY;
+    if (!set_rest) return lo;
+    for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
+        const double r = cb_rest_from_distance(pm[i], com, min_cor, max_cor, scale, n_exp);
+        rest[i] = r;
+        lo = fmin(lo, r);
+    }
     __syncthreads();
+    return lo;
 }
 
 // What a collision pass's resolving CTA takes over inside the callback loop: random_comet's

@@ -22,6 +22,7 @@
 
 #include "callbacks.cuh"
 #include "gtd_internal.cuh"
+#include "gtd_math.cuh"
 #include "gtd_system.cuh"
 
 namespace gtd {
@@ -506,7 +507,7 @@ __global__ void __launch_bounds__(kResolveThreads, 1) restitution_kernel(int64_t
                                                                          double *rest, double4 *vel, int *status,
                                                                          PassHooks hk) {
     extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ double hsh[32];
+    __shared__ double hsh[96];
     __shared__ double hcom[3];
     const int c = *count;
     if (hk.for_all)
@@ -528,6 +529,170 @@ __global__ void __launch_bounds__(kResolveThreads, 1) restitution_kernel(int64_t
             cudaGraphSetConditional(hk.handle, go ? 1u : 0u);
         }
     }
+}
+
+// ---- the callback loop's steps as two kernels each ------------------------------------------------
+// A small system's step is a chain of short kernels whose latency bounds it: kick-drift, force and kick,
+// detection, resolution, and every other step the loop's own nodes.  Here the force kernel also detects
+// the overlaps, on the separations it forms anyway, and the resolving CTA, which knows the next verdict,
+// also opens the next step: two kernels.  Every value is the one the separate kernels give.  512 steps of
+// 727 bodies with both functors: 15.3 ms in five kernels a step and conditional nodes, 9.0 ms in two.
+
+// The force at src with the closing half kick, and the overlapping pairs o < i, as fused_small_kernel
+// (direct.cu) and overlap_pairs_kernel do.  I bodies per warp, kPairSlices warps share them.
+constexpr int kPairSlices = 4;
+
+template <int I>
+__global__ void __launch_bounds__(kPairSlices * 32) paired_force_kernel(int64_t n, const double4 *__restrict__ src,
+                                                                        const double *__restrict__ rad, double G,
+                                                                        double h2, double4 *vel, double4 *acc,
+                                                                        Cand *cand, int *count, int cap,
+                                                                        const CbCtl *ctl) {
+    __shared__ double part[kPairSlices][I][3];
+    const int slice = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t i0 = (int64_t)blockIdx.x * I;
+    const bool go = ctl->go != 0;  // a step after a false verdict writes nothing
+    double4 p[I];
+    double ri[I], ax[I], ay[I], az[I];
+#pragma unroll
+    for (int k = 0; k < I; ++k) {
+        const bool have = i0 + k < n;
+        p[k] = have ? src[i0 + k] : make_double4(0.0, 0.0, 0.0, 0.0);
+        ri[k] = have ? rad[i0 + k] : 0.0;
+        ax[k] = ay[k] = az[k] = 0.0;
+    }
+#pragma unroll 4
+    for (int64_t j = (int64_t)slice * 32 + lane; j < n; j += 32 * kPairSlices) {
+        const double4 q = src[j];
+        const double rj = rad[j];
+        const double gm = q.w * G;
+#pragma unroll
+        for (int k = 0; k < I; ++k) {
+            const double dx = q.x - p[k].x, dy = q.y - p[k].y, dz = q.z - p[k].z;
+            const double r2 = fma(dz, dz, fma(dy, dy, dx * dx));
+            const double sc = r2 > 0.0 ? gm * inv_r3(r2) : 0.0;
+            ax[k] = fma(sc, dx, ax[k]);
+            ay[k] = fma(sc, dy, ay[k]);
+            az[k] = fma(sc, dz, az[k]);
+            // r2 and the exact test's d2 differ by a few 2^-53 (or by underflows, the addend): past this
+            // bound that test finds nothing
+            const double rsum = __dadd_rn(ri[k], rj), r2s = __dmul_rn(rsum, rsum);
+            if (r2 <= fma(r2s, 1.0 + 0x1p-38, 1e-300) && j > i0 + k && i0 + k < n && go) {
+                const double d2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
+                if (!(d2 > __dmul_rn(r2s, 1.0 + 0x1p-40))) {
+                    const double d = sqrt(d2);
+                    if (rsum > d) {
+                        const int at = atomicAdd(count, 1);
+                        if (at < cap) cand[at] = Cand{(int32_t)(i0 + k), (int32_t)j, d};
+                    }
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int k = 0; k < I; ++k) {
+            ax[k] += __shfl_xor_sync(0xffffffffu, ax[k], o);
+            ay[k] += __shfl_xor_sync(0xffffffffu, ay[k], o);
+            az[k] += __shfl_xor_sync(0xffffffffu, az[k], o);
+        }
+    if (lane == 0) {
+#pragma unroll
+        for (int k = 0; k < I; ++k) {
+            part[slice][k][0] = ax[k];
+            part[slice][k][1] = ay[k];
+            part[slice][k][2] = az[k];
+        }
+    }
+    __syncthreads();
+    if (go && slice == 0 && lane < I && i0 + lane < n) {
+        double a[3];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            a[d] = part[0][lane][d];
+#pragma unroll
+            for (int k = 1; k < kPairSlices; ++k) a[d] += part[k][lane][d];
+        }
+        const int64_t i = i0 + lane;
+        acc[i] = make_double4(a[0], a[1], a[2], 0.0);
+        double4 v = vel[i];
+        v.x = fma(h2, a[0], v.x); v.y = fma(h2, a[1], v.y); v.z = fma(h2, a[2], v.z);
+        vel[i] = v;
+    }
+}
+
+// The opening half kick and drift of a step (kick_drift_kernel, direct.cu), by one CTA.
+__device__ __forceinline__ void paired_kick_drift(int64_t n, const double4 *cur, double4 *dst, double4 *vel,
+                                                  const double4 *acc, double h) {
+    const double h2 = 0.5 * h;
+    for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
+        const double4 x = cur[i], a = acc[i];
+        double4 v = vel[i];
+        v.x = fma(h2, a.x, v.x); v.y = fma(h2, a.y, v.y); v.z = fma(h2, a.z, v.z);
+        vel[i] = v;
+        dst[i] = make_double4(fma(h, v.x, x.x), fma(h, v.y, x.y), fma(h, v.z, x.z), x.w);
+    }
+}
+
+// First node of a launch: the verdict and, if it is true, the opening of the first step.
+__global__ void __launch_bounds__(kResolveThreads) paired_open_kernel(int64_t n, const double4 *cur, double4 *dst,
+                                                                      double4 *vel, const double4 *acc, const double *rest,
+                                                                      double h, const int *status, PassHooks hk) {
+    __shared__ double sh[32];
+    __shared__ int go_s;
+    const double lo = hk.mode == 2 ? cb_min_rest(rest, n, sh) : INFINITY;
+    if (threadIdx.x == 0) {
+        hk.ctl->iter = 0;
+        hk.ctl->chunk = 0;
+        go_s = cb_verdict(hk.ctl, hk.mode, lo, hk.bound, hk.probing, status);
+        cudaGraphSetConditional(hk.handle, go_s ? 1u : 0u);
+    }
+    __syncthreads();
+    if (go_s) paired_kick_drift(n, cur, dst, vel, acc, h);
+}
+
+// The step's for_all_bods, its resolution, the next verdict (unless the chunk is full: the next launch's
+// first node takes it) and the next step's opening.  closes: the last kernel of an iteration.
+__global__ void __launch_bounds__(kResolveThreads, 1)
+    paired_resolve_kernel(int64_t n, Cand *cand, int *count, int cap, const double4 *cur, double4 *dst, double4 *vel,
+                          const double4 *acc, double *rest, double h, int *status, PassHooks hk, int closes) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ double sh[96];
+    __shared__ double com[3];
+    __shared__ int go_s;
+    if (!hk.ctl->go) {
+        if (closes && threadIdx.x == 0) cudaGraphSetConditional(hk.handle, 0u);
+        return;
+    }
+    const int c = *count;
+    double lo = INFINITY;
+    if (hk.for_all) {
+        lo = cb_for_all_block(n, cur, rest, hk.ctl, hk.weighted, 1, hk.min_cor, hk.max_cor, hk.scale, hk.n_exp, sh, com);
+    } else if (hk.mode == 2) {
+        for (int64_t i = threadIdx.x; i < n; i += blockDim.x) lo = fmin(lo, rest[i]);
+    }
+    if (c > cap) {
+        if (threadIdx.x == 0) *status = GTD_ERR_CAPACITY;
+    } else if (c > kFastCand) {
+        if (threadIdx.x == 0) resolve_serial(cand, c, cap, nullptr, cur, rest, vel);
+    } else if (c > 0) {
+        resolve_groups(smem, cand, c, nullptr, cur, rest, vel);
+    }
+    __syncthreads();
+    if (hk.mode == 2) lo = cb_block_min(lo, sh);
+    if (threadIdx.x == 0) {
+        if (c <= cap) *count = 0;
+        if (hk.ctl->chunk >= kChunkSteps) {
+            go_s = 0;
+            hk.ctl->go = 0;
+        } else {
+            go_s = cb_verdict(hk.ctl, hk.mode, lo, hk.bound, hk.probing, status);
+        }
+        if (closes) cudaGraphSetConditional(hk.handle, go_s ? 1u : 0u);
+    }
+    __syncthreads();
+    if (go_s) paired_kick_drift(n, cur, dst, vel, acc, h);
 }
 
 // ---- Barnes-Hut path: bh_s_coll (gregsys.hpp:631-688) ----------------------------------------
@@ -734,6 +899,8 @@ static int ensure_coll(gtd_system *s) {
     if (s->coll_buf && s->coll_bytes >= need) return GTD_OK;
     GTD_CUDA(cudaFuncSetAttribute(restitution_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)resolve_smem_bytes()));
+    GTD_CUDA(cudaFuncSetAttribute(paired_resolve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)resolve_smem_bytes()));
     release_collide(s);
     GTD_CUDA(cudaMalloc(&s->coll_buf, need));
     s->coll_bytes = need;
@@ -820,6 +987,34 @@ int enqueue_collisions(gtd_system *s, const PassHooks *hooks) {
                                                                          hk);
     GTD_CHECK_LAUNCH();
     s->launches += 2;
+    return GTD_OK;
+}
+
+int enqueue_paired_open(gtd_system *s, const PassHooks &hk) {
+    CollPtrs p = coll_ptrs(s);
+    paired_open_kernel<<<1, kResolveThreads, 0, s->stream>>>(s->n, s->pm[s->cur], s->pm[s->cur ^ 1], s->vel, s->acc, s->rest,
+                                                            s->dt, p.status, hk);
+    GTD_CHECK_LAUNCH();
+    return GTD_OK;
+}
+
+// Two bodies per warp from the size where they pay in the fused force kernel.
+int enqueue_paired_step(gtd_system *s, int at, const PassHooks &hk, bool closes) {
+    CollPtrs p = coll_ptrs(s);
+    cudaStream_t st = s->stream;
+    const double4 *x = s->pm[at];
+    const double h2 = 0.5 * s->dt;
+    if (s->n <= 900)
+        paired_force_kernel<1><<<(unsigned)s->n, kPairSlices * 32, 0, st>>>(s->n, x, s->rad, s->G, h2, s->vel, s->acc, p.cand,
+                                                                           p.count, kMaxCand, hk.ctl);
+    else
+        paired_force_kernel<2><<<(unsigned)((s->n + 1) / 2), kPairSlices * 32, 0, st>>>(
+            s->n, x, s->rad, s->G, h2, s->vel, s->acc, p.cand, p.count, kMaxCand, hk.ctl);
+    GTD_CHECK_LAUNCH();
+    paired_resolve_kernel<<<1, kResolveThreads, resolve_smem_bytes(), st>>>(s->n, p.cand, p.count, kMaxCand, x,
+                                                                            s->pm[at ^ 1], s->vel, s->acc, s->rest, s->dt,
+                                                                            p.status, hk, closes ? 1 : 0);
+    GTD_CHECK_LAUNCH();
     return GTD_OK;
 }
 

@@ -220,6 +220,10 @@ struct PassHooks;
 int prepare_collisions(gtd_system *s, int **status);
 int enqueue_collisions(gtd_system *s, const gtd::PassHooks *hooks);
 int run_collisions(gtd_system *s);
+// the callback loop's steps as two kernels each (collide.cu): the opening verdict and kick-drift, and a
+// step at the positions in pm[at]
+int enqueue_paired_open(gtd_system *s, const gtd::PassHooks &hk);
+int enqueue_paired_step(gtd_system *s, int at, const gtd::PassHooks &hk, bool closes);
 // pieces of evolve for the callback-driven loop (system.cu)
 int cb_evolve_begin(gtd_system *s, int method);
 int cb_direct_step(gtd_system *s);
