@@ -137,11 +137,10 @@ __device__ __forceinline__ double cb_rest_from_distance(const double4 &p, const 
 // the sum, so it carries: com = (com + sum x) / N, or (com + sum m x) / M with GREGSYS_MERGERS;
 // then, with set_rest, every body takes its restitution from the distance to it.  The sum is
 // strided over kForAllLanes threads whatever the block size (512 or more), so every caller gets the
-// same bits.  sh: 96 doubles, com: 3 doubles of shared memory.  With set_rest, returns the smallest
-// restitution the thread set (INFINITY for none).
+// same bits.  sh: 96 doubles, com: 3 doubles of shared memory.
 constexpr int kForAllLanes = 512;
 
-__device__ __forceinline__ double cb_for_all_block(int64_t n, const double4 *pm, double *rest, CbCtl *c, int weighted,
+__device__ __forceinline__ void cb_for_all_block(int64_t n, const double4 *pm, double *rest, CbCtl *c, int weighted,
                                                  int set_rest, double min_cor, double max_cor, double scale,
                                                  double n_exp, double *sh, double *com) {
     double s[3] = {0.0, 0.0, 0.0};
@@ -163,15 +162,10 @@ __device__ __forceinline__ double cb_for_all_block(int64_t n, const double4 *pm,
         com[k] = c->com[k] = (c->com[k] + (k == 0 ? s[0] : k == 1 ? s[1] : s[2])) / c->divisor;
     }
     __syncthreads();
-    double lo = INFINITY;
-    if (!set_rest) return lo;
-    for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
-        const double r = cb_rest_from_distance(pm[i], com, min_cor, max_cor, scale, n_exp);
-        rest[i] = r;
-        lo = fmin(lo, r);
-    }
+    if (!set_rest) return;
+    for (int64_t i = threadIdx.x; i < n; i += blockDim.x)
+        rest[i] = cb_rest_from_distance(pm[i], com, min_cor, max_cor, scale, n_exp);
     __syncthreads();
-    return lo;
 }
 
 // What a collision pass's resolving CTA takes over inside the callback loop: random_comet's

@@ -533,77 +533,99 @@ __global__ void __launch_bounds__(kResolveThreads, 1) restitution_kernel(int64_t
 
 // ---- the callback loop's steps as two kernels each ------------------------------------------------
 // A small system's step is a chain of short kernels whose latency bounds it: kick-drift, force and kick,
-// detection, resolution, and every other step the loop's own nodes.  Here the force kernel also detects
-// the overlaps, on the separations it forms anyway, and the resolving CTA, which knows the next verdict,
-// also opens the next step: two kernels.  Every value is the one the separate kernels give.  512 steps of
-// 727 bodies with both functors: 15.3 ms in five kernels a step and conditional nodes, 9.0 ms in two.
+// detection, resolution with for_all_bods, and every other step the loop's own nodes.  Here all that is
+// per body stands in the force kernel: both half kicks, the restitution (a pow, by a warp of its own,
+// behind the force), the detection, on the separations the force forms anyway, and the positions the next
+// step starts from, right unless a collision changes a velocity.  The resolving CTA is left with the rare
+// collisions, the centre of the next positions and the verdict: one round of loads and one block
+// reduction when nothing collides.  Every value is the one the separate kernels give.  512 steps of 727
+// bodies with both functors: 15.3 ms in five kernels a step and conditional nodes, 9.0 ms in two with
+// for_all_bods and the kick-drift in the resolving CTA (where they took most of its time), 5.1 ms
+// so.  A programmatic launch of either kernel gave nothing (5.1 ms).
 
-// The force at src with the closing half kick, and the overlapping pairs o < i, as fused_small_kernel
-// (direct.cu) and overlap_pairs_kernel do.  I bodies per warp, kPairSlices warps share them.
+// The force at src, the half kicks around it, the next positions (in dst), the overlapping pairs o < i
+// and, with hk.for_all, the restitution, as fused_small_kernel and kick_drift_kernel (direct.cu),
+// overlap_pairs_kernel and cb_for_all_block do.  I bodies per block, shared by kPairSlices warps; one
+// more warp for the restitution.
 constexpr int kPairSlices = 4;
 
+__device__ __forceinline__ double4 half_kick(double4 v, const double4 &a, double h2) {
+    v.x = fma(h2, a.x, v.x); v.y = fma(h2, a.y, v.y); v.z = fma(h2, a.z, v.z);
+    return v;
+}
+
+// A step's opening half kick and drift: where its force is evaluated.
+__device__ __forceinline__ double4 opened(const double4 &x, const double4 &v0, const double4 &a, double h) {
+    const double4 v = half_kick(v0, a, 0.5 * h);
+    return make_double4(fma(h, v.x, x.x), fma(h, v.y, x.y), fma(h, v.z, x.z), x.w);
+}
+
 template <int I>
-__global__ void __launch_bounds__(kPairSlices * 32) paired_force_kernel(int64_t n, const double4 *__restrict__ src,
-                                                                        const double *__restrict__ rad, double G,
-                                                                        double h2, double4 *vel, double4 *acc,
-                                                                        Cand *cand, int *count, int cap,
-                                                                        const CbCtl *ctl) {
+__global__ void __launch_bounds__((kPairSlices + 1) * 32)
+    paired_force_kernel(int64_t n, const double4 *__restrict__ src, double4 *__restrict__ dst,
+                        const double *__restrict__ rad, double G, double h, double4 *vel, double4 *acc, double *rest,
+                        Cand *cand, int *count, int cap, PassHooks hk) {
     __shared__ double part[kPairSlices][I][3];
     const int slice = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t i0 = (int64_t)blockIdx.x * I;
-    const bool go = ctl->go != 0;  // a step after a false verdict writes nothing
-    double4 p[I];
-    double ri[I], ax[I], ay[I], az[I];
-#pragma unroll
-    for (int k = 0; k < I; ++k) {
-        const bool have = i0 + k < n;
-        p[k] = have ? src[i0 + k] : make_double4(0.0, 0.0, 0.0, 0.0);
-        ri[k] = have ? rad[i0 + k] : 0.0;
-        ax[k] = ay[k] = az[k] = 0.0;
-    }
-#pragma unroll 4
-    for (int64_t j = (int64_t)slice * 32 + lane; j < n; j += 32 * kPairSlices) {
-        const double4 q = src[j];
-        const double rj = rad[j];
-        const double gm = q.w * G;
+    const bool go = hk.ctl->go != 0;  // a step after a false verdict writes nothing
+    if (slice < kPairSlices) {
+        double4 p[I];
+        double ri[I], ax[I], ay[I], az[I];
 #pragma unroll
         for (int k = 0; k < I; ++k) {
-            const double dx = q.x - p[k].x, dy = q.y - p[k].y, dz = q.z - p[k].z;
-            const double r2 = fma(dz, dz, fma(dy, dy, dx * dx));
-            const double sc = r2 > 0.0 ? gm * inv_r3(r2) : 0.0;
-            ax[k] = fma(sc, dx, ax[k]);
-            ay[k] = fma(sc, dy, ay[k]);
-            az[k] = fma(sc, dz, az[k]);
-            // r2 and the exact test's d2 differ by a few 2^-53 (or by underflows, the addend): past this
-            // bound that test finds nothing
-            const double rsum = __dadd_rn(ri[k], rj), r2s = __dmul_rn(rsum, rsum);
-            if (r2 <= fma(r2s, 1.0 + 0x1p-38, 1e-300) && j > i0 + k && i0 + k < n && go) {
-                const double d2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
-                if (!(d2 > __dmul_rn(r2s, 1.0 + 0x1p-40))) {
-                    const double d = sqrt(d2);
-                    if (rsum > d) {
-                        const int at = atomicAdd(count, 1);
-                        if (at < cap) cand[at] = Cand{(int32_t)(i0 + k), (int32_t)j, d};
+            const bool have = i0 + k < n;
+            p[k] = have ? src[i0 + k] : make_double4(0.0, 0.0, 0.0, 0.0);
+            ri[k] = have ? rad[i0 + k] : 0.0;
+            ax[k] = ay[k] = az[k] = 0.0;
+        }
+#pragma unroll 4
+        for (int64_t j = (int64_t)slice * 32 + lane; j < n; j += 32 * kPairSlices) {
+            const double4 q = src[j];
+            const double rj = rad[j];
+            const double gm = q.w * G;
+#pragma unroll
+            for (int k = 0; k < I; ++k) {
+                const double dx = q.x - p[k].x, dy = q.y - p[k].y, dz = q.z - p[k].z;
+                const double r2 = fma(dz, dz, fma(dy, dy, dx * dx));
+                const double sc = r2 > 0.0 ? gm * inv_r3(r2) : 0.0;
+                ax[k] = fma(sc, dx, ax[k]);
+                ay[k] = fma(sc, dy, ay[k]);
+                az[k] = fma(sc, dz, az[k]);
+                // r2 and the exact test's d2 differ by a few 2^-53 (or by underflows, the addend): past
+                // this bound that test finds nothing
+                const double rsum = __dadd_rn(ri[k], rj), r2s = __dmul_rn(rsum, rsum);
+                if (r2 <= fma(r2s, 1.0 + 0x1p-38, 1e-300) && j > i0 + k && i0 + k < n && go) {
+                    const double d2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
+                    if (!(d2 > __dmul_rn(r2s, 1.0 + 0x1p-40))) {
+                        const double d = sqrt(d2);
+                        if (rsum > d) {
+                            const int at = atomicAdd(count, 1);
+                            if (at < cap) cand[at] = Cand{(int32_t)(i0 + k), (int32_t)j, d};
+                        }
                     }
                 }
             }
         }
-    }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
+        for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
-        for (int k = 0; k < I; ++k) {
-            ax[k] += __shfl_xor_sync(0xffffffffu, ax[k], o);
-            ay[k] += __shfl_xor_sync(0xffffffffu, ay[k], o);
-            az[k] += __shfl_xor_sync(0xffffffffu, az[k], o);
+            for (int k = 0; k < I; ++k) {
+                ax[k] += __shfl_xor_sync(0xffffffffu, ax[k], o);
+                ay[k] += __shfl_xor_sync(0xffffffffu, ay[k], o);
+                az[k] += __shfl_xor_sync(0xffffffffu, az[k], o);
+            }
+        if (lane == 0) {
+#pragma unroll
+            for (int k = 0; k < I; ++k) {
+                part[slice][k][0] = ax[k];
+                part[slice][k][1] = ay[k];
+                part[slice][k][2] = az[k];
+            }
         }
-    if (lane == 0) {
-#pragma unroll
-        for (int k = 0; k < I; ++k) {
-            part[slice][k][0] = ax[k];
-            part[slice][k][1] = ay[k];
-            part[slice][k][2] = az[k];
-        }
+    } else if (go && lane < I && i0 + lane < n) {  // this warp is there only with hk.for_all
+        rest[i0 + lane] =
+            cb_rest_from_distance(src[i0 + lane], hk.ctl->com, hk.min_cor, hk.max_cor, hk.scale, hk.n_exp);
     }
     __syncthreads();
     if (go && slice == 0 && lane < I && i0 + lane < n) {
@@ -615,84 +637,126 @@ __global__ void __launch_bounds__(kPairSlices * 32) paired_force_kernel(int64_t 
             for (int k = 1; k < kPairSlices; ++k) a[d] += part[k][lane][d];
         }
         const int64_t i = i0 + lane;
-        acc[i] = make_double4(a[0], a[1], a[2], 0.0);
-        double4 v = vel[i];
-        v.x = fma(h2, a[0], v.x); v.y = fma(h2, a[1], v.y); v.z = fma(h2, a[2], v.z);
+        const double h2 = 0.5 * h;
+        const double4 x = src[i], a0 = acc[i], a1 = make_double4(a[0], a[1], a[2], 0.0);
+        const double4 v = half_kick(half_kick(vel[i], a0, h2), a1, h2);
+        acc[i] = a1;
         vel[i] = v;
+        dst[i] = opened(x, v, a1, h);
     }
 }
 
-// The opening half kick and drift of a step (kick_drift_kernel, direct.cu), by one CTA.
-__device__ __forceinline__ void paired_kick_drift(int64_t n, const double4 *cur, double4 *dst, double4 *vel,
-                                                  const double4 *acc, double h) {
-    const double h2 = 0.5 * h;
-    for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
-        const double4 x = cur[i], a = acc[i];
-        double4 v = vel[i];
-        v.x = fma(h2, a.x, v.x); v.y = fma(h2, a.y, v.y); v.z = fma(h2, a.z, v.z);
-        vel[i] = v;
-        dst[i] = make_double4(fma(h, v.x, x.x), fma(h, v.y, x.y), fma(h, v.z, x.z), x.w);
+// One thread's part of the sums of for_all_bods' centre, strided and ordered as cb_for_all_block's.
+__device__ __forceinline__ void paired_centre_add(const double4 &p, int weighted, double (&s)[3]) {
+    static_assert(kForAllLanes == kResolveThreads, "the centre's sums are strided over kForAllLanes threads");
+    if (weighted) {
+        s[0] += p.w * p.x;
+        s[1] += p.w * p.y;
+        s[2] += p.w * p.z;
+    } else {
+        s[0] += p.x;
+        s[1] += p.y;
+        s[2] += p.z;
     }
 }
 
-// First node of a launch: the verdict and, if it is true, the opening of the first step.
-__global__ void __launch_bounds__(kResolveThreads) paired_open_kernel(int64_t n, const double4 *cur, double4 *dst,
-                                                                      double4 *vel, const double4 *acc, const double *rest,
-                                                                      double h, const int *status, PassHooks hk) {
-    __shared__ double sh[32];
-    __shared__ int go_s;
-    const double lo = hk.mode == 2 ? cb_min_rest(rest, n, sh) : INFINITY;
-    if (threadIdx.x == 0) {
-        hk.ctl->iter = 0;
-        hk.ctl->chunk = 0;
-        go_s = cb_verdict(hk.ctl, hk.mode, lo, hk.bound, hk.probing, status);
-        cudaGraphSetConditional(hk.handle, go_s ? 1u : 0u);
-    }
+// The end of a step and of the opening: the verdict (below: some restitution is below the bound) and, if
+// it is true, the centre that the step's for_all_bods carries on to (s: per-thread sums).  Warps 0 to 2
+// sum a component each and find the verdict from c, the control block as the kernel began; thread 0
+// writes it.  full: the chunk is, no verdict.
+__device__ __forceinline__ void paired_close(const PassHooks &hk, CbCtl c, bool below, double (&s)[3], int status, bool full,
+                                             bool set_handle, double *sh) {
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5, nw = kResolveThreads >> 5;
+    for (int d = 16; d > 0; d >>= 1)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) s[k] += __shfl_down_sync(0xffffffffu, s[k], d);
+    if (lane == 0)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) sh[32 * k + w] = s[k];
     __syncthreads();
-    if (go_s) paired_kick_drift(n, cur, dst, vel, acc, h);
+    if (w >= 3) return;
+    bool go = false;
+    if (!full) go = cb_verdict(&c, hk.mode, below ? 0.0 : 1.0, 1.0, hk.probing, &status);
+    double sum = lane < nw ? sh[32 * w + lane] : 0.0;
+    for (int d = 16; d > 0; d >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, d);
+    if (lane != 0) return;
+    CbCtl *o = hk.ctl;
+    if (go && hk.for_all) o->com[w] = ((w == 0 ? c.com[0] : w == 1 ? c.com[1] : c.com[2]) + sum) / c.divisor;
+    if (w != 0) return;
+    o->go = go ? 1u : 0u;
+    o->done = c.done;
+    o->capped = c.capped;
+    o->status = c.status;
+    o->steps = c.steps;
+    o->chunk = c.chunk;
+    o->count = c.count;
+    if (set_handle) cudaGraphSetConditional(hk.handle, go ? 1u : 0u);
 }
 
-// The step's for_all_bods, its resolution, the next verdict (unless the chunk is full: the next launch's
-// first node takes it) and the next step's opening.  closes: the last kernel of an iteration.
+// First node of a launch: the verdict, the first step's positions (for a false verdict nobody reads
+// them) and its centre.
+__global__ void __launch_bounds__(kResolveThreads) paired_open_kernel(int64_t n, const double4 *cur, double4 *dst,
+                                                                      const double4 *vel, const double4 *acc,
+                                                                      const double *rest, double h, const int *status,
+                                                                      PassHooks hk) {
+    __shared__ double sh[96];
+    CbCtl c = *hk.ctl;
+    c.chunk = 0;
+    const int st = *status;
+    bool below = false;
+    double s[3] = {0.0, 0.0, 0.0};
+    for (int64_t i = threadIdx.x; i < n; i += kResolveThreads) {
+        const double4 p = opened(cur[i], vel[i], acc[i], h);
+        dst[i] = p;
+        paired_centre_add(p, hk.weighted, s);
+        below |= rest[i] < hk.bound;
+    }
+    below = __syncthreads_or(below);  // and every thread has its copy of the control block
+    paired_close(hk, c, below, s, st, false, true, sh);
+}
+
+// The step's resolution (the next positions made anew if anything collided), the next verdict, unless
+// the chunk is full (the next launch's first node takes it), and the next centre.  closes: the last
+// kernel of an iteration.
 __global__ void __launch_bounds__(kResolveThreads, 1)
     paired_resolve_kernel(int64_t n, Cand *cand, int *count, int cap, const double4 *cur, double4 *dst, double4 *vel,
-                          const double4 *acc, double *rest, double h, int *status, PassHooks hk, int closes) {
+                          const double4 *acc, const double *rest, double h, int *status, PassHooks hk, int closes) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ double sh[96];
-    __shared__ double com[3];
-    __shared__ int go_s;
-    if (!hk.ctl->go) {
+    const CbCtl ctl = *hk.ctl;
+    const int c = *count;
+    int st = *status;
+    bool below = false;
+    double s[3] = {0.0, 0.0, 0.0};
+#pragma unroll 2
+    for (int64_t i = threadIdx.x; i < n; i += kResolveThreads) {
+        paired_centre_add(dst[i], hk.weighted, s);
+        below |= rest[i] < hk.bound;
+    }
+    if (!ctl.go) {
         if (closes && threadIdx.x == 0) cudaGraphSetConditional(hk.handle, 0u);
         return;
     }
-    const int c = *count;
-    double lo = INFINITY;
-    if (hk.for_all) {
-        lo = cb_for_all_block(n, cur, rest, hk.ctl, hk.weighted, 1, hk.min_cor, hk.max_cor, hk.scale, hk.n_exp, sh, com);
-    } else if (hk.mode == 2) {
-        for (int64_t i = threadIdx.x; i < n; i += blockDim.x) lo = fmin(lo, rest[i]);
-    }
-    if (c > cap) {
-        if (threadIdx.x == 0) *status = GTD_ERR_CAPACITY;
-    } else if (c > kFastCand) {
-        if (threadIdx.x == 0) resolve_serial(cand, c, cap, nullptr, cur, rest, vel);
-    } else if (c > 0) {
-        resolve_groups(smem, cand, c, nullptr, cur, rest, vel);
-    }
-    __syncthreads();
-    if (hk.mode == 2) lo = cb_block_min(lo, sh);
-    if (threadIdx.x == 0) {
-        if (c <= cap) *count = 0;
-        if (hk.ctl->chunk >= kChunkSteps) {
-            go_s = 0;
-            hk.ctl->go = 0;
+    if (c > 0) {
+        if (c > cap) {
+            st = GTD_ERR_CAPACITY;
+            if (threadIdx.x == 0) *status = st;
+        } else if (c > kFastCand) {
+            if (threadIdx.x == 0) resolve_serial(cand, c, cap, nullptr, cur, rest, vel);
         } else {
-            go_s = cb_verdict(hk.ctl, hk.mode, lo, hk.bound, hk.probing, status);
+            resolve_groups(smem, cand, c, nullptr, cur, rest, vel);
         }
-        if (closes) cudaGraphSetConditional(hk.handle, go_s ? 1u : 0u);
+        __syncthreads();
+        if (threadIdx.x == 0 && c <= cap) *count = 0;
+        s[0] = s[1] = s[2] = 0.0;
+        for (int64_t i = threadIdx.x; i < n; i += kResolveThreads) {
+            const double4 p = opened(cur[i], vel[i], acc[i], h);
+            dst[i] = p;
+            paired_centre_add(p, hk.weighted, s);
+        }
     }
-    __syncthreads();
-    if (go_s) paired_kick_drift(n, cur, dst, vel, acc, h);
+    below = __syncthreads_or(below);  // and every thread has its copy of the control block
+    paired_close(hk, ctl, below, s, st, ctl.chunk >= kChunkSteps, closes != 0, sh);
 }
 
 // ---- Barnes-Hut path: bh_s_coll (gregsys.hpp:631-688) ----------------------------------------
@@ -998,22 +1062,19 @@ int enqueue_paired_open(gtd_system *s, const PassHooks &hk) {
     return GTD_OK;
 }
 
-// Two bodies per warp from the size where they pay in the fused force kernel.
+// Two bodies per block from the size where they pay in the fused force kernel.
 int enqueue_paired_step(gtd_system *s, int at, const PassHooks &hk, bool closes) {
     CollPtrs p = coll_ptrs(s);
     cudaStream_t st = s->stream;
-    const double4 *x = s->pm[at];
-    const double h2 = 0.5 * s->dt;
-    if (s->n <= 900)
-        paired_force_kernel<1><<<(unsigned)s->n, kPairSlices * 32, 0, st>>>(s->n, x, s->rad, s->G, h2, s->vel, s->acc, p.cand,
-                                                                           p.count, kMaxCand, hk.ctl);
-    else
-        paired_force_kernel<2><<<(unsigned)((s->n + 1) / 2), kPairSlices * 32, 0, st>>>(
-            s->n, x, s->rad, s->G, h2, s->vel, s->acc, p.cand, p.count, kMaxCand, hk.ctl);
+    double4 *x = s->pm[at], *dst = s->pm[at ^ 1];
+    const int I = s->n <= 900 ? 1 : 2;
+    auto *f = I == 1 ? paired_force_kernel<1> : paired_force_kernel<2>;
+    f<<<(unsigned)((s->n + I - 1) / I), (kPairSlices + (hk.for_all ? 1 : 0)) * 32, 0, st>>>(
+        s->n, x, dst, s->rad, s->G, s->dt, s->vel, s->acc, s->rest, p.cand, p.count, kMaxCand, hk);
     GTD_CHECK_LAUNCH();
-    paired_resolve_kernel<<<1, kResolveThreads, resolve_smem_bytes(), st>>>(s->n, p.cand, p.count, kMaxCand, x,
-                                                                            s->pm[at ^ 1], s->vel, s->acc, s->rest, s->dt,
-                                                                            p.status, hk, closes ? 1 : 0);
+    paired_resolve_kernel<<<1, kResolveThreads, resolve_smem_bytes(), st>>>(s->n, p.cand, p.count, kMaxCand, x, dst, s->vel,
+                                                                            s->acc, s->rest, s->dt, p.status, hk,
+                                                                            closes ? 1 : 0);
     GTD_CHECK_LAUNCH();
     return GTD_OK;
 }
