@@ -698,12 +698,16 @@ __global__ void integrate_warp_kernel(IntArgs a) {
 // one body per warp and four groups per CTA throughout / with these:
 //   N = 150 2.72 / 2.47, 592 3.37 / 3.37, 727 4.39 / 3.9, 1024 5.04 / 4.77, 1300 7.75 / 5.62, 2000 12.7 / 8.8,
 //   3000 24.0 / 18.0, 4096 35.2 / 25.3
+// Steps that follow one another are chained launches, let go after the pair loop (at the kernel's start the
+// waiting blocks take room that the last ones of this grid need: 1776 7.5 -> 8.5):
+//   N = 150 2.47 -> 2.20, 592 3.37 -> 3.1, 727 3.88 -> 3.75, 1024 4.77 -> 4.26, 2000 8.8 -> 8.9, 4096 25.4 -> 24.9
 constexpr int kFusedSlices = 4;  // warps per group
 
 template <int EPI, int I, int kFusedGroups, int MINB>
 __global__ void __launch_bounds__(kFusedGroups * kFusedSlices * 32, MINB)
     fused_small_kernel(StepArgs st, const double4 *__restrict__ src, double G) {
     __shared__ double part[kFusedSlices][kFusedGroups][I][3];
+    cudaGridDependencySynchronize();
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int bl = w % kFusedGroups, slice = w / kFusedGroups;
     const int64_t i0 = ((int64_t)blockIdx.x * kFusedGroups + bl) * I;
@@ -730,6 +734,7 @@ __global__ void __launch_bounds__(kFusedGroups * kFusedSlices * 32, MINB)
             }
         }
     }
+    cudaTriggerProgrammaticLaunchCompletion();
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
@@ -760,9 +765,9 @@ __global__ void __launch_bounds__(kFusedGroups * kFusedSlices * 32, MINB)
 }
 
 template <int I, int GROUPS, int MINB>
-static void launch_fused(int64_t n, const double4 *src, double G, int epi, const StepArgs &st, cudaStream_t s) {
+static void launch_fused(int64_t n, const double4 *src, double G, int epi, const StepArgs &st, cudaStream_t s, bool early) {
     const unsigned grid = (unsigned)((n + GROUPS * I - 1) / (GROUPS * I));
-    auto go = [&](auto k) { k<<<grid, GROUPS * kFusedSlices * 32, 0, s>>>(st, src, G); };
+    auto go = [&](auto k) { launch_chained(early, k, grid, GROUPS * kFusedSlices * 32, 0, s, st, src, G); };
     switch (epi) {
         case EPI_ACC: go(fused_small_kernel<EPI_ACC, I, GROUPS, MINB>); break;
         case EPI_KDK: go(fused_small_kernel<EPI_KDK, I, GROUPS, MINB>); break;
@@ -776,13 +781,14 @@ static void launch_fused(int64_t n, const double4 *src, double G, int epi, const
     }
 }
 
-int launch_fused_small(int64_t n, const double4 *src, double G, int epi, const StepArgs &st, cudaStream_t s) {
+int launch_fused_small(int64_t n, const double4 *src, double G, int epi, const StepArgs &st, cudaStream_t s,
+                       bool early) {
     if (n == 0) return GTD_OK;
-    if (n <= 900) launch_fused<1, 2, 4>(n, src, G, epi, st, s);
-    else if (n <= 5 * 148 * 2) launch_fused<2, 1, 5>(n, src, G, epi, st, s);
-    else if (n <= 8 * 148 * 2) launch_fused<2, 1, 8>(n, src, G, epi, st, s);
-    else if (n <= 3 * 148 * 8) launch_fused<4, 2, 3>(n, src, G, epi, st, s);
-    else launch_fused<2, 1, 8>(n, src, G, epi, st, s);
+    if (n <= 900) launch_fused<1, 2, 4>(n, src, G, epi, st, s, early);
+    else if (n <= 5 * 148 * 2) launch_fused<2, 1, 5>(n, src, G, epi, st, s, early);
+    else if (n <= 8 * 148 * 2) launch_fused<2, 1, 8>(n, src, G, epi, st, s, early);
+    else if (n <= 3 * 148 * 8) launch_fused<4, 2, 3>(n, src, G, epi, st, s, early);
+    else launch_fused<2, 1, 8>(n, src, G, epi, st, s, early);
     GTD_CHECK_LAUNCH();
     return GTD_OK;
 }

@@ -25,6 +25,25 @@ int cuda_fail(cudaError_t e, const char *what, const char *file, int line);
 
 #define GTD_CHECK_LAUNCH() GTD_CUDA(cudaPeekAtLastError())
 
+// Launches k; with chained, its blocks may be set up while the kernel before it in the stream still runs.
+// Such a kernel begins with cudaGridDependencySynchronize(), so that all memory is as that kernel leaves
+// it, and calls cudaTriggerProgrammaticLaunchCompletion() once a next one's blocks may take its SMs'
+// room.  Errors show in GTD_CHECK_LAUNCH().
+template <typename... P, typename... A>
+void launch_chained(bool chained, void (*k)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, A &&...a) {
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3(grid);
+    c.blockDim = dim3(block);
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    c.attrs = &at;
+    c.numAttrs = chained ? 1 : 0;
+    (void)cudaLaunchKernelEx(&c, k, static_cast<P>(a)...);
+}
+
 // ---- direct-summation work decomposition (stream-K over (i-block, j-tile) pairs) --------------
 //
 // The N x N interaction square is cut into R = ceil(N/BI) rows of i-bodies and J = ceil(N/BJ)
@@ -104,7 +123,8 @@ int noalloc_variant(int precision, int64_t n);
 int force_launch_count(const ForcePlan &p);
 // Up to this many bodies an FP64 force evaluation and its update run as one fused launch.
 constexpr int64_t kFusedMaxN = 4096;
-int launch_fused_small(int64_t n, const double4 *src, double G, int epi, const StepArgs &st, cudaStream_t s);
+int launch_fused_small(int64_t n, const double4 *src, double G, int epi, const StepArgs &st, cudaStream_t s,
+                       bool early = false);
 void remember_variant(int device, int precision, int64_t n, int variant);
 int tuned_variant(int device, int precision, int64_t n);
 size_t partial_bytes(const ForcePlan &p);

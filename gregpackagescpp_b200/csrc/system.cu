@@ -178,7 +178,7 @@ int force_and_integrate(gtd_system *s, const double4 *src, int epi, const StepAr
     int rc;
     if (s->precision == GTD_PREC_F64 && s->n <= kFusedMaxN) {
         if (s->time_force && (rc = timed_event(s))) return rc;
-        rc = launch_fused_small(s->n, src, s->G, epi, st, s->stream);
+        rc = launch_fused_small(s->n, src, s->G, epi, st, s->stream, true);
         if (rc) return rc;
         if (s->time_force && (rc = timed_event(s))) return rc;
         s->launches += 1;
