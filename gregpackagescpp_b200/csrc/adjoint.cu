@@ -432,7 +432,7 @@ static int adj_new(gtd_adjoint **out, int device, int64_t n, uint64_t steps, uin
         A->every = std::max<uint64_t>(1, (uint64_t)std::llround(std::sqrt((double)steps)));
     A->G = G;
     A->h = dt;
-    A->small_force = n <= kFusedMaxN;
+    A->small_force = n <= kFusedAutoMaxN;
     A->small_vjp = n <= kVjpSmallMaxN;
     if (!A->small_force) A->fplan = make_plan(n, GTD_PREC_F64, device, tuned_variant(device, GTD_PREC_F64, n));
     if (!A->small_vjp) {

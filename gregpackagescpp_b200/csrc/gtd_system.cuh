@@ -18,9 +18,10 @@ struct GraphKey {
     int variant = 0;
     double G = 0, dt = 0;
     const void *p0 = nullptr, *p1 = nullptr, *part = nullptr, *pred = nullptr;
+    bool fused = false;
     bool operator==(const GraphKey &o) const {
         return method == o.method && cur == o.cur && n == o.n && variant == o.variant && G == o.G && dt == o.dt &&
-               p0 == o.p0 && p1 == o.p1 && part == o.part && pred == o.pred;
+               p0 == o.p0 && p1 == o.p1 && part == o.part && pred == o.pred && fused == o.fused;
     }
 };
 

@@ -174,9 +174,19 @@ static int timed_event(gtd_system *s) {
     return GTD_OK;
 }
 
+// Whether a force evaluation and its update are one fused FP64 launch.  With the mixed precision it is both
+// the faster kernel and the more precise one at these sizes, where launches and the slots' sum outweigh
+// the pair terms, and its steps replay from a graph: a KDK step of 100 bodies 1.9 us (two launches and
+// the host's 25), 1024 4.3 (30), 2048 8.8 (30), 4096 25 (39), 4736 32 (44).  Up to 4736 bodies the {2, 1, 8}
+// shape's CTAs make two whole rounds: FP64 4300 27.9 us against 29.4, 4736 31.9 against 37.1.
+static bool fused_force(const gtd_system *s) {
+    if (s->precision == GTD_PREC_F64 && s->n <= kFusedMaxN) return true;
+    return s->n <= kFusedAutoMaxN && !s->variant_pinned && !variant_tuned(s->device, s->precision, s->n);
+}
+
 int force_and_integrate(gtd_system *s, const double4 *src, int epi, const StepArgs &st) {
     int rc;
-    if (s->precision == GTD_PREC_F64 && s->n <= kFusedMaxN) {
+    if (fused_force(s)) {
         if (s->time_force && (rc = timed_event(s))) return rc;
         rc = launch_fused_small(s->n, src, s->G, epi, st, s->stream, true);
         if (rc) return rc;
@@ -317,10 +327,11 @@ int output_rows(gtd_system *s, std::vector<int64_t> &row) {
 }
 
 // The mixed kernel centres each row's FP32 frame on the row; Hilbert-ordered bodies keep rows
-// compact, so the mixed path reorders at the start of an evolve and every reorder_interval steps.
+// compact, so the mixed path reorders at the start of an evolve and every reorder_interval steps (where
+// the fused kernel runs, there are no frames and no reason to).
 static int maybe_reorder(gtd_system *s, bool force) {
     // collisions scan the bodies in upload order (as the reference scans its vector): no reordering
-    if (s->precision != GTD_PREC_MIXED || s->n < 2 || s->coll != GTD_NO_COLL) return GTD_OK;
+    if (s->precision != GTD_PREC_MIXED || s->n < 2 || s->coll != GTD_NO_COLL || fused_force(s)) return GTD_OK;
     if (!force && s->steps_since_reorder < (uint64_t)s->reorder_interval) return GTD_OK;
     s->steps_since_reorder = 0;
     return reorder_bodies(s);
@@ -349,14 +360,14 @@ static int evolve_begin(gtd_system *s, int method) {
     return GTD_OK;
 }
 
-// Steady-state steps with no host logic between them (FP64, no collisions, recording or force
+// Steady-state steps with no host logic between them (FP64 kernels, no collisions, recording or force
 // timing) are replayed from a CUDA graph of kGraphSteps steps: at small N the launches, not the
 // arithmetic, set the step time.  kGraphSteps is even, so the position double buffer ends where it
 // started and one graph per (method, buffer parity, parameters) serves every replay.
 constexpr int kGraphSteps = 16;
 
 static bool graph_eligible(const gtd_system *s) {
-    if (s->precision != GTD_PREC_F64 || s->coll != GTD_NO_COLL || s->rec_every || s->time_force || s->step_hook)
+    if ((s->precision != GTD_PREC_F64 && !fused_force(s)) || s->coll != GTD_NO_COLL || s->rec_every || s->time_force || s->step_hook)
         return false;
     if ((s->method == GTD_LEAPFROG_KDK || s->method == GTD_LEAPFROG_DKD) && s->synced) return false;
     return true;
@@ -368,14 +379,15 @@ void release_graph(gtd_system *s) {
 }
 
 static int run_graph_chunk(gtd_system *s) {
-    int rc = ensure_plan(s);  // no allocation inside the capture
+    const bool fused = fused_force(s);
+    int rc = fused ? GTD_OK : ensure_plan(s);  // no allocation inside the capture
     if (rc) return rc;
     if (s->method == GTD_MODIFIED_EULER || s->method == GTD_MIDPOINT) {
         rc = ensure_pred(s);
         if (rc) return rc;
     }
     const GraphKey key{s->method, s->cur, s->n, s->variant, s->G, s->dt, s->pm[0], s->pm[1], s->partials,
-                       s->pred_pos};
+                       s->pred_pos, fused};
     if (!s->graph || !(key == s->graph_key)) {
         release_graph(s);
         const int cur0 = s->cur;
@@ -457,7 +469,7 @@ int cb_select_branch(int method) { return check_option(method) ? select_branch(m
 // Allocates what the steps of s->method use, so that they can be captured.
 int cb_prepare_steps(gtd_system *s) {
     int rc = GTD_OK;
-    if (!(s->precision == GTD_PREC_F64 && s->n <= kFusedMaxN)) rc = ensure_plan(s);
+    if (!fused_force(s)) rc = ensure_plan(s);
     if (!rc && (s->method == GTD_MODIFIED_EULER || s->method == GTD_MIDPOINT)) rc = ensure_pred(s);
     return rc;
 }
@@ -768,14 +780,14 @@ int gtd_system_autotune_direct(gtd_system *s, int reps, int *best, double *best_
     if (s->n == 0) return fail(GTD_ERR_INVALID_ARGUMENT, "autotune needs bodies");
     DeviceGuard g(s->device);
     if (reps < 1) reps = 1;
-    int rc = maybe_reorder(s, true);
-    if (rc) return rc;
     struct RestorePin {
         gtd_system *s;
         bool pinned;
         ~RestorePin() { s->variant_pinned = pinned; }
     } restore{s, s->variant_pinned};
     s->variant_pinned = true;  // while timing, ensure_plan keeps the variant under test
+    int rc = maybe_reorder(s, true);
+    if (rc) return rc;
     int arg = s->variant;
     double bestv = 1e300;
     for (int v = 0; v < variant_count(s->precision); ++v) {
