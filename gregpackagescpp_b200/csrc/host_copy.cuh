@@ -14,9 +14,11 @@ struct HostSpan {
     size_t bytes;
 };
 
-// A handle's pinned staging ring, made on the first large copy and freed with the handle.
+// A handle's pinned staging ring, made when its large copies have come to what that pays for, and freed
+// with the handle.
 struct HostRing {
     char *mem = nullptr;
+    size_t moved = 0;                 // bytes of large copies, up to that point
     std::vector<cudaEvent_t> events;  // one per slot
 };
 void release_host_ring(HostRing &ring);
