@@ -244,17 +244,20 @@ __device__ __forceinline__ int lcp_digits(unsigned long long a, unsigned long lo
 // Per slot: common octal prefix with the next slot and the number of nodes the slot opens.
 template <bool F>
 __global__ void lcp_count_kernel(const unsigned long long *codes, const int32_t *perm, const double4 *pm, int64_t n,
-                                 int32_t *lcp, uint32_t *cnt, int *status) {
+                                 int32_t *lcp, uint32_t *cnt, int *status, uint32_t *deepest) {
     using TT = TreeT<F>;
     const int64_t a = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    int la = -1;
+    if (a + 1 < n) la = lcp_digits(codes[a], codes[a + 1]);
+    // the deepest internal node: how many levels of moments follow (few warps find a new maximum)
+    const unsigned most = __reduce_max_sync(0xffffffffu, (unsigned)max(min(la, kMaxDepth - 1), 0));
+    if ((threadIdx.x & 31) == 0 && most > *(volatile uint32_t *)deepest) atomicMax(deepest, most);
     if (a > n) return;
     if (a == n) {
         cnt[n] = 0;
         return;
     }
-    int la = -1;
     if (a + 1 < n) {
-        la = lcp_digits(codes[a], codes[a + 1]);
         if (la == kMaxDepth) {
             const double4 p = pm[perm[a]], q = pm[perm[a + 1]];
             if (TT::rnd(p.x) == TT::rnd(q.x) && TT::rnd(p.y) == TT::rnd(q.y) && TT::rnd(p.z) == TT::rnd(q.z))
@@ -300,6 +303,9 @@ struct EmitArgs {
     int32_t *first, *count, *skip, *own;
     double4 *com;
     double *width;
+    void *slot_pos;       // slot-ordered bodies, as slot_body
+    double G;
+    uint32_t *depth_cnt;  // internal nodes per depth, to add to
 };
 
 template <bool F>
@@ -315,11 +321,21 @@ __device__ double cell_width(unsigned long long code, int depth, const double *b
     return (double)TT::sub(hi, lo);
 }
 
+// A body as the walks read it: position in T and G m.
 template <bool F>
-__global__ void emit_kernel(EmitArgs e) {
+__device__ __forceinline__ void slot_body(void *slot_pos, int64_t s, const double4 &p, double G) {
+    if (F) {
+        reinterpret_cast<float4 *>(slot_pos)[s] = make_float4(__double2float_rn(p.x), __double2float_rn(p.y),
+                                                              __double2float_rn(p.z), (float)(G * (double)(float)p.w));
+    } else {
+        reinterpret_cast<double4 *>(slot_pos)[s] = make_double4(p.x, p.y, p.z, G * p.w);
+    }
+}
+
+// Thread per slot: the nodes it opens, its leaf and the bodies in it.
+template <bool F>
+__device__ __forceinline__ void emit_slot(const EmitArgs &e, int64_t a, uint32_t *cnt) {
     using TT = TreeT<F>;
-    const int64_t a = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (a >= e.n) return;
     const int lm = a > 0 ? e.lcp[a - 1] : -1;
     const int la = a + 1 < e.n ? e.lcp[a] : -1;
     const int lim = la < kMaxDepth - 1 ? la : kMaxDepth - 1;
@@ -333,6 +349,7 @@ __global__ void emit_kernel(EmitArgs e) {
         e.count[node] = (int32_t)(last - a + 1);
         e.skip[node] = (int32_t)e.node_start[last + 1];
         e.width[node] = cell_width<F>(ca, d, e.box);
+        atomicAdd(&cnt[d], 1u);
     }
     if (lm < kMaxDepth) {
         const int64_t last = la == kMaxDepth ? range_end(e.codes, e.n, a, kMaxDepth) : a;
@@ -348,6 +365,7 @@ __global__ void emit_kernel(EmitArgs e) {
             const double4 p = e.pm[e.perm[a]];
             e.com[node] = make_double4((double)TT::rnd(p.x), (double)TT::rnd(p.y), (double)TT::rnd(p.z),
                                        (double)TT::rnd(p.w));
+            slot_body<F>(e.slot_pos, a, p, e.G);
         } else {
             double ms = 0.0, mx = 0.0, my = 0.0, mz = 0.0;
             for (int64_t q = a; q <= last; ++q) {
@@ -357,6 +375,7 @@ __global__ void emit_kernel(EmitArgs e) {
                 mx = __dadd_rn(mx, __dmul_rn(mb, (double)TT::rnd(p.x)));
                 my = __dadd_rn(my, __dmul_rn(mb, (double)TT::rnd(p.y)));
                 mz = __dadd_rn(mz, __dmul_rn(mb, (double)TT::rnd(p.z)));
+                slot_body<F>(e.slot_pos, q, p, e.G);
             }
             e.com[node] = make_double4(__ddiv_rn(mx, ms), __ddiv_rn(my, ms), __ddiv_rn(mz, ms), ms);
         }
@@ -364,38 +383,25 @@ __global__ void emit_kernel(EmitArgs e) {
     }
 }
 
-__global__ void depth_offsets_kernel(uint32_t *depth_off) {
-    // depth_off[0..20]: counts in, exclusive offsets out; depth_off[22..42]: cursors
-    if (threadIdx.x != 0) return;
-    uint32_t run = 0;
-    for (int d = 0; d < kMaxDepth; ++d) {
-        const uint32_t c = depth_off[d];
-        depth_off[d] = run;
-        depth_off[22 + d] = run;
-        run += c;
-    }
-    depth_off[kMaxDepth] = run;
-}
-
-// Internal nodes per depth.  Each CTA counts a chunk of kDepthChunk nodes in shared memory and adds
-// its counts with one global atomic per depth: a global atomic per node would serialise ~N atomics
-// on 21 addresses (about 1 ms at N = 4194304).
-constexpr int kDepthChunk = 16 * kTT;
-
-__global__ void __launch_bounds__(kTT) depth_count_kernel(const int8_t *depth, const int8_t *leaf, int64_t n_nodes,
-                                                          uint32_t *depth_off) {
+// Internal nodes per depth are counted where they are emitted: each CTA counts in shared memory and adds
+// its counts with one global atomic per depth (a global atomic per node would serialise ~N atomics on 21
+// addresses, about 1 ms at N = 4194304).
+template <bool F>
+__global__ void __launch_bounds__(kTT) emit_kernel(EmitArgs e) {
     __shared__ uint32_t cnt[kMaxDepth];
     const int t = threadIdx.x;
     if (t < kMaxDepth) cnt[t] = 0;
     __syncthreads();
-    const int64_t base = (int64_t)blockIdx.x * kDepthChunk;
-    for (int k = 0; k < kDepthChunk / kTT; ++k) {
-        const int64_t nd = base + (int64_t)k * kTT + t;
-        if (nd < n_nodes && !leaf[nd]) atomicAdd(&cnt[depth[nd]], 1u);
-    }
+    const int64_t a = (int64_t)blockIdx.x * blockDim.x + t;
+    if (a < e.n) emit_slot<F>(e, a, cnt);
     __syncthreads();
-    if (t < kMaxDepth && cnt[t]) atomicAdd(&depth_off[t], cnt[t]);
+    if (t < kMaxDepth && cnt[t]) atomicAdd(&e.depth_cnt[t], cnt[t]);
 }
+
+// depth_off: [0, 21) the internal nodes per depth, [22, 43) how many of them are listed, [64, 86) the
+// exclusive sums of the counts, [90] the deepest level that has any.
+constexpr int kDepthWords = 96, kDeepest = 90;
+constexpr int kDepthChunk = 16 * kTT;  // nodes per CTA of the listing
 
 // Lists the internal nodes by depth (the order inside a depth is free: each node's moments are
 // computed from its own children alone).  A CTA ranks its chunk's nodes per depth in shared memory
@@ -403,9 +409,20 @@ __global__ void __launch_bounds__(kTT) depth_count_kernel(const int8_t *depth, c
 __global__ void __launch_bounds__(kTT) depth_scatter_kernel(const int8_t *depth, const int8_t *leaf, int64_t n_nodes,
                                                             uint32_t *depth_off, int32_t *list) {
     constexpr int kItems = kDepthChunk / kTT;
-    __shared__ uint32_t cnt[kMaxDepth], start[kMaxDepth];
+    __shared__ uint32_t cnt[kMaxDepth], start[kMaxDepth], off[32];
     const int t = threadIdx.x;
     if (t < kMaxDepth) cnt[t] = 0;
+    if (t < 32) {
+        const uint32_t c = t < kMaxDepth ? depth_off[t] : 0u;
+        uint32_t incl = c;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (t >= o) incl += y;
+        }
+        off[t] = incl - c;
+        if (blockIdx.x == 0 && t <= kMaxDepth) depth_off[64 + t] = incl - c;
+    }
     __syncthreads();
     const int64_t base = (int64_t)blockIdx.x * kDepthChunk;
     int8_t d[kItems];
@@ -421,17 +438,20 @@ __global__ void __launch_bounds__(kTT) depth_scatter_kernel(const int8_t *depth,
         }
     }
     __syncthreads();
-    if (t < kMaxDepth && cnt[t]) start[t] = atomicAdd(&depth_off[22 + t], cnt[t]);
+    if (t < kMaxDepth && cnt[t]) start[t] = off[t] + atomicAdd(&depth_off[22 + t], cnt[t]);
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < kItems; ++k)
         if (d[k] >= 0) list[start[d[k]] + r[k]] = (int32_t)(base + (int64_t)k * kTT + t);
 }
 
-// Internal nodes of one depth: FP64 moments of the children in octant order.
+// Internal nodes of one depth: FP64 moments of the children in octant order.  A chained launch per
+// level, from the deepest that has internal nodes.
 __global__ void com_level_kernel(const int32_t *list, const uint32_t *depth_off, int d, const int32_t *skip,
                                  double4 *com) {
-    const uint32_t b = depth_off[d], e = depth_off[d + 1];
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
+    const uint32_t b = depth_off[64 + d], e = depth_off[64 + d + 1];
     for (uint32_t k = b + blockIdx.x * blockDim.x + threadIdx.x; k < e; k += gridDim.x * blockDim.x) {
         const int32_t nd = list[k];
         const int32_t end = skip[nd];
@@ -479,19 +499,6 @@ __global__ void walk_records_kernel(int64_t n_nodes, const double4 *com, const d
         w2_64[nd] = w * w;
     }
     rec_b[nd] = b;
-}
-
-template <bool F>
-__global__ void slot_bodies_kernel(const double4 *pm, const int32_t *perm, int64_t n, double G, void *slot_pos) {
-    const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= n) return;
-    const double4 p = pm[perm[s]];
-    if (F) {
-        reinterpret_cast<float4 *>(slot_pos)[s] = make_float4(__double2float_rn(p.x), __double2float_rn(p.y),
-                                                              __double2float_rn(p.z), (float)(G * (double)(float)p.w));
-    } else {
-        reinterpret_cast<double4 *>(slot_pos)[s] = make_double4(p.x, p.y, p.z, G * p.w);
-    }
 }
 
 // ---- warp-cooperative walk ---------------------------------------------------------------------
@@ -1082,7 +1089,7 @@ static int ensure_tree_n(gtd_system *s, int64_t n) {
     total += carve_size(4 * nn);                // slot_cnt
     total += carve_size(4 * s->scratch_words);  // scratch
     total += carve_size(8 * 6 * kBBoxBlocks);   // bbox partials
-    total += carve_size(8 * 6) + carve_size(64) + carve_size(4 * 64);
+    total += carve_size(8 * 6) + carve_size(64) + carve_size(4 * kDepthWords);
     GTD_CUDA(cudaMalloc(&s->tree_nbuf, total));
     char *c = reinterpret_cast<char *>(s->tree_nbuf);
     s->codes = carve<unsigned long long>(c, nn);
@@ -1099,7 +1106,7 @@ static int ensure_tree_n(gtd_system *s, int64_t n) {
     s->bbox_part = carve<double>(c, 6 * kBBoxBlocks);
     s->box_dev = carve<double>(c, 6);
     s->status = carve<int>(c, 16);
-    s->depth_off = carve<uint32_t>(c, 64);
+    s->depth_off = carve<uint32_t>(c, kDepthWords);
     GTD_CUDA(cudaMemsetAsync(s->status, 0, 16 * sizeof(int), s->stream));  // [0] build, [1] walk
     if (!s->host_total) GTD_CUDA(cudaMallocHost(&s->host_total, 16 * sizeof(uint32_t)));
     s->tree_n = n;
@@ -1171,9 +1178,8 @@ static int hilbert_sort(gtd_system *s) {
     return radix_sort_u64(s->codes, s->perm, s->codes_alt, s->perm_alt, n, 63, s->scratch, st, &s->launches);
 }
 
-static int read_status(gtd_system *s) {
-    GTD_CUDA(cudaMemcpyAsync(s->host_total + 1, s->status, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
-    GTD_CUDA(cudaStreamSynchronize(s->stream));
+// The error of a build whose status word is in host_total[1].
+static int build_error(gtd_system *s) {
     const int st = (int)s->host_total[1];
     if (st == GTD_ERR_INVALID_BODY_PLACEMENT)
         return fail(st, "Error: a body does not lie within the Barnes-Hut root cube (non-finite position?).");
@@ -1197,38 +1203,39 @@ static int bh_build_impl(gtd_system *s, int tree_float) {
     if (rc) return rc;
     cudaStream_t st = s->stream;
     const double4 *pm = s->pm[s->cur];
+    GTD_CUDA(cudaMemsetAsync(s->depth_off, 0, kDepthWords * sizeof(uint32_t), st));
     if (tree_float)
         lcp_count_kernel<true><<<blocks_for(n + 1), kTT, 0, st>>>(s->codes, s->perm, pm, n, s->lcp, s->node_start,
-                                                                  s->status);
+                                                                  s->status, s->depth_off + kDeepest);
     else
         lcp_count_kernel<false><<<blocks_for(n + 1), kTT, 0, st>>>(s->codes, s->perm, pm, n, s->lcp, s->node_start,
-                                                                   s->status);
+                                                                   s->status, s->depth_off + kDeepest);
     GTD_CHECK_LAUNCH();
     s->launches += 1;
     rc = exclusive_scan_u32(s->node_start, s->node_start, n + 1, s->scratch, st, &s->launches);
     if (rc) return rc;
     GTD_CUDA(cudaMemcpyAsync(s->host_total, s->node_start + n, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     GTD_CUDA(cudaMemcpyAsync(s->host_total + 1, s->status, sizeof(int), cudaMemcpyDeviceToHost, st));
+    GTD_CUDA(cudaMemcpyAsync(s->host_total + 2, s->depth_off + kDeepest, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     GTD_CUDA(cudaStreamSynchronize(st));
-    rc = read_status(s);
+    rc = build_error(s);
     if (rc) return rc;
     const int64_t nodes = s->host_total[0];
     rc = ensure_tree_nodes(s, nodes);
     if (rc) return rc;
-    GTD_CUDA(cudaMemsetAsync(s->depth_off, 0, 64 * sizeof(uint32_t), st));
     EmitArgs e{n, s->codes, s->perm, s->lcp, s->node_start, pm, s->box_dev, s->ndepth, s->nleaf, s->nfirst,
-               s->ncount, s->nskip, s->own_leaf, s->ncom, s->nwidth};
+               s->ncount, s->nskip, s->own_leaf, s->ncom, s->nwidth, s->slot_pos, s->G, s->depth_off};
     if (tree_float) emit_kernel<true><<<blocks_for(n), kTT, 0, st>>>(e);
     else emit_kernel<false><<<blocks_for(n), kTT, 0, st>>>(e);
     GTD_CHECK_LAUNCH();
     const unsigned depth_blocks = (unsigned)((nodes + kDepthChunk - 1) / kDepthChunk);
-    depth_count_kernel<<<depth_blocks, kTT, 0, st>>>(s->ndepth, s->nleaf, nodes, s->depth_off);
-    depth_offsets_kernel<<<1, 32, 0, st>>>(s->depth_off);
     depth_scatter_kernel<<<depth_blocks, kTT, 0, st>>>(s->ndepth, s->nleaf, nodes, s->depth_off, s->depth_list);
     GTD_CHECK_LAUNCH();
-    s->launches += 4;
-    for (int d = kMaxDepth - 1; d >= 0; --d) {
-        com_level_kernel<<<4 * 148, kTT, 0, st>>>(s->depth_list, s->depth_off, d, s->nskip, s->ncom);
+    s->launches += 2;
+    const int deepest = std::min((int)s->host_total[2], kMaxDepth - 1);
+    for (int d = deepest; d >= 0; --d) {
+        launch_chained(d < deepest, com_level_kernel, 4 * 148, kTT, 0, st, s->depth_list, s->depth_off, d, s->nskip,
+                       s->ncom);
         s->launches += 1;
     }
     GTD_CHECK_LAUNCH();
@@ -1246,10 +1253,7 @@ static int bh_build_impl(gtd_system *s, int tree_float) {
                                                                        s->ncount, s->nskip, s->G, s->nwalk_a,
                                                                        s->nwalk_b, s->nwalk_w2);
     GTD_CHECK_LAUNCH();
-    if (tree_float) slot_bodies_kernel<true><<<blocks_for(n), kTT, 0, st>>>(pm, s->perm, n, s->G, s->slot_pos);
-    else slot_bodies_kernel<false><<<blocks_for(n), kTT, 0, st>>>(pm, s->perm, n, s->G, s->slot_pos);
-    GTD_CHECK_LAUNCH();
-    s->launches += 2;
+    s->launches += 1;
     s->n_nodes = nodes;
     s->tree_valid = true;
     return GTD_OK;
