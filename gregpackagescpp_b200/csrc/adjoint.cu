@@ -96,6 +96,8 @@ __global__ void __launch_bounds__(T, MINB) vjp_kernel(VjpArgs a) {
     extern __shared__ __align__(16) unsigned char vjp_smem[];
     Smem &S = *reinterpret_cast<Smem *>(vjp_smem);
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
     auto stage = [&](int buf, const double4 &x, const double4 &w) {
         const int e = (t >> 5) * 64 + lane;
         S.xy[buf][e] = S.xy[buf][e + 32] = make_double2(x.x, x.y);
@@ -313,7 +315,11 @@ static void launch_vjp_small(int64_t n, const double4 *x, const double4 *w, cons
                    GROUPS * kVjpSlices * 32, 0, st, n, x, w, up);
 }
 
-__global__ void __launch_bounds__(kRedWarps * 32) vjp_reduce_kernel(SymSlots s, double *base_out, VjpUpdate up) {
+__global__ void __launch_bounds__(kRedWarps * 32) vjp_reduce_kernel(SymSlots s, double *base_out, VjpUpdate up,
+                                                                    unsigned *queue) {
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
+    if (blockIdx.x == 0 && threadIdx.x == 0) *queue = 0;  // the batch's counter, for the next VJP
     sym_reduce<4>(s, [&](int64_t i, const double (&v)[4]) {
         if (base_out) {  // not the last batch
 #pragma unroll
@@ -462,10 +468,21 @@ static int adj_step(gtd_adjoint *A, const double4 *src, double4 *dst, double c, 
         A->launches += 1;
         return launch_fused_small(A->n, src, A->G, EPI_KICK_DRIFT, sa, st, true);
     }
-    int rc = launch_force(GTD_PREC_F64, A->fplan, src, A->G, A->fpart, st);
-    if (!rc) rc = launch_integrate(A->fplan, A->fpart, EPI_KICK_DRIFT, sa, st);
+    int rc = launch_force(GTD_PREC_F64, A->fplan, src, A->G, A->fpart, st, true);
+    if (!rc) rc = launch_integrate(A->fplan, A->fpart, EPI_KICK_DRIFT, sa, st, true);
     A->launches += (uint64_t)force_launch_count(A->fplan);
     return rc;
+}
+
+// The queue counters of the pair kernels, zero before a sweep; each reduction restores its own.
+static int adj_reset(gtd_adjoint *A, cudaStream_t st) {
+    if (!A->small_force && A->fplan.sym) {
+        const int rc = sym_reset(A->fplan, A->fpart, st);
+        if (rc) return rc;
+    }
+    if (!A->small_vjp)
+        GTD_CUDA(cudaMemsetAsync(A->vpart, 0, (size_t)sym_layout(A->vgeom, kSymSlotBytes, 4).batches * sizeof(unsigned), st));
+    return GTD_OK;
 }
 
 // The VJP at x_k with w = c_k lv, and the update; w for x_{k-1} is left in the other buffer.
@@ -485,7 +502,6 @@ static int adj_vjp(gtd_adjoint *A, const double4 *x, uint64_t k, int &cur, cudaS
     const SymGeom &g = A->vgeom;
     const SymLayout lay = sym_layout(g, kSymSlotBytes, 4);
     char *mem = reinterpret_cast<char *>(A->vpart);
-    GTD_CUDA(cudaMemsetAsync(mem, 0, (size_t)lay.batches * sizeof(unsigned), st));
     int64_t batch = 0;
     for (int64_t Pa = 0; Pa < g.Gs; ++batch) {
         const int64_t Pb = sym_batch_end(g, Pa, kSymSlotBytes, 4);
@@ -493,10 +509,10 @@ static int adj_vjp(gtd_adjoint *A, const double4 *x, uint64_t k, int &cur, cudaS
         const VjpArgs va{g, x, w, const_cast<double *>(s.rowpart), const_cast<double *>(s.colpart), s.unit0,
                          sym_tri(g, Pb) * sym_block_units(g), s.col0, reinterpret_cast<unsigned *>(mem) + batch};
         const int grid = (int)std::min<int64_t>(A->vgrid, va.unit1 - va.unit0);
-        kVjpKernel<<<grid, kVjpShape.threads, kVjpSmem, st>>>(va);
+        launch_chained(true, kVjpKernel, grid, kVjpShape.threads, kVjpSmem, st, va);
         GTD_CHECK_LAUNCH();
         double *base = Pb < g.Gs ? reinterpret_cast<double *>(mem + lay.base) : nullptr;
-        vjp_reduce_kernel<<<(unsigned)((g.n + 31) / 32), kRedWarps * 32, 0, st>>>(s, base, up);
+        launch_chained(true, vjp_reduce_kernel, (unsigned)((g.n + 31) / 32), kRedWarps * 32, 0, st, s, base, up, va.queue);
         GTD_CHECK_LAUNCH();
         A->launches += 2;
         Pa = Pb;
@@ -577,12 +593,14 @@ int gtd_adjoint_forward(gtd_adjoint *A, const double *x0, const double *v0, cons
     const size_t b4 = sizeof(double4) * (size_t)n;
     const uint64_t T = A->steps, C = A->every;
     const double h = A->h;
+    int rc = adj_reset(A, st);
+    if (rc) return rc;
     auto at = [&](uint64_t k) { return A->pos + (size_t)(C ? k & 1 : k) * (size_t)n; };
     pack_kernel<<<g1(n), 256, 0, st>>>(n, x0, m, v0, at(0), A->v);
     GTD_CHECK_LAUNCH();
     A->launches += 1;
     for (uint64_t k = 0; k <= T; ++k) {
-        const int rc = adj_step(A, at(k), k < T ? at(k + 1) : nullptr, k == 0 || k == T ? 0.5 * h : h, st);
+        rc = adj_step(A, at(k), k < T ? at(k + 1) : nullptr, k == 0 || k == T ? 0.5 * h : h, st);
         if (rc) return rc;
         if (C && k < T && k % C == 0) {
             double4 *c = A->ck + 3 * (size_t)n * (size_t)(k / C);
@@ -610,6 +628,10 @@ int gtd_adjoint_backward(gtd_adjoint *A, const double *gxT, const double *gvT, d
     const double h = A->h;
     const uint64_t T = A->steps, C = A->every;
     int cur = 0;
+    {
+        const int rc = adj_reset(A, st);
+        if (rc) return rc;
+    }
     reverse_begin_kernel<<<g1(n), 256, 0, st>>>(n, gxT, gvT, 0.5 * h, A->lx, A->lv, A->mu, A->w[0]);
     GTD_CHECK_LAUNCH();
     A->launches += 1;

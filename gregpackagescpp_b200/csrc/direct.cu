@@ -442,13 +442,14 @@ constexpr int kNumF64 = sizeof(kF64Variants) / sizeof(kF64Variants[0]);
 int variant_count(int precision) { return precision == GTD_PREC_MIXED ? kNumMixed : kNumF64; }
 
 // Variant for a handle nobody tuned: the unordered-pair kernels (direct_sym.cu), per step on B200
-//   mixed   N = 8192 65 us (ordered pairs 75), 16384 162 (192), 65536 1.59 ms (2.32), 262144 21.8 ms (29.3)
-//   FP64    N = 4500 35 us (39), 8192 68 (92), 16384 212 (295), 65536 2.95 ms (4.33)
-// but FP64 systems of up to 17 rows and tiles of 256 bodies, whose 289 ordered tiles all run at once, one
-// per CTA: N = 4200 29 us against 35.
+//   mixed   N = 8192 58 us (ordered pairs 75), 16384 160 (192), 65536 1.58 ms (2.32), 262144 21.8 ms (29.3)
+//   FP64    N = 5000 35 us (41), 8192 65 (92), 16384 212 (295), 65536 2.95 ms (4.33)
+// Systems of up to kFusedAutoMaxN bodies take the fused kernel instead; where one was tuned, or for FP64
+// handles' plans, up to 17 rows and tiles of 256 bodies, the 289 ordered tiles all run at once, one per CTA:
+// N = 4200 29 us against 35.
 // From N = 32768 the mixed kernel folds its FP32 sums half as often: 3 % faster, and its rounding
 // (RMS 3.8e-8 of a body's acceleration at N = 262144 against 3.2e-8) is still that of the ordered
-// kernel's fold of 128 (4.0e-8).  FP64 systems up to kFusedMaxN bodies take the fused kernel instead.
+// kernel's fold of 128 (4.0e-8).
 int default_variant(int precision, int64_t n) {
     if (precision == GTD_PREC_MIXED) return n >= 32768 ? 9 : 10;
     if (n <= 17 * 256) return 1;
@@ -601,9 +602,9 @@ int fit_plan_partials(ForcePlan &p, size_t max_bytes) {
 }
 
 int launch_force(int precision, const ForcePlan &p, const double4 *src, double G, double *partials,
-                 cudaStream_t s) {
+                 cudaStream_t s, bool chained) {
     if (p.n == 0) return GTD_OK;
-    if (p.sym) return sym_launch_force(precision, p, src, G, partials, s);
+    if (p.sym) return sym_launch_force(precision, p, src, G, partials, chained, s);
     unsigned *queue = p.segs > 0 ? reinterpret_cast<unsigned *>(reinterpret_cast<char *>(partials) + queue_offset(p))
                                  : nullptr;
     ForceKArgs a{p.n, p.rows, p.tiles, p.total, p.grid, p.bi, src, G, partials, p.near2, p.segs, p.seg_tiles,
@@ -798,9 +799,9 @@ int launch_fused_small(int64_t n, const double4 *src, double G, int epi, const S
     return GTD_OK;
 }
 
-int launch_integrate(const ForcePlan &p, const double *partials, int epi, const StepArgs &st, cudaStream_t s) {
+int launch_integrate(const ForcePlan &p, const double *partials, int epi, const StepArgs &st, cudaStream_t s, bool chained) {
     if (p.n == 0) return GTD_OK;
-    if (p.sym) return sym_launch_finish(p, partials, epi, st, nullptr, s);
+    if (p.sym) return sym_launch_finish(p, partials, epi, st, nullptr, chained, s);
     IntArgs a{p.n, p.tiles, p.total, p.grid, p.bi, epi, partials, st, p.segs};
     const int threads = 256;
     // A row's force spread over more than ~4 slots, with too few bodies for a thread each to keep
@@ -837,7 +838,7 @@ __global__ void sum_partials_kernel(IntArgs a, double *acc3) {
 
 int launch_sum_partials(const ForcePlan &p, const double *partials, double *acc3, cudaStream_t s) {
     if (p.n == 0) return GTD_OK;
-    if (p.sym) return sym_launch_finish(p, partials, EPI_ACC, StepArgs{}, acc3, s);
+    if (p.sym) return sym_launch_finish(p, partials, EPI_ACC, StepArgs{}, acc3, false, s);
     IntArgs a{p.n, p.tiles, p.total, p.grid, p.bi, EPI_ACC, partials, StepArgs{}, p.segs};
     sum_partials_kernel<<<(unsigned)((p.n + 255) / 256), 256, 0, s>>>(a, acc3);
     GTD_CHECK_LAUNCH();

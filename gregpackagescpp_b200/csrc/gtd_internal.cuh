@@ -75,7 +75,11 @@ SymShape sym_shape(int precision, int kind);
 size_t sym_partial_bytes(const ForcePlan &p);
 int sym_fit(ForcePlan &p, size_t max_bytes);
 int sym_launches(const ForcePlan &p);
-int sym_launch_force(int precision, const ForcePlan &p, const double4 *src, double G, double *partials, cudaStream_t s);
+// The unordered-pair kernels' queue counters (at the start of the partial sums) are zero between force
+// evaluations: sym_reset makes them so, each reduction restores its own.
+int sym_reset(const ForcePlan &p, double *partials, cudaStream_t s);
+int sym_launch_force(int precision, const ForcePlan &p, const double4 *src, double G, double *partials, bool chained,
+                     cudaStream_t s);
 
 // Mixed kernel: a fold that holds a pair closer than 2 |X_i| / (K - 1) to one of its i-bodies (X_i:
 // the body's coordinates in its row's FP32 frame) is recomputed on the precise path, so that the
@@ -135,17 +139,19 @@ size_t partial_bytes(const ForcePlan &p);
 int fit_plan_partials(ForcePlan &p, size_t max_bytes);
 // acc3[3 i + d] = the summed partials of body i (the force alone, in the bodies' order).
 int launch_sum_partials(const ForcePlan &p, const double *partials, double *acc3, cudaStream_t s);
-// Force on every body of `src` (positions + G-free masses), written as partial sums.
+// Force on every body of `src` (positions + G-free masses), written as partial sums.  chained: as in
+// launch_chained, for unordered-pair plans.
 int launch_force(int precision, const ForcePlan &p, const double4 *src, double G, double *partials,
-                 cudaStream_t s);
+                 cudaStream_t s, bool chained = false);
 // Combines the partials of each body and applies the integrator epilogue.
-int launch_integrate(const ForcePlan &p, const double *partials, int epi, const StepArgs &a, cudaStream_t s);
+int launch_integrate(const ForcePlan &p, const double *partials, int epi, const StepArgs &a, cudaStream_t s,
+                     bool chained = false);
 // Kick-drift (KDK start) and half drift (DKD start) on a synchronised state.
 int launch_kick_drift(int64_t n, const double4 *cur, double4 *dst, double4 *vel, const double4 *acc, double h,
                       cudaStream_t s);
 int launch_half_drift(int64_t n, const double4 *cur, double4 *dst, const double4 *vel, double h, cudaStream_t s);
 
-int sym_launch_finish(const ForcePlan &p, const double *partials, int epi, const StepArgs &st, double *acc3,
+int sym_launch_finish(const ForcePlan &p, const double *partials, int epi, const StepArgs &st, double *acc3, bool chained,
                       cudaStream_t s);
 
 // FP64 diagnostics: out[0]=KE, out[1]=PE, out[2..4]=momentum, out[5..7]=sum m x, out[8]=sum m.

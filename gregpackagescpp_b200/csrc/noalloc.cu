@@ -104,6 +104,7 @@ extern "C" int gtd_direct_accelerations_noalloc(int64_t n, const double *pm4, do
     ForcePlan p = make_plan(n, precision, dev, noalloc_variant(precision, n));
     rc = fit_plan_partials(p, kNoAllocScratchBytes);
     if (rc) return rc;
+    if (p.sym && (rc = sym_reset(p, static_cast<double *>(scratch), st))) return rc;
     rc = launch_force(precision, p, reinterpret_cast<const double4 *>(pm4), G, static_cast<double *>(scratch), st);
     if (rc) return rc;
     return launch_sum_partials(p, static_cast<const double *>(scratch), acc3, st);

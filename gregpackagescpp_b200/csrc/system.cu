@@ -135,6 +135,11 @@ int ensure_plan(gtd_system *s) {
         GTD_CUDA(cudaMalloc(&s->partials, need));
         s->part_bytes = need;
     }
+    if (s->plan.sym) {
+        const int rc = sym_reset(s->plan, s->partials, s->stream);
+        if (rc) s->plan.n = 0;  // no plan
+        return rc;
+    }
     return GTD_OK;
 }
 
@@ -197,11 +202,13 @@ int force_and_integrate(gtd_system *s, const double4 *src, int epi, const StepAr
     rc = ensure_plan(s);
     if (rc) return rc;
     if (s->time_force && (rc = timed_event(s))) return rc;
-    rc = launch_force(s->precision, s->plan, src, s->G, s->partials, s->stream);
-    if (rc) return rc;
-    if (s->time_force && (rc = timed_event(s))) return rc;
-    rc = launch_integrate(s->plan, s->partials, epi, st, s->stream);
-    if (rc) return rc;
+    rc = launch_force(s->precision, s->plan, src, s->G, s->partials, s->stream, true);
+    if (!rc && s->time_force) rc = timed_event(s);
+    if (!rc) rc = launch_integrate(s->plan, s->partials, epi, st, s->stream, true);
+    if (rc) {
+        s->plan.n = 0;  // half an evaluation: the next one makes the plan and its counters anew
+        return rc;
+    }
     s->launches += (uint64_t)force_launch_count(s->plan);
     return GTD_OK;
 }
@@ -795,12 +802,16 @@ int gtd_system_autotune_direct(gtd_system *s, int reps, int *best, double *best_
         rc = ensure_plan(s);
         if (rc) return rc;
         // warm-up launch, then the median of `reps` timed force launches
-        rc = launch_force(s->precision, s->plan, s->pm[s->cur], s->G, s->partials, s->stream);
+        s->plan.n = 0;  // force kernels alone leave their counters used: whoever comes next makes them anew
+        ForcePlan p = s->plan;
+        p.n = s->n;
+        rc = launch_force(s->precision, p, s->pm[s->cur], s->G, s->partials, s->stream);
         if (rc) return rc;
         std::vector<float> t(reps);
         for (int k = 0; k < reps; ++k) {
+            if (p.sym && (rc = sym_reset(p, s->partials, s->stream))) return rc;
             GTD_CUDA(cudaEventRecord(s->ev0, s->stream));
-            rc = launch_force(s->precision, s->plan, s->pm[s->cur], s->G, s->partials, s->stream);
+            rc = launch_force(s->precision, p, s->pm[s->cur], s->G, s->partials, s->stream);
             if (rc) return rc;
             GTD_CUDA(cudaEventRecord(s->ev1, s->stream));
             GTD_CUDA(cudaEventSynchronize(s->ev1));
