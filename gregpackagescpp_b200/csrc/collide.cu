@@ -607,22 +607,16 @@ __global__ void __launch_bounds__((kPairSlices + 1) * 32)
                 }
             }
         }
+        double sums[3 * I];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-            for (int k = 0; k < I; ++k) {
-                ax[k] += __shfl_xor_sync(0xffffffffu, ax[k], o);
-                ay[k] += __shfl_xor_sync(0xffffffffu, ay[k], o);
-                az[k] += __shfl_xor_sync(0xffffffffu, az[k], o);
-            }
-        if (lane == 0) {
-#pragma unroll
-            for (int k = 0; k < I; ++k) {
-                part[slice][k][0] = ax[k];
-                part[slice][k][1] = ay[k];
-                part[slice][k][2] = az[k];
-            }
+        for (int k = 0; k < I; ++k) {
+            sums[3 * k] = ax[k];
+            sums[3 * k + 1] = ay[k];
+            sums[3 * k + 2] = az[k];
         }
+        int at;
+        const double sum = warp_sums(sums, at);
+        if (at >= 0) (&part[slice][0][0])[at] = sum;
     } else if (go && lane < I && i0 + lane < n) {  // this warp is there only with hk.for_all
         rest[i0 + lane] =
             cb_rest_from_distance(src[i0 + lane], hk.ctl->com, hk.min_cor, hk.max_cor, hk.scale, hk.n_exp);

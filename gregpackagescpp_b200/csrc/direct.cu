@@ -699,17 +699,39 @@ __global__ void integrate_warp_kernel(IntArgs a) {
 // I, the bodies a warp shares its loads between, grows with the system: at one body a chunk's loads take as
 // many L1 cycles as its arithmetic takes FP64 cycles (8 each), and the CTAs should fit the GPU at once -
 // past that the step takes the time of two rounds.  Shapes {bodies per warp, groups per CTA, CTAs per SM}
-// and the bodies a round holds on 148 SMs: {1, 2, 4} 1184, {2, 1, 5} 1480, {2, 1, 8} 2368, {4, 2, 3} 3552;
-// larger systems take {2, 1, 8} again, whose rounds are short.  Microseconds a step on B200, with
-// one body per warp and four groups per CTA throughout / with these:
-//   N = 150 2.72 / 2.47, 592 3.37 / 3.37, 727 4.39 / 3.9, 1024 5.04 / 4.77, 1300 7.75 / 5.62, 2000 12.7 / 8.8,
-//   3000 24.0 / 18.0, 4096 35.2 / 25.3
-// Steps that follow one another are chained launches, let go after the pair loop (at the kernel's start the
-// waiting blocks take room that the last ones of this grid need: 1776 7.5 -> 8.5):
-//   N = 150 2.47 -> 2.20, 592 3.37 -> 3.1, 727 3.88 -> 3.75, 1024 4.77 -> 4.26, 2000 8.8 -> 8.9, 4096 25.4 -> 24.9
+// and the bodies a round holds on 148 SMs: {1, 2, 4} 1184 (two CTAs an SM up to 592 bodies, where it is the
+// faster one), {2, 1, 5} 1480, {2, 1, 8} 2368, {4, 2, 3} 3552; larger systems take {2, 1, 8} again, whose
+// rounds are short.  The first two have the registers for four chunks in flight (FOURS), which pays from
+// two chunks a warp on.  The warps' sums pass through warp_sums: with butterflies their exchanges were a
+// tenth of a step of 1024 bodies.  Steps that follow one another are chained launches, let go after the pair
+// loop (at the kernel's start the waiting blocks take room that the last ones of this grid need).
+// Microseconds a KDK step on B200 with one body per warp and four groups per CTA throughout, these shapes,
+// chained launches, and all of it:
+//   N = 150 2.72 / 2.47 / 2.20 / 2.20, 400 3.5 / 3.5 / 3.23 / 2.46, 592 3.37 / 3.37 / 3.1 / 3.1,
+//   727 4.39 / 3.9 / 3.75 / 3.36, 1024 5.04 / 4.77 / 4.26 / 4.02, 1300 7.75 / 5.62 / 5.16 / 5.03,
+//   2000 12.7 / 8.8 / 8.9 / 8.7, 3000 24.0 / 18.0 / 17.9 / 17.6, 4096 35.2 / 25.3 / 24.9 / 24.5
 constexpr int kFusedSlices = 4;  // warps per group
 
-template <int EPI, int I, int kFusedGroups, int MINB>
+// The chunks of a warp: rounds(R, j) takes R of them from entry j of this lane on, of which only the last
+// may reach past n.  R is 4 and at the end what is left, so that no warp takes its last chunks one after
+// another, as a compiler's remainder loop does.
+template <int R>
+struct Rounds {
+    static constexpr int value = R;
+};
+template <typename F>
+__device__ __forceinline__ void fused_chunks(int n, int slice, F &&rounds) {
+    constexpr int kStride = 32 * kFusedSlices;
+    const int lane = threadIdx.x & 31;
+    int b = slice * 32;  // warp-uniform
+    for (; b + 3 * kStride < n; b += 4 * kStride) rounds(Rounds<4>{}, b + lane);
+    if (b >= n) return;
+    if (b + kStride >= n) rounds(Rounds<1>{}, b + lane);
+    else if (b + 2 * kStride >= n) rounds(Rounds<2>{}, b + lane);
+    else rounds(Rounds<3>{}, b + lane);
+}
+
+template <int EPI, int I, int kFusedGroups, int MINB, bool FOURS>
 __global__ void __launch_bounds__(kFusedGroups * kFusedSlices * 32, MINB)
     fused_small_kernel(StepArgs st, const double4 *__restrict__ src, double G) {
     __shared__ double part[kFusedSlices][kFusedGroups][I][3];
@@ -725,9 +747,7 @@ __global__ void __launch_bounds__(kFusedGroups * kFusedSlices * 32, MINB)
         ax[k] = ay[k] = az[k] = 0.0;
     }
     if (i0 < st.n) {
-#pragma unroll 4
-        for (int64_t j = (int64_t)slice * 32 + lane; j < st.n; j += 32 * kFusedSlices) {
-            const double4 q = src[j];
+        auto pair = [&](const double4 &q) {
             const double gm = q.w * G;
 #pragma unroll
             for (int k = 0; k < I; ++k) {
@@ -738,25 +758,35 @@ __global__ void __launch_bounds__(kFusedGroups * kFusedSlices * 32, MINB)
                 ay[k] = fma(sc, dy, ay[k]);
                 az[k] = fma(sc, dz, az[k]);
             }
+        };
+        if constexpr (FOURS) {
+            fused_chunks((int)st.n, slice, [&](auto rounds, int j) {
+                constexpr int R = decltype(rounds)::value;
+                double4 q[R];
+#pragma unroll
+                for (int r = 0; r < R; ++r) {  // past the end: nothing, at the first body's place
+                    const int e = j + r * 32 * kFusedSlices;
+                    q[r] = r < R - 1 || e < (int)st.n ? src[e] : make_double4(p[0].x, p[0].y, p[0].z, 0.0);
+                }
+#pragma unroll
+                for (int r = 0; r < R; ++r) pair(q[r]);
+            });
+        } else {
+#pragma unroll 4
+            for (int64_t j = (int64_t)slice * 32 + lane; j < st.n; j += 32 * kFusedSlices) pair(src[j]);
         }
     }
     cudaTriggerProgrammaticLaunchCompletion();
+    double sums[3 * I];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-        for (int k = 0; k < I; ++k) {
-            ax[k] += __shfl_xor_sync(0xffffffffu, ax[k], o);
-            ay[k] += __shfl_xor_sync(0xffffffffu, ay[k], o);
-            az[k] += __shfl_xor_sync(0xffffffffu, az[k], o);
-        }
-    if (lane == 0) {
-#pragma unroll
-        for (int k = 0; k < I; ++k) {
-            part[slice][bl][k][0] = ax[k];
-            part[slice][bl][k][1] = ay[k];
-            part[slice][bl][k][2] = az[k];
-        }
+    for (int k = 0; k < I; ++k) {
+        sums[3 * k] = ax[k];
+        sums[3 * k + 1] = ay[k];
+        sums[3 * k + 2] = az[k];
     }
+    int at;
+    const double sum = warp_sums(sums, at);
+    if (at >= 0) (&part[slice][bl][0][0])[at] = sum;
     __syncthreads();
     if (slice == 0 && lane < I && i0 + lane < st.n) {
         double s[3];
@@ -770,28 +800,29 @@ __global__ void __launch_bounds__(kFusedGroups * kFusedSlices * 32, MINB)
     }
 }
 
-template <int I, int GROUPS, int MINB>
+template <int I, int GROUPS, int MINB, bool FOURS = false>
 static void launch_fused(int64_t n, const double4 *src, double G, int epi, const StepArgs &st, cudaStream_t s, bool early) {
     const unsigned grid = (unsigned)((n + GROUPS * I - 1) / (GROUPS * I));
     auto go = [&](auto k) { launch_chained(early, k, grid, GROUPS * kFusedSlices * 32, 0, s, st, src, G); };
     switch (epi) {
-        case EPI_ACC: go(fused_small_kernel<EPI_ACC, I, GROUPS, MINB>); break;
-        case EPI_KDK: go(fused_small_kernel<EPI_KDK, I, GROUPS, MINB>); break;
-        case EPI_DKD: go(fused_small_kernel<EPI_DKD, I, GROUPS, MINB>); break;
-        case EPI_EULER: go(fused_small_kernel<EPI_EULER, I, GROUPS, MINB>); break;
-        case EPI_PREDICT: go(fused_small_kernel<EPI_PREDICT, I, GROUPS, MINB>); break;
-        case EPI_CORR_MEULER: go(fused_small_kernel<EPI_CORR_MEULER, I, GROUPS, MINB>); break;
-        case EPI_CORR_MIDPOINT: go(fused_small_kernel<EPI_CORR_MIDPOINT, I, GROUPS, MINB>); break;
-        case EPI_ACC3: go(fused_small_kernel<EPI_ACC3, I, GROUPS, MINB>); break;
-        default: go(fused_small_kernel<EPI_KICK_DRIFT, I, GROUPS, MINB>); break;
+        case EPI_ACC: go(fused_small_kernel<EPI_ACC, I, GROUPS, MINB, FOURS>); break;
+        case EPI_KDK: go(fused_small_kernel<EPI_KDK, I, GROUPS, MINB, FOURS>); break;
+        case EPI_DKD: go(fused_small_kernel<EPI_DKD, I, GROUPS, MINB, FOURS>); break;
+        case EPI_EULER: go(fused_small_kernel<EPI_EULER, I, GROUPS, MINB, FOURS>); break;
+        case EPI_PREDICT: go(fused_small_kernel<EPI_PREDICT, I, GROUPS, MINB, FOURS>); break;
+        case EPI_CORR_MEULER: go(fused_small_kernel<EPI_CORR_MEULER, I, GROUPS, MINB, FOURS>); break;
+        case EPI_CORR_MIDPOINT: go(fused_small_kernel<EPI_CORR_MIDPOINT, I, GROUPS, MINB, FOURS>); break;
+        case EPI_ACC3: go(fused_small_kernel<EPI_ACC3, I, GROUPS, MINB, FOURS>); break;
+        default: go(fused_small_kernel<EPI_KICK_DRIFT, I, GROUPS, MINB, FOURS>); break;
     }
 }
 
 int launch_fused_small(int64_t n, const double4 *src, double G, int epi, const StepArgs &st, cudaStream_t s,
                        bool early) {
     if (n == 0) return GTD_OK;
-    if (n <= 900) launch_fused<1, 2, 4>(n, src, G, epi, st, s, early);
-    else if (n <= 5 * 148 * 2) launch_fused<2, 1, 5>(n, src, G, epi, st, s, early);
+    if (n <= 128) launch_fused<1, 2, 4>(n, src, G, epi, st, s, early);
+    else if (n <= 592) launch_fused<1, 2, 4, true>(n, src, G, epi, st, s, early);
+    else if (n <= 5 * 148 * 2) launch_fused<2, 1, 5, true>(n, src, G, epi, st, s, early);
     else if (n <= 8 * 148 * 2) launch_fused<2, 1, 8>(n, src, G, epi, st, s, early);
     else if (n <= 3 * 148 * 8) launch_fused<4, 2, 3>(n, src, G, epi, st, s, early);
     else launch_fused<2, 1, 8>(n, src, G, epi, st, s, early);

@@ -36,4 +36,30 @@ __device__ __forceinline__ double inv_r(double r2) {
     return y * fma(e, fma(0.375, e, 0.5), 1.0);
 }
 
+// NV sums over a warp's lanes, each with the additions of a butterfly (x + shfl_xor(x, 16), 8, .. 1), spread
+// over the lanes: at every round a lane passes on the half of the values that its partner keeps, so that
+// six sums take 8 exchanges of a double where butterflies take 30.  Returns this lane's sum and its number
+// in `at`, or -1 in lanes that hold a copy or nothing.
+template <int NV, int O = 16>
+__device__ __forceinline__ double warp_sums(const double (&v)[NV], int &at, int first = 0, int left = NV) {
+    const int lane = threadIdx.x & 31;
+    if constexpr (NV == 1) {
+        double s = v[0];
+#pragma unroll
+        for (int o = O; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        at = left > 0 && (lane & (2 * O - 1)) == 0 ? first : -1;
+        return s;
+    } else {
+        constexpr int K = (NV + 1) / 2;
+        const bool up = (lane & O) != 0;
+        double w[K];
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            const double lo = v[k], hi = K + k < NV ? v[K + k < NV ? K + k : 0] : 0.0;
+            w[k] = (up ? hi : lo) + __shfl_xor_sync(0xffffffffu, up ? lo : hi, O);
+        }
+        return warp_sums<K, O / 2>(w, at, up ? first + K : first, up ? left - K : min(left, K));
+    }
+}
+
 }  // namespace gtd

@@ -182,7 +182,7 @@ static int timed_event(gtd_system *s) {
 // Whether a force evaluation and its update are one fused FP64 launch.  With the mixed precision it is both
 // the faster kernel and the more precise one at these sizes, where launches and the slots' sum outweigh
 // the pair terms, and its steps replay from a graph: a KDK step of 100 bodies 1.9 us (two launches and
-// the host's 25), 1024 4.3 (30), 2048 8.8 (30), 4096 25 (39), 4736 32 (44).  Up to 4736 bodies the {2, 1, 8}
+// the host's 25), 1024 4.0 (30), 2048 8.7 (30), 4096 24.5 (39), 4736 32 (44).  Up to 4736 bodies the {2, 1, 8}
 // shape's CTAs make two whole rounds: FP64 4300 27.9 us against 29.4, 4736 31.9 against 37.1.
 static bool fused_force(const gtd_system *s) {
     if (s->precision == GTD_PREC_F64 && s->n <= kFusedMaxN) return true;
