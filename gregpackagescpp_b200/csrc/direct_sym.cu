@@ -558,9 +558,11 @@ __global__ void __launch_bounds__(kRedWarps * 32) sym_reduce_kernel(SymReduceArg
 // FP64: 0 up to N = 32768, 1 above (the wider group selects coincident bodies away over the same 1024
 // bodies as the ordered kernel that ran there).  Mixed: 0 folds a row after 128 columns and a column
 // after 16 steps (64 terms per packed half), as the ordered kernel does from N = 32768; 1 folds both
-// twice as often, as it does below.
+// twice as often, as it does below.  A unit's own cost is higher in the mixed kernel (its rows' frame and
+// boxes); with the FP64 kernel's 0.1 the units came out too short: N = 12000 116 us a step against 104,
+// 40000 672 against 650.
 static const SymShape kSymF64[] = {{4, 128, 64, 512}, {4, 128, 128, 1024}};
-static const SymShape kSymMixed[] = {{4, 128, 128, 512}, {4, 128, 64, 512}};
+static const SymShape kSymMixed[] = {{4, 128, 128, 512, 0.3}, {4, 128, 64, 512, 0.3}};
 
 SymShape sym_shape(int precision, int kind) { return precision == GTD_PREC_MIXED ? kSymMixed[kind] : kSymF64[kind]; }
 

@@ -19,6 +19,7 @@ struct SymGeom {
 constexpr size_t kSymSlotBytes = (size_t)5 << 28;  // 1.25 GiB
 struct SymShape {
     int i, threads, tile, group;
+    double unit = 0.1;  // what a unit costs beside its tiles, in tiles of 64 columns
 };
 
 // First unit block (P, P): super-groups P, Q of L groups, Q >= P, in row-major order.
@@ -85,13 +86,13 @@ inline SymGeom sym_geometry(int64_t n, const SymShape &sh, int sms, int per_sm) 
     const int64_t ctas = (int64_t)sms * per_sm;
     const int64_t blocks = g.G * (g.G + 1) / 2 * g.s;
     // The columns of a unit: where there are few groups each is cut into q parts.  A unit costs its
-    // tiles plus about a tenth of a 64-column tile, an SM runs per_sm units side by side (fewer leave
+    // tiles and sh.unit, an SM runs per_sm units side by side (fewer leave
     // its pipe partly idle), and the SM with the most units sets the time.
     double best = 0.0;
     for (int q = 1; g.kw % q == 0; q *= 2) {
         const double each = (double)((blocks * q + sms - 1) / sms);
         const double side = std::min<double>(each, per_sm);
-        const double cost = each * ((double)(g.kw / q) * g.TC / 64 + 0.1) * (side + per_sm) / (2.0 * side);
+        const double cost = each * ((double)(g.kw / q) * g.TC / 64 + sh.unit) * (side + per_sm) / (2.0 * side);
         if (q == 1 || cost < best) {
             best = cost;
             g.q = q;
