@@ -534,7 +534,8 @@ def run_ours(args, rank, world, local):
                          "algorithmic_bytes": 32 * n + part_bytes.value,
                          "algorithmic_bytes_note": "positions 32 B per body read once + the work units' FP64 "
                                                    f"partial sums ({units.value} units)",
-                         "kernel": "force_mixed_kernel", "flops_per_interaction": FLOPS_PER_INTERACTION,
+                         "kernel": "force_mixed_sym_kernel" if tuned["mixed"]["variant"] >= 9 else "force_mixed_kernel",
+                         "flops_per_interaction": FLOPS_PER_INTERACTION,
                          "peak_source": "measured FFMA/FFMA2 microkernel on this GPU (gtd_measure_fma_peak)",
                          "fp64_peak": peak64.value / 1e12, "hbm_peak_GBs": hbm_peak / 1e9,
                          "hbm_peak_source": hbm_src},

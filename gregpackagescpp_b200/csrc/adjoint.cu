@@ -323,7 +323,7 @@ __global__ void __launch_bounds__(kRedWarps * 32) vjp_reduce_kernel(SymSlots s, 
     });
 }
 
-// Two rows per thread, 3 CTAs per SM: 0.43 ms at N = 16384, 72 % of the FP64 pipe (the form with 47
+// Two rows per thread, 3 CTAs per SM: 0.43 ms at N = 16384, 69 % of the FP64 pipe (the form with 47
 // operations and a thread per body for the sums: 0.53).  Eight sums per body with u never formed (39
 // operations too) ran at 0.48 ms: twice the shuffles.  Four rows per thread: 240 registers, no faster.
 constexpr SymShape kVjpShape{2, 128, 64, 256};

@@ -15,7 +15,7 @@ constexpr int kThreadsMost = 8, kSlotsEach = 2;
 constexpr size_t kRingFrom = (size_t)4 << 20;  // smaller copies: starting the threads costs what they save
 // Pinning the ring takes 3.7 ms and the threads save 0.15 ms a MB: a handle's ring is made once the large
 // copies of its life, this one included, come to what that pays for.
-constexpr size_t kRingPays = (size_t)24 << 20;
+constexpr size_t kRingPays = (size_t)40 << 20;
 
 void release_host_ring(HostRing &ring) {
     for (cudaEvent_t e : ring.events) cudaEventDestroy(e);

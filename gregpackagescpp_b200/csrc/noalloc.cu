@@ -89,9 +89,9 @@ extern "C" int gtd_direct_accelerations_noalloc(int64_t n, const double *pm4, do
                     "pm4 and acc3 must be device (or managed) memory of the current device %d", dev);
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     if (n <= kFusedAutoMaxN) {
-        // one launch without partial sums: FP64 3.6 us at n = 1000 (6 with the launch), against 37 us for the wide kernel, whose
-        // 512-body rows give 8 CTAs there, and its sum; mixed 18.5 us there with the pair kernel and its sum,
-        // 27 against 29 at 4096
+        // one launch without partial sums.  FP64: 3.65 us at n = 1000 (8 with the launch), against 37 for the
+        // wide kernel, whose 512-body rows give 8 CTAs there, and its sum.  Mixed, launches included: the pair
+        // kernel and its sum took 18.5 us at n = 1000, 29 at 4096; this 6 and 26
         StepArgs sa{};
         sa.n = n;
         sa.acc = reinterpret_cast<double4 *>(acc3);

@@ -273,11 +273,14 @@ GTD_API int gtd_system_autotune_direct(gtd_system *sys, int reps, int *best, dou
  * gregsys.hpp:352-357).  The FP32 pair terms use coordinates relative to a per-row centre; a
  * pair closer than 2|X_i|/(k - 1) to body i (X_i its offset from that centre) would lose more
  * than k 2^-24 of its relative accuracy to their rounding, so the j-range holding it is summed
- * again from hi/lo coordinate splits.  Default k = 8; k <= 1 turns the check off. */
+ * again from hi/lo coordinate splits.  Default k = 8; k <= 1 turns the check off.  Handles of up to
+ * 4736 bodies whose variant is neither pinned nor tuned sum all pairs in FP64 and need no check. */
 GTD_API int gtd_system_set_mixed_near_factor(gtd_system *sys, double k);
 /* The split of the handle's direct-sum force (no counterpart in the reference): the work units of
- * one force evaluation (mixed: (row, segment) units taken from a work queue; FP64: (row, tile)
- * pairs) and the bytes of partial sums they write. */
+ * one force evaluation (row blocks against runs of columns, taken from a work queue; (row, tile)
+ * pairs for the ordered FP64 variants) and the bytes of partial sums they write.  Handles of up to
+ * 4736 bodies whose variant is neither pinned nor tuned (FP64: up to 4096 in any case) run one launch
+ * without either; the numbers are then the variant's. */
 GTD_API int gtd_system_direct_plan_info(gtd_system *sys, int64_t *units, int64_t *partial_bytes);
 /* Measured throughput of a dependent-FMA microkernel on `device` (all SMs): precision
  * GTD_PREC_MIXED gives FP32 FFMA FLOP/s, GTD_PREC_F64 gives FP64 DFMA FLOP/s (2 flops per FMA). */
@@ -325,7 +328,8 @@ GTD_API int gtd_bh_accelerations(gtd_system *sys, double *a3, uint32_t *n_inter)
  * host threads) race on it and must be serialised by the caller.  Nothing in it needs clearing
  * between calls (every partial sum read is written first by the same call).  The array's address
  * is kept per device after the first call; cudaDeviceReset discards the array, so the entry point
- * must not be used after a device reset.  pm4 and acc3 that are not device (or managed) memory of
+ * must not be used after a device reset.  Up to 4736 bodies the force is one FP64 launch in either
+ * precision and the array is not used.  pm4 and acc3 that are not device (or managed) memory of
  * the current device are rejected with GTD_ERR_INVALID_ARGUMENT before anything is launched.
  * GTD_PREC_MIXED sums the bodies in the order given (gtd_system reorders them spatially first);
  * its test bar against the FP64 result is 1e-6 RMS relative.  stream: a cudaStream_t or NULL; the

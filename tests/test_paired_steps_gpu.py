@@ -1,6 +1,6 @@
 """The callback loop's two-kernel steps (collide.cu) against the same loop run eagerly, with a kernel
 each for kick-drift, force, detection and resolution: the same bits, at the edges of the sizes that
-take them, with and without the functors, over full, part and odd chunks of steps."""
+take them and just above, with and without the functors, over full, part and odd chunks of steps."""
 
 import numpy as np
 import pytest
@@ -10,7 +10,7 @@ from gregpackagescpp_b200 import RestFromCom, System, WhileRestBelow, _lib
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n", [2, 3, 129, 900, 901, 4095, 4096])
+@pytest.mark.parametrize("n", [2, 3, 129, 900, 901, 4095, 4096, 5000])
 @pytest.mark.parametrize("steps,functors", [(1, True), (64, True), (65, False), (131, True)])
 def test_paired_steps_bit_identical(gpu, n, steps, functors):
     rng = np.random.default_rng(n + steps)
