@@ -640,12 +640,13 @@ __global__ void __launch_bounds__(kTT, sizeof(T) == 4 ? 6 : 1) walk_kernel(int64
 // lanes that refused it.  Evaluation: every lane runs down the list (three broadcast shared-memory
 // reads per two entries, stored as interleaved pairs) and keeps the terms its mask bit selects, with
 // walk_kernel's arithmetic per term; only the order of the sum differs.
-// Resident warps hide the traversal's dependent loads: 4 warps per CTA with 6.25 KB of shared
+// Resident warps hide the traversal's dependent loads: 4 warps per CTA with 6.75 KB of shared
 // memory each and at most 64 registers give 8 CTAs (32 warps) per SM (13.1 ms per walk at
 // N = 4194304, against 15.2 ms with a 512-entry stack at 24 warps per SM).
 // Double trees: the same traversal in FP64 (the bounds hold at any precision), entries of 32 bytes evaluated
-// by 17 FP64 operations each: 0.88 ms per walk at N = 131072, 3.17 at 524288, against 1.92 and 5.19 for
-// walk_kernel.
+// by 17 FP64 operations each: 0.84 ms per walk at N = 131072 against 1.92 for walk_kernel, 3.03 at 524288
+// against 5.19.  The nodes in between are read from shared memory by all lanes (four shuffled doubles a
+// node: 0.88 ms at N = 131072).
 constexpr int kLwWarps = 4;      // warps per CTA
 constexpr int kLwStack = 320;    // stack entries per warp (a walk of 2M bodies peaks near 220)
 constexpr int kLwDfs = kLwStack - 64;  // above this many entries the warp pops one entry at a time
@@ -663,8 +664,11 @@ struct LwWarp<float> {
     // evaluation reads two entries with two float4 loads whose halves are its FP32x2 operands
     float4 pxy[kLwList / 2], pzw[kLwList / 2];
     unsigned lm[kLwList];            // lanes that take it
+    float4 nd[32];                   // centre and width^2 of the nodes that every lane tests
+    __device__ __forceinline__ void put_node(unsigned l, const float4 &A, float w2) { nd[l] = make_float4(A.x, A.y, A.z, w2); }
+    __device__ __forceinline__ float4 node(int j) const { return nd[j]; }
 };
-static_assert(kLwList % 2 == 0 && (3 * kLwStack * sizeof(int)) % 16 == 0, "float4 pairs of list entries");
+static_assert(kLwList % 4 == 0 && (3 * kLwStack * sizeof(int)) % 16 == 0, "float4 pairs of list entries");
 
 template <>
 struct LwWarp<double> {
@@ -672,6 +676,15 @@ struct LwWarp<double> {
     unsigned mk[kLwStack];
     double2 xy[kLwList], zw[kLwList];
     unsigned lm[kLwList];
+    double2 nxy[32], nzw[32];
+    __device__ __forceinline__ void put_node(unsigned l, const double4 &A, double w2) {
+        nxy[l] = make_double2(A.x, A.y);
+        nzw[l] = make_double2(A.z, w2);
+    }
+    __device__ __forceinline__ double4 node(int j) const {
+        const double2 a = nxy[j], b = nzw[j];
+        return make_double4(a.x, a.y, b.x, b.y);
+    }
 };
 
 // writes list entry `at`
@@ -845,8 +858,9 @@ __global__ void __launch_bounds__(kLwWarps * 32, sizeof(T) == 4 ? 8 : 4)
     __syncwarp();
     // every pop takes one (node, warp) pair and each node enters the stack once per warp: at most
     // n_nodes batches
-    for (int64_t batch = 0; top > 0; ++batch) {
-        if (batch > n_nodes) {
+    const int ibase = (int)base;
+    for (int batch = 0; top > 0; ++batch) {
+        if (batch > nn) {
             if (lane == 0) atomicExch(status, 2);
             break;
         }
@@ -906,20 +920,23 @@ __global__ void __launch_bounds__(kLwWarps * 32, sizeof(T) == 4 ? 8 : 4)
         // the in-between nodes: each lane of the node's mask applies walk_kernel's test
         unsigned acc = 0;
         unsigned mm = __ballot_sync(0xffffffffu, mixed);
+        if (mm) {  // one broadcast read per node, where shuffles of its four values take as many
+            if (mixed) W.put_node(lane, A, w2);
+            __syncwarp();
+        }
         while (mm) {
             const int j = __ffs(mm) - 1;
             mm &= mm - 1;
-            const T cx = __shfl_sync(0xffffffffu, A.x, j), cy = __shfl_sync(0xffffffffu, A.y, j);
-            const T cz = __shfl_sync(0xffffffffu, A.z, j), cw = __shfl_sync(0xffffffffu, w2, j);
-            const T dx = sub_t(cx, p.x), dy = sub_t(cy, p.y), dz = sub_t(cz, p.z);
+            const V N = W.node(j);
+            const T dx = sub_t(N.x, p.x), dy = sub_t(N.y, p.y), dz = sub_t(N.z, p.z);
             // every lane tests; lane j keeps the answers of the lanes in its node's mask
-            const unsigned a = __ballot_sync(0xffffffffu, cw < mul_t(th2, lw_r2(dx, dy, dz)));
+            const unsigned a = __ballot_sync(0xffffffffu, N.w < mul_t(th2, lw_r2(dx, dy, dz)));
             if ((int)lane == j) acc = a & mk;
         }
         unsigned em = 0;
         if (leaf && count == 1) {
-            const int64_t own = (int64_t)B.y - base;  // the lane whose body this leaf holds
-            em = mk & ~((own >= 0 && own < 32) ? (1u << own) : 0u);
+            const unsigned own = (unsigned)(B.y - ibase);  // the lane whose body this leaf holds
+            em = mk & ~(own < 32u ? (1u << own) : 0u);
         } else if (far) {
             em = mk;
         } else if (mixed) {
@@ -963,8 +980,8 @@ __global__ void __launch_bounds__(kLwWarps * 32, sizeof(T) == 4 ? 8 : 4)
                     __syncwarp();
                 }
                 const int q = f + q0 + (int)lane;
-                const int64_t own = (int64_t)q - base;
-                const unsigned m1 = bm & ~((own >= 0 && own < 32) ? (1u << own) : 0u);
+                const unsigned own = (unsigned)(q - ibase);
+                const unsigned m1 = bm & ~(own < 32u ? (1u << own) : 0u);
                 const bool ap = q0 + (int)lane < c && m1 != 0u;
                 const unsigned b2 = __ballot_sync(0xffffffffu, ap);
                 if (ap) {
