@@ -76,6 +76,7 @@ struct gtd_system {
     uint64_t force_launches = 0;
 
     // Barnes-Hut linear octree (octree.cu); arrays indexed by sorted slot [n] or by node [cap]
+    int sort_full = 0;  // builds that take the full sort (long runs of equal prefixes were met)
     bool tree_valid = false;
     int tree_float = 1;
     int64_t tree_n = 0;                 // bodies the n-sized arrays were sized for

@@ -399,8 +399,9 @@ __global__ void __launch_bounds__(kTT) emit_kernel(EmitArgs e) {
 }
 
 // depth_off: [0, 21) the internal nodes per depth, [22, 43) how many of them are listed, [64, 86) the
-// exclusive sums of the counts, [90] the deepest level that has any.
-constexpr int kDepthWords = 96, kDeepest = 90;
+// exclusive sums of the counts, [90] the deepest level that has any, [91] whether the sort by prefix met a
+// run it leaves to the full sort.
+constexpr int kDepthWords = 96, kDeepest = 90, kLongRun = 91;
 constexpr int kDepthChunk = 16 * kTT;  // nodes per CTA of the listing
 
 // Lists the internal nodes by depth (the order inside a depth is free: each node's moments are
@@ -1154,8 +1155,9 @@ static int ensure_tree_nodes(gtd_system *s, int64_t nodes) {
     return GTD_OK;
 }
 
-// Morton codes of the current positions, sorted (codes, perm).  Leaves the box in s->box_dev.
-static int morton_sort(gtd_system *s, bool tree_float) {
+// Morton codes of the current positions, sorted (codes, perm), by prefix unless the full sort is wanted.
+// Leaves the box in s->box_dev.
+static int morton_sort(gtd_system *s, bool tree_float, bool full) {
     const int64_t n = s->n;
     int rc = ensure_tree_n(s, n);
     if (rc) return rc;
@@ -1174,7 +1176,9 @@ static int morton_sort(gtd_system *s, bool tree_float) {
     }
     GTD_CHECK_LAUNCH();
     s->launches += 3;
-    return radix_sort_u64(s->codes, s->perm, s->codes_alt, s->perm_alt, n, 63, s->scratch, st, &s->launches);
+    if (full) return radix_sort_u64(s->codes, s->perm, s->codes_alt, s->perm_alt, n, 63, s->scratch, st, &s->launches);
+    return radix_sort_prefix63(s->codes, s->perm, s->codes_alt, s->perm_alt, n, s->scratch, s->depth_off + kLongRun, st,
+                               &s->launches);
 }
 
 // Hilbert order of the current positions in s->perm (slot -> body), over the root box of the T=double
@@ -1216,27 +1220,40 @@ static int bh_build_impl(gtd_system *s, int tree_float) {
                                                     "Barnes-Hut cube.");
     }
     s->tree_float = tree_float ? 1 : 0;
-    int rc = morton_sort(s, tree_float != 0);
+    int rc = ensure_tree_n(s, n);
     if (rc) return rc;
     cudaStream_t st = s->stream;
     const double4 *pm = s->pm[s->cur];
-    GTD_CUDA(cudaMemsetAsync(s->depth_off, 0, kDepthWords * sizeof(uint32_t), st));
-    if (tree_float)
-        lcp_count_kernel<true><<<blocks_for(n + 1), kTT, 0, st>>>(s->codes, s->perm, pm, n, s->lcp, s->node_start,
-                                                                  s->status, s->depth_off + kDeepest);
-    else
-        lcp_count_kernel<false><<<blocks_for(n + 1), kTT, 0, st>>>(s->codes, s->perm, pm, n, s->lcp, s->node_start,
-                                                                   s->status, s->depth_off + kDeepest);
-    GTD_CHECK_LAUNCH();
-    s->launches += 1;
-    rc = exclusive_scan_u32(s->node_start, s->node_start, n + 1, s->scratch, st, &s->launches);
-    if (rc) return rc;
-    GTD_CUDA(cudaMemcpyAsync(s->host_total, s->node_start + n, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-    GTD_CUDA(cudaMemcpyAsync(s->host_total + 1, s->status, sizeof(int), cudaMemcpyDeviceToHost, st));
-    GTD_CUDA(cudaMemcpyAsync(s->host_total + 2, s->depth_off + kDeepest, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-    GTD_CUDA(cudaStreamSynchronize(st));
-    rc = build_error(s);
-    if (rc) return rc;
+    // Five sort passes order the codes of a tree whose 13-level cells hold a few bodies each; where a run of
+    // equal prefixes is too long (a tight cluster in a wide box), the rest of the sort follows, and the next
+    // builds of the handle take the full sort at once.
+    bool full = s->sort_full > 0;
+    if (full) s->sort_full -= 1;
+    for (bool again = false;; again = true) {
+        GTD_CUDA(cudaMemsetAsync(s->depth_off, 0, kDepthWords * sizeof(uint32_t), st));
+        rc = again ? radix_sort_u64(s->codes, s->perm, s->codes_alt, s->perm_alt, n, 63, s->scratch, st, &s->launches)
+                   : morton_sort(s, tree_float != 0, full);
+        if (rc) return rc;
+        if (tree_float)
+            lcp_count_kernel<true><<<blocks_for(n + 1), kTT, 0, st>>>(s->codes, s->perm, pm, n, s->lcp, s->node_start,
+                                                                      s->status, s->depth_off + kDeepest);
+        else
+            lcp_count_kernel<false><<<blocks_for(n + 1), kTT, 0, st>>>(s->codes, s->perm, pm, n, s->lcp, s->node_start,
+                                                                       s->status, s->depth_off + kDeepest);
+        GTD_CHECK_LAUNCH();
+        s->launches += 1;
+        rc = exclusive_scan_u32(s->node_start, s->node_start, n + 1, s->scratch, st, &s->launches);
+        if (rc) return rc;
+        GTD_CUDA(cudaMemcpyAsync(s->host_total, s->node_start + n, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+        GTD_CUDA(cudaMemcpyAsync(s->host_total + 1, s->status, sizeof(int), cudaMemcpyDeviceToHost, st));
+        GTD_CUDA(cudaMemcpyAsync(s->host_total + 2, s->depth_off + kDeepest, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+        GTD_CUDA(cudaStreamSynchronize(st));
+        rc = build_error(s);
+        if (rc) return rc;
+        if (full || !s->host_total[2 + kLongRun - kDeepest]) break;
+        full = true;
+        s->sort_full = 64;
+    }
     const int64_t nodes = s->host_total[0];
     rc = ensure_tree_nodes(s, nodes);
     if (rc) return rc;

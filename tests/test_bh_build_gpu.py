@@ -50,3 +50,21 @@ def test_forces_on_laid_out_bodies(gpu, tree_float):
     got = got[0] if isinstance(got, tuple) else got
     err = np.linalg.norm(got - want, axis=1) / np.linalg.norm(want, axis=1)
     assert err.max() < (1e-4 if tree_float else 1e-12)
+
+
+@pytest.mark.parametrize("run", [31, 32, 33, 1000])
+def test_build_with_runs_of_equal_prefixes(gpu, oracle, run):
+    """A cluster whose bodies share all that the five passes of the build's sort order by, up to the length
+    that is sorted in place and beyond (the full sort, which the handle's next builds take at once)."""
+    rng = np.random.default_rng(run)
+    x = np.concatenate([rng.uniform(0.0, 1.0, (500, 3)), 0.3 + rng.uniform(0.0, 2.0 ** -17, (run, 3))])
+    x = np.ascontiguousarray(x[rng.permutation(len(x))])
+    m = rng.uniform(0.5, 1.5, len(x))
+    s, t = gpu_tree(m, x, 0)
+    o = oracle.bh_tree(x, m, 0)
+    try:
+        compare_tree(t, o)
+        s.bh_build(0)
+        compare_tree(s.bh_tree(), o)
+    finally:
+        oracle.bh_free(o)
