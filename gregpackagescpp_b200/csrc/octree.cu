@@ -97,6 +97,8 @@ __global__ void bbox_partial_kernel(const double4 *pm, int64_t n, double *part) 
 // result); then one thread does the reference's arithmetic for the cube, greg8tree.hpp:1037-1046, in T.
 template <bool F>
 __global__ void bbox_final_kernel(const double *part, int blocks, double *box, int *status) {
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
     using TT = TreeT<F>;
     using T = typename TT::T;
     const int lane = threadIdx.x & 31;
@@ -166,6 +168,8 @@ __device__ __forceinline__ bool morton_of(double x, double y, double z, const do
 template <bool F>
 __global__ void morton_kernel(const double4 *pm, int64_t n, const double *box_g, unsigned long long *keys,
                               int32_t *vals, int *status) {
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
     __shared__ double box[6];
     if (threadIdx.x < 6) box[threadIdx.x] = box_g[threadIdx.x];
     __syncthreads();
@@ -245,6 +249,8 @@ __device__ __forceinline__ int lcp_digits(unsigned long long a, unsigned long lo
 template <bool F>
 __global__ void lcp_count_kernel(const unsigned long long *codes, const int32_t *perm, const double4 *pm, int64_t n,
                                  int32_t *lcp, uint32_t *cnt, int *status, uint32_t *deepest) {
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
     using TT = TreeT<F>;
     const int64_t a = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     int la = -1;
@@ -409,6 +415,8 @@ constexpr int kDepthChunk = 16 * kTT;  // nodes per CTA of the listing
 // and reserves one range per depth with a single global atomic.
 __global__ void __launch_bounds__(kTT) depth_scatter_kernel(const int8_t *depth, const int8_t *leaf, int64_t n_nodes,
                                                             uint32_t *depth_off, int32_t *list) {
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
     constexpr int kItems = kDepthChunk / kTT;
     __shared__ uint32_t cnt[kMaxDepth], start[kMaxDepth], off[32];
     const int t = threadIdx.x;
@@ -475,6 +483,8 @@ template <bool F, bool IL = false>
 __global__ void walk_records_kernel(int64_t n_nodes, const double4 *com, const double *width, const int8_t *leaf,
                                     const int32_t *first, const int32_t *count, const int32_t *skip, double G,
                                     void *rec_a, int4 *rec_b, double *w2_64) {
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
     const int64_t nd = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (nd >= n_nodes) return;
     const double4 c = com[nd];
@@ -1167,12 +1177,12 @@ static int morton_sort(gtd_system *s, bool tree_float, bool full) {
     const int bb = (int)std::min<int64_t>(kBBoxBlocks, std::max<int64_t>(1, (n + kTT - 1) / kTT));
     if (tree_float) {
         bbox_partial_kernel<true><<<bb, kTT, 0, st>>>(pm, n, s->bbox_part);
-        bbox_final_kernel<true><<<1, 32, 0, st>>>(s->bbox_part, bb, s->box_dev, s->status);
-        morton_kernel<true><<<blocks_for(n), kTT, 0, st>>>(pm, n, s->box_dev, s->codes, s->perm, s->status);
+        launch_chained(true, bbox_final_kernel<true>, 1, 32, 0, st, s->bbox_part, bb, s->box_dev, s->status);
+        launch_chained(true, morton_kernel<true>, blocks_for(n), kTT, 0, st, pm, n, s->box_dev, s->codes, s->perm, s->status);
     } else {
         bbox_partial_kernel<false><<<bb, kTT, 0, st>>>(pm, n, s->bbox_part);
-        bbox_final_kernel<false><<<1, 32, 0, st>>>(s->bbox_part, bb, s->box_dev, s->status);
-        morton_kernel<false><<<blocks_for(n), kTT, 0, st>>>(pm, n, s->box_dev, s->codes, s->perm, s->status);
+        launch_chained(true, bbox_final_kernel<false>, 1, 32, 0, st, s->bbox_part, bb, s->box_dev, s->status);
+        launch_chained(true, morton_kernel<false>, blocks_for(n), kTT, 0, st, pm, n, s->box_dev, s->codes, s->perm, s->status);
     }
     GTD_CHECK_LAUNCH();
     s->launches += 3;
@@ -1211,6 +1221,9 @@ static int build_error(gtd_system *s) {
     return GTD_OK;
 }
 
+// The build's kernels are chained launches where one follows another: a step of 1000 bodies 0.205 ms with
+// full launches, 0.191 so; 16384 0.41 and 0.395.  (The walk, the scatter and the drift chained as well: a
+// step of 16384 bodies 0.57 ms.)
 static int bh_build_impl(gtd_system *s, int tree_float) {
     const int64_t n = s->n;
     s->tree_valid = false;
@@ -1234,12 +1247,8 @@ static int bh_build_impl(gtd_system *s, int tree_float) {
         rc = again ? radix_sort_u64(s->codes, s->perm, s->codes_alt, s->perm_alt, n, 63, s->scratch, st, &s->launches)
                    : morton_sort(s, tree_float != 0, full);
         if (rc) return rc;
-        if (tree_float)
-            lcp_count_kernel<true><<<blocks_for(n + 1), kTT, 0, st>>>(s->codes, s->perm, pm, n, s->lcp, s->node_start,
-                                                                      s->status, s->depth_off + kDeepest);
-        else
-            lcp_count_kernel<false><<<blocks_for(n + 1), kTT, 0, st>>>(s->codes, s->perm, pm, n, s->lcp, s->node_start,
-                                                                       s->status, s->depth_off + kDeepest);
+        launch_chained(true, tree_float ? lcp_count_kernel<true> : lcp_count_kernel<false>, blocks_for(n + 1), kTT, 0, st,
+                       s->codes, s->perm, pm, n, s->lcp, s->node_start, s->status, s->depth_off + kDeepest);
         GTD_CHECK_LAUNCH();
         s->launches += 1;
         rc = exclusive_scan_u32(s->node_start, s->node_start, n + 1, s->scratch, st, &s->launches);
@@ -1263,29 +1272,21 @@ static int bh_build_impl(gtd_system *s, int tree_float) {
     else emit_kernel<false><<<blocks_for(n), kTT, 0, st>>>(e);
     GTD_CHECK_LAUNCH();
     const unsigned depth_blocks = (unsigned)((nodes + kDepthChunk - 1) / kDepthChunk);
-    depth_scatter_kernel<<<depth_blocks, kTT, 0, st>>>(s->ndepth, s->nleaf, nodes, s->depth_off, s->depth_list);
+    launch_chained(true, depth_scatter_kernel, depth_blocks, kTT, 0, st, s->ndepth, s->nleaf, nodes, s->depth_off, s->depth_list);
     GTD_CHECK_LAUNCH();
     s->launches += 2;
     const int deepest = std::min((int)s->host_total[2], kMaxDepth - 1);
     for (int d = deepest; d >= 0; --d) {
-        launch_chained(d < deepest, com_level_kernel, 4 * 148, kTT, 0, st, s->depth_list, s->depth_off, d, s->nskip,
+        launch_chained(true, com_level_kernel, 4 * 148, kTT, 0, st, s->depth_list, s->depth_off, d, s->nskip,
                        s->ncom);
         s->launches += 1;
     }
     GTD_CHECK_LAUNCH();
     s->walk_interleaved = (tree_float && walk_variant_of(s) >= 1) ? 1 : 0;
-    if (s->walk_interleaved)
-        walk_records_kernel<true, true><<<blocks_for(nodes), kTT, 0, st>>>(nodes, s->ncom, s->nwidth, s->nleaf,
-                                                                            s->nfirst, s->ncount, s->nskip, s->G,
-                                                                            s->nwalk_a, s->nwalk_b, s->nwalk_w2);
-    else if (tree_float)
-        walk_records_kernel<true><<<blocks_for(nodes), kTT, 0, st>>>(nodes, s->ncom, s->nwidth, s->nleaf, s->nfirst,
-                                                                      s->ncount, s->nskip, s->G, s->nwalk_a,
-                                                                      s->nwalk_b, s->nwalk_w2);
-    else
-        walk_records_kernel<false><<<blocks_for(nodes), kTT, 0, st>>>(nodes, s->ncom, s->nwidth, s->nleaf, s->nfirst,
-                                                                       s->ncount, s->nskip, s->G, s->nwalk_a,
-                                                                       s->nwalk_b, s->nwalk_w2);
+    launch_chained(true, s->walk_interleaved ? walk_records_kernel<true, true>
+                         : tree_float ? walk_records_kernel<true> : walk_records_kernel<false>,
+                   blocks_for(nodes), kTT, 0, st, nodes, s->ncom, s->nwidth, s->nleaf, s->nfirst, s->ncount, s->nskip, s->G,
+                   s->nwalk_a, s->nwalk_b, s->nwalk_w2);
     GTD_CHECK_LAUNCH();
     s->launches += 1;
     s->n_nodes = nodes;
