@@ -26,6 +26,7 @@
 #include <numeric>
 #include <vector>
 
+#include "ensemble_rows.cuh"
 #include "gtd_internal.cuh"
 #include "host_copy.cuh"
 
@@ -396,15 +397,14 @@ __device__ __forceinline__ int ens_force_rows(int r0, int s, int nc, int npad, c
     int own[IB];        // fold of the row's own body
 #pragma unroll
     for (int b = 0; b < IB; ++b) {
-        const int i = r0 + b * s;
-        const int ic = i < nc ? i : r0;  // a missing row repeats the first; its result is dropped
+        const int ic = ens_staged_row(r0 + b * s, r0, nc);
         nx[b] = make_float2(-sx[ic], -sx[ic]);
         ny[b] = make_float2(-sy[ic], -sy[ic]);
         nz[b] = make_float2(-sz[ic], -sz[ic]);
         ax[b] = ay[b] = az[b] = 0.0;
         mnf[b] = INFINITY;
         mnr[b] = 0xffffffffu;
-        own[b] = ic / kEnsFold;
+        own[b] = ens_stand_in(r0 + b * s, r0, nc) / kEnsFold;
     }
     const float2 fl2 = make_float2(floor2, floor2);
     const unsigned fbits = (unsigned)__float_as_int(floor2) + 1u;
@@ -579,11 +579,10 @@ __global__ void __launch_bounds__(IB == 1 ? 512 : 256) ensemble_step_kernel(EnsA
     double4 *pos = a.pos + b0, *vel = a.vel + b0, *acc = a.acc + b0;
     double *rad = a.rad + b0;
     int n = a.cnt[s];
-    // the rows of [row0, row1): each of the first sw threads (sw the smallest multiple of 32 with
-    // IB sw >= rows) takes t, t + sw, ...: threads hold IB valid rows except in the last warp, and whole
-    // warps past sw sit out
+    // the rows of [row0, row1): each of the first sw threads takes t, t + sw, ...: threads hold IB valid
+    // rows except in the last warp, and whole warps past sw sit out
     auto rows = [&](int row0, int row1, const EnsInfo &f, bool kick, EnsCand *list) {
-        const int sw = ((row1 - row0 + IB - 1) / IB + 31) & ~31;
+        const int sw = ens_row_threads(row1 - row0, IB);
         if (t < sw)
             ens_force_rows<IB>(row0 + t, sw, row1, (n + 1) & ~1, sx, sy, sz, sm, pos, vel, acc, rad, f.rmax, f.slack, kick,
                                h2, f.floor2, list);
@@ -671,7 +670,6 @@ void with_ens_kernel(int ib, F &&f) {
     else f(ensemble_step_kernel<1>);
 }
 
-int ens_stride(int max_n) { return std::max(2, (max_n + 1) & ~1); }
 int ens_smem_bytes(int max_n) { return 4 * ens_stride(max_n) * (int)sizeof(float); }
 
 }  // namespace gtd
