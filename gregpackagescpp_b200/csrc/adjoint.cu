@@ -253,7 +253,7 @@ constexpr int kVjpSlices = 4;
 
 template <int I, int GROUPS, int MINB>
 __global__ void __launch_bounds__(GROUPS * kVjpSlices * 32, MINB)
-    vjp_small_kernel(int64_t n, const double4 *__restrict__ x, const double4 *__restrict__ w, VjpUpdate up) {
+    vjp_small_kernel(int64_t n, const double4 *x, const double4 *w, VjpUpdate up) {
     __shared__ double part[kVjpSlices][GROUPS][I][4];
     cudaGridDependencySynchronize();
     const int wp = threadIdx.x >> 5, lane = threadIdx.x & 31;

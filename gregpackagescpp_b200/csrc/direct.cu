@@ -733,7 +733,7 @@ __device__ __forceinline__ void fused_chunks(int n, int slice, F &&rounds) {
 
 template <int EPI, int I, int kFusedGroups, int MINB, bool FOURS>
 __global__ void __launch_bounds__(kFusedGroups * kFusedSlices * 32, MINB)
-    fused_small_kernel(StepArgs st, const double4 *__restrict__ src, double G) {
+    fused_small_kernel(StepArgs st, const double4 *src, double G) {
     __shared__ double part[kFusedSlices][kFusedGroups][I][3];
     cudaGridDependencySynchronize();
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;

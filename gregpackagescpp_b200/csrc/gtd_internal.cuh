@@ -28,7 +28,9 @@ int cuda_fail(cudaError_t e, const char *what, const char *file, int line);
 // Launches k; with chained, its blocks may be set up while the kernel before it in the stream still runs.
 // Such a kernel begins with cudaGridDependencySynchronize(), so that all memory is as that kernel leaves
 // it, and calls cudaTriggerProgrammaticLaunchCompletion() once a next one's blocks may take its SMs'
-// room.  Errors show in GTD_CHECK_LAUNCH().
+// room.  What the kernel before it writes is never passed as const __restrict__: that promises memory
+// which does not change while this kernel lives, and lets its loads go by the read-only path or ahead of
+// the wait.  Errors show in GTD_CHECK_LAUNCH().
 template <typename... P, typename... A>
 void launch_chained(bool chained, void (*k)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, A &&...a) {
     cudaLaunchAttribute at;
