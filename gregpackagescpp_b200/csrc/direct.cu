@@ -484,11 +484,6 @@ int tuned_variant(int device, int precision, int64_t n) {
     return it != g_tuned.end() ? it->second : default_variant(precision, n);
 }
 
-bool variant_tuned(int device, int precision, int64_t n) {
-    std::lock_guard<std::mutex> lock(g_tuned_mu);
-    return g_tuned.count(std::make_tuple(device, precision, size_class(n))) != 0;
-}
-
 int variant_info(int precision, int v, int *i, int *fold) {
     if (v < 0 || v >= variant_count(precision)) return fail(GTD_ERR_INVALID_ARGUMENT, "variant %d out of range", v);
     const VariantInfo &vi = precision == GTD_PREC_MIXED ? kMixedVariants[v] : kF64Variants[v];

@@ -128,13 +128,12 @@ int noalloc_variant(int precision, int64_t n);
 // Kernels that a force evaluation and its integration launch.
 int force_launch_count(const ForcePlan &p);
 // Up to this many bodies an FP64 force evaluation and its update run as one fused launch (direct.cu), and
-// up to kFusedAutoMaxN, in either precision, where no variant was pinned or tuned.
+// up to kFusedAutoMaxN, in either precision, where no variant was pinned.
 constexpr int64_t kFusedMaxN = 4096, kFusedAutoMaxN = 4736;
 int launch_fused_small(int64_t n, const double4 *src, double G, int epi, const StepArgs &st, cudaStream_t s,
                        bool early = false);
 void remember_variant(int device, int precision, int64_t n, int variant);
 int tuned_variant(int device, int precision, int64_t n);
-bool variant_tuned(int device, int precision, int64_t n);  // remembered, not the default
 size_t partial_bytes(const ForcePlan &p);
 // Shrinks the plan's partial-sum footprint to at most max_bytes (fewer queue segments, or a smaller
 // stream-K grid); GTD_ERR_CAPACITY when even the smallest split does not fit.

@@ -183,10 +183,11 @@ static int timed_event(gtd_system *s) {
 // the faster kernel and the more precise one at these sizes, where launches and the slots' sum outweigh
 // the pair terms, and its steps replay from a graph: a KDK step of 100 bodies 1.9 us (two launches and
 // the host's 25), 1024 4.0 (30), 2048 8.7 (30), 4096 24.5 (39), 4736 32 (44).  Up to 4736 bodies the {2, 1, 8}
-// shape's CTAs make two whole rounds: FP64 4300 27.9 us against 29.4, 4736 31.9 against 37.1.
+// shape's CTAs make two whole rounds: FP64 4300 27.9 us against 29.4, 4736 31.9 against 37.1.  Only a pinned
+// variant is taken instead: a tuned one is the fastest of the variants, and those are slower.
 static bool fused_force(const gtd_system *s) {
     if (s->precision == GTD_PREC_F64 && s->n <= kFusedMaxN) return true;
-    return s->n <= kFusedAutoMaxN && !s->variant_pinned && !variant_tuned(s->device, s->precision, s->n);
+    return s->n <= kFusedAutoMaxN && !s->variant_pinned;
 }
 
 int force_and_integrate(gtd_system *s, const double4 *src, int epi, const StepArgs &st) {

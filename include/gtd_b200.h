@@ -262,7 +262,9 @@ GTD_API int gtd_system_force_timing(gtd_system *sys, double *total_ms, uint64_t 
  * bodies (a warm-up and `reps` timed force launches each, median), keeps the fastest for the handle
  * and remembers it for the process: every handle without a pinned variant on the same device, with
  * the same precision and an N of the same bit length, then uses it (untuned: a fixed choice by
- * precision and N).  It leaves the bodies untouched apart from their order on the device.
+ * precision and N).  Handles of up to 4736 bodies without a pinned variant run one fused FP64 launch
+ * per force, which is faster than every variant, whatever was tuned.  It leaves the bodies untouched
+ * apart from their order on the device.
  * gtd_system_set_direct_variant pins a variant for the handle; variant < 0 unpins it. */
 GTD_API int gtd_direct_variant_count(int precision, int *count);
 GTD_API int gtd_direct_variant_info(int precision, int variant, int *i_per_thread, int *fold);
@@ -274,12 +276,12 @@ GTD_API int gtd_system_autotune_direct(gtd_system *sys, int reps, int *best, dou
  * pair closer than 2|X_i|/(k - 1) to body i (X_i its offset from that centre) would lose more
  * than k 2^-24 of its relative accuracy to their rounding, so the j-range holding it is summed
  * again from hi/lo coordinate splits.  Default k = 8; k <= 1 turns the check off.  Handles of up to
- * 4736 bodies whose variant is neither pinned nor tuned sum all pairs in FP64 and need no check. */
+ * 4736 bodies whose variant is not pinned sum all pairs in FP64 and need no check. */
 GTD_API int gtd_system_set_mixed_near_factor(gtd_system *sys, double k);
 /* The split of the handle's direct-sum force (no counterpart in the reference): the work units of
  * one force evaluation (row blocks against runs of columns, taken from a work queue; (row, tile)
  * pairs for the ordered FP64 variants) and the bytes of partial sums they write.  Handles of up to
- * 4736 bodies whose variant is neither pinned nor tuned (FP64: up to 4096 in any case) run one launch
+ * 4736 bodies whose variant is not pinned (FP64: up to 4096 in any case) run one launch
  * without either; the numbers are then the variant's. */
 GTD_API int gtd_system_direct_plan_info(gtd_system *sys, int64_t *units, int64_t *partial_bytes);
 /* Measured throughput of a dependent-FMA microkernel on `device` (all SMs): precision

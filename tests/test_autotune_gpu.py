@@ -1,0 +1,47 @@
+"""gtd_system_autotune_direct never leaves a handle on a slower kernel: at the sizes of the fused FP64
+launch, which no variant beats, tuning changes nothing for a handle without a pinned variant."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from gregpackagescpp_b200 import System, _lib
+from gregpackagescpp_b200.ics import UNITS_G6674, plummer
+
+pytestmark = pytest.mark.gpu
+
+
+def _system(n, precision):
+    m, x, v = plummer(n, n)
+    s = System(m, x, v, timestep=3600.0, num_iterations=20, units_format=UNITS_G6674, precision=precision)
+    s._push()
+    return s
+
+
+def _tune(s, reps=1):
+    best = C.c_int()
+    _lib.check(s._L.gtd_system_autotune_direct(s._h, reps, C.byref(best), None))
+    return best.value
+
+
+@pytest.mark.parametrize("tuned", ["itself", "another"])
+@pytest.mark.parametrize("n,precision", [(100, "mixed"), (1024, "mixed"), (4700, "mixed"), (1024, "f64"), (4700, "f64")])
+def test_tuning_keeps_the_fused_launch(gpu, n, precision, tuned):
+    """Tuned itself, or by another handle of its size class: force and steps have the bits and the number
+    of launches of a handle nobody tuned; a pinned variant is still taken (mixed: FP32 pair terms)."""
+    want = _system(n, precision)
+    before = want.launch_count()
+    a = want.accelerations()
+    launches = want.launch_count() - before
+    want.evolve(System.leapfrog_kdk)
+    s, other = _system(n, precision), _system(n + (n & 1) + 1, precision)
+    best = _tune(s if tuned == "itself" else other)
+    before = s.launch_count()
+    assert np.array_equal(s.accelerations(), a)
+    assert s.launch_count() - before == launches
+    s.evolve(System.leapfrog_kdk)
+    assert np.array_equal(s.x, want.x) and np.array_equal(s.v, want.v)
+    if precision == "mixed":
+        p = _system(n, precision)
+        _lib.check(p._L.gtd_system_set_direct_variant(p._h, best))
+        assert not np.array_equal(p.accelerations(), a)
