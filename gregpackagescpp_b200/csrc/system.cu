@@ -802,18 +802,19 @@ int gtd_system_autotune_direct(gtd_system *s, int reps, int *best, double *best_
         s->variant = v;
         rc = ensure_plan(s);
         if (rc) return rc;
-        // warm-up launch, then the median of `reps` timed force launches
-        s->plan.n = 0;  // force kernels alone leave their counters used: whoever comes next makes them anew
-        ForcePlan p = s->plan;
-        p.n = s->n;
-        rc = launch_force(s->precision, p, s->pm[s->cur], s->G, s->partials, s->stream);
-        if (rc) return rc;
-        std::vector<float> t(reps);
-        for (int k = 0; k < reps; ++k) {
-            if (p.sym && (rc = sym_reset(p, s->partials, s->stream))) return rc;
+        // a warm-up evaluation, then the median of `reps` timed ones: the force kernel and the sum of its partial
+        // sums, which the unordered-pair variants have more of.  The sums go to the idle position buffer.
+        StepArgs st = step_args(s, s->pm[s->cur], true);
+        st.acc = s->pm[s->cur ^ 1];
+        std::vector<float> t((size_t)reps);
+        for (int k = -1; k < reps; ++k) {
             GTD_CUDA(cudaEventRecord(s->ev0, s->stream));
-            rc = launch_force(s->precision, p, s->pm[s->cur], s->G, s->partials, s->stream);
-            if (rc) return rc;
+            rc = launch_force(s->precision, s->plan, s->pm[s->cur], s->G, s->partials, s->stream, true);
+            if (!rc) rc = launch_integrate(s->plan, s->partials, EPI_ACC, st, s->stream, true);
+            if (rc) {
+                s->plan.n = 0;  // as in force_and_integrate
+                return rc;
+            }
             GTD_CUDA(cudaEventRecord(s->ev1, s->stream));
             GTD_CUDA(cudaEventSynchronize(s->ev1));
             GTD_CUDA(cudaEventElapsedTime(&t[k], s->ev0, s->ev1));

@@ -259,7 +259,8 @@ GTD_API int gtd_system_time_force_kernels(gtd_system *sys, int enable);
 GTD_API int gtd_system_force_timing(gtd_system *sys, double *total_ms, uint64_t *launches, int reset);
 /* Force-kernel variants (i-bodies per thread; for GTD_PREC_MIXED also the j-bodies summed in FP32
  * between FP64 folds).  gtd_system_autotune_direct times every variant on the handle's current
- * bodies (a warm-up and `reps` timed force launches each, median), keeps the fastest for the handle
+ * bodies (a warm-up and `reps` timed force evaluations each, their partial sums added up, median;
+ * *best_ms: the fastest variant's), keeps the fastest for the handle
  * and remembers it for the process: every handle without a pinned variant on the same device, with
  * the same precision and an N of the same bit length, then uses it (untuned: a fixed choice by
  * precision and N).  Handles of up to 4736 bodies without a pinned variant run one fused FP64 launch

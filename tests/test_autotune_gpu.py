@@ -45,3 +45,18 @@ def test_tuning_keeps_the_fused_launch(gpu, n, precision, tuned):
         p = _system(n, precision)
         _lib.check(p._L.gtd_system_set_direct_variant(p._h, best))
         assert not np.array_equal(p.accelerations(), a)
+
+
+def test_whole_evaluations_are_timed(gpu):
+    """A variant is judged by its force kernel and the sum of its partial sums: both run, reps + 1 times per
+    variant (two launches each at this size), and the bodies and what a step gives from them stay."""
+    n, reps = 9000, 2
+    want, s = _system(n, "f64"), _system(n, "f64")
+    count, before = C.c_int(), s.launch_count()
+    _lib.check(s._L.gtd_direct_variant_count(_lib.PREC_F64, C.byref(count)))
+    best = _tune(s, reps)
+    assert s.launch_count() - before == count.value * (reps + 1) * 2
+    _lib.check(want._L.gtd_system_set_direct_variant(want._h, best))
+    for h in (s, want):
+        h.evolve(System.leapfrog_kdk)
+    assert np.array_equal(s.x, want.x) and np.array_equal(s.v, want.v)
