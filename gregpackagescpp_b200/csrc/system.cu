@@ -817,9 +817,9 @@ int gtd_system_autotune_direct(gtd_system *s, int reps, int *best, double *best_
             }
             GTD_CUDA(cudaEventRecord(s->ev1, s->stream));
             GTD_CUDA(cudaEventSynchronize(s->ev1));
-            GTD_CUDA(cudaEventElapsedTime(&t[k], s->ev0, s->ev1));
+            if (k >= 0) GTD_CUDA(cudaEventElapsedTime(&t[(size_t)k], s->ev0, s->ev1));
         }
-        s->launches += (uint64_t)reps + 1;
+        s->launches += (uint64_t)(reps + 1) * (uint64_t)force_launch_count(s->plan);
         std::sort(t.begin(), t.end());
         const double med = t[reps / 2];
         if (med < bestv) {
