@@ -119,6 +119,31 @@ void release_bodies(gtd_system *s) {
     s->cap = 0;
 }
 
+// Memory for the plan's partial sums.  Where that much cannot be had, the unordered-pair kernels take more
+// and smaller batches (N = 262144: 1.34 GB in two batches, 38 MB at the least).
+static int ensure_partials(gtd_system *s) {
+    size_t need = partial_bytes(s->plan);
+    if (need <= s->part_bytes) return GTD_OK;
+    release_graph(s);  // its kernels hold the old address
+    cudaFree(s->partials);
+    s->partials = nullptr;
+    s->part_bytes = 0;
+    cudaError_t e;
+    while ((e = cudaMalloc(&s->partials, need)) != cudaSuccess) {
+        s->partials = nullptr;
+        ForcePlan p = s->plan;
+        if (e != cudaErrorMemoryAllocation || !p.sym || sym_fit(p, need / 2)) {
+            s->plan.n = 0;  // no plan
+            return cuda_fail(e, "partial sums", __FILE__, __LINE__);
+        }
+        cudaGetLastError();
+        s->plan = p;
+        need = partial_bytes(p);
+    }
+    s->part_bytes = need;
+    return GTD_OK;
+}
+
 int ensure_plan(gtd_system *s) {
     if (!s->variant_pinned) s->variant = tuned_variant(s->device, s->precision, s->n);
     if (s->plan.n == s->n && s->plan_prec == s->precision && s->plan.variant == s->variant && s->partials) {
@@ -128,19 +153,9 @@ int ensure_plan(gtd_system *s) {
     s->plan = make_plan(s->n, s->precision, s->device, s->variant);
     s->plan.near2 = near2_of(s->near_factor);
     s->plan_prec = s->precision;
-    const size_t need = partial_bytes(s->plan);
-    if (need > s->part_bytes) {
-        cudaFree(s->partials);
-        s->partials = nullptr;
-        GTD_CUDA(cudaMalloc(&s->partials, need));
-        s->part_bytes = need;
-    }
-    if (s->plan.sym) {
-        const int rc = sym_reset(s->plan, s->partials, s->stream);
-        if (rc) s->plan.n = 0;  // no plan
-        return rc;
-    }
-    return GTD_OK;
+    int rc = ensure_partials(s);
+    if (!rc && s->plan.sym && (rc = sym_reset(s->plan, s->partials, s->stream))) s->plan.n = 0;  // no plan
+    return rc;
 }
 
 static int ensure_pred(gtd_system *s) {
