@@ -288,6 +288,7 @@ static int build_loop_graph(gtd_system *s, const int *coll_status, cudaGraphExec
     uint64_t per_step = 0;
     bool fused = false;
     const bool builtin = s->cb.cont_kind != 1;
+    HoldPlan hold(s);
     int rc = [&]() -> int {
         cudaGraphConditionalHandle hw, h1, h2, h3;
         GTD_CUDA(cudaGraphConditionalHandleCreate(&hw, G, 1, cudaGraphCondAssignDefault));

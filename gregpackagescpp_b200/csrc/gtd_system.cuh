@@ -56,6 +56,7 @@ struct gtd_system {
     int plan_prec = -1;
     int variant = 0;              // force-kernel variant in use
     bool variant_pinned = false;  // set by gtd_system_set_direct_variant; else the process-wide choice
+    bool plan_held = false;       // steps are being captured: the variant and the plan stay (HoldPlan)
     double near_factor = gtd::kDefaultNearFactor;  // mixed kernel's precise-path factor K
     double *partials = nullptr;
     size_t part_bytes = 0;
@@ -241,4 +242,11 @@ int ensure_body_capacity(gtd_system *s, int64_t n);
 int ensure_stage(gtd_system *s, size_t bytes);
 int set_loaded_bodies(gtd_system *s, int64_t n);
 int ensure_plan(gtd_system *s);
+// While one lives, ensure_plan keeps the plan as it stands: the steps of a captured graph all run one plan,
+// whatever another thread tunes meanwhile, and none of them allocates.
+struct HoldPlan {
+    gtd_system *s;
+    explicit HoldPlan(gtd_system *sys) : s(sys) { s->plan_held = true; }
+    ~HoldPlan() { s->plan_held = false; }
+};
 int force_and_integrate(gtd_system *s, const double4 *src, int epi, const gtd::StepArgs &st);

@@ -145,7 +145,7 @@ static int ensure_partials(gtd_system *s) {
 }
 
 int ensure_plan(gtd_system *s) {
-    if (!s->variant_pinned) s->variant = tuned_variant(s->device, s->precision, s->n);
+    if (!s->variant_pinned && !s->plan_held) s->variant = tuned_variant(s->device, s->precision, s->n);
     if (s->plan.n == s->n && s->plan_prec == s->precision && s->plan.variant == s->variant && s->partials) {
         s->plan.near2 = near2_of(s->near_factor);
         return GTD_OK;
@@ -417,7 +417,10 @@ static int run_graph_chunk(gtd_system *s) {
         const bool synced0 = s->synced;
         const uint64_t launches0 = s->launches;
         GTD_CUDA(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
-        for (int c = 0; c < kGraphSteps && !rc; ++c) rc = direct_step(s, s->method, false);
+        {
+            HoldPlan hold(s);
+            for (int c = 0; c < kGraphSteps && !rc; ++c) rc = direct_step(s, s->method, false);
+        }
         cudaGraph_t g = nullptr;
         const cudaError_t ce = cudaStreamEndCapture(s->stream, &g);
         s->graph_launches = s->launches - launches0;

@@ -60,3 +60,39 @@ def test_whole_evaluations_are_timed(gpu):
     for h in (s, want):
         h.evolve(System.leapfrog_kdk)
     assert np.array_equal(s.x, want.x) and np.array_equal(s.v, want.v)
+
+
+def test_tuning_while_a_graph_is_captured(gpu):
+    """Another thread tunes the size class while the callback loop is being captured (a hook runs then): the
+    handle keeps the variant that the run began with, and the loop stays a graph."""
+    import threading
+
+    from gregpackagescpp_b200 import DeviceHook
+    n = 6000
+    small, large, s, want = (_system(k, "f64") for k in (4200, 8191, n, n))
+    first = _tune(large)
+    _lib.check(want._L.gtd_system_set_direct_variant(want._h, first))
+    seen = []
+
+    def tune():
+        # 4200 and 8191 bodies have other fastest variants; take turns until the choice differs
+        for h in (small, large, small):
+            seen.append(_tune(h))
+            if seen[-1] != first:
+                break
+
+    @C.CFUNCTYPE(C.c_int, C.c_void_p, C.c_void_p)
+    def hook(user, bodies):
+        if not seen:
+            t = threading.Thread(target=tune)
+            t.start()
+            t.join()
+        return 0
+
+    each = DeviceHook(C.cast(hook, C.c_void_p).value)
+    none = C.CFUNCTYPE(C.c_int, C.c_void_p, C.c_void_p)(lambda user, bodies: 0)
+    s.evolve(System.leapfrog_kdk, None, each, None)
+    assert seen and seen[-1] != first, (first, seen)
+    assert s.callback_stats()["graph_loop"]
+    want.evolve(System.leapfrog_kdk, None, DeviceHook(C.cast(none, C.c_void_p).value), None)
+    assert np.array_equal(s.x, want.x) and np.array_equal(s.v, want.v)
