@@ -24,6 +24,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cfloat>
 #include <type_traits>
 
 #include "direct_epilogue.cuh"
@@ -221,8 +222,9 @@ struct SymMixedSmem {
 // One chunk of 64 columns (32 packed pairs).  kSym: rows and columns, lane l on packed column
 // (l + s) mod 32 at step s.  Otherwise: rows alone, every lane on the same column.  The precise path
 // takes its differences from the hi/lo splits.  A vanishing separation (the self pair, coincident
-// bodies) is selected away wherever it can occur: on the ordered path and on the precise one.
-template <int I, int T, int U, int NH, bool kSym, bool kPrecise>
+// bodies) is selected away wherever it can occur: on the ordered path, on the precise one and (kGuard) in
+// the guarded chunks of the kernel without the close-pair check.
+template <int I, int T, int U, int NH, bool kSym, bool kPrecise, bool kGuard = kPrecise || !kSym>
 __device__ __forceinline__ void sym_mixed_chunk(const float4 *xy, const float4 *zm, const float2 *lx, const float2 *ly,
                                                 const float2 *lz, const float (*ilo)[I][T], const float2 (&nx)[I],
                                                 const float2 (&ny)[I], const float2 (&nz)[I], const float2 (&mi)[I],
@@ -268,7 +270,7 @@ __device__ __forceinline__ void sym_mixed_chunk(const float4 *xy, const float4 *
                 r2 = __ffma2_rn(dy, dy, r2);
                 r2 = __ffma2_rn(dz, dz, r2);
                 float2 inv = make_float2(rsqrt_approx(r2.x), rsqrt_approx(r2.y));
-                if (kPrecise || !kSym) {
+                if (kGuard) {
                     inv.x = r2.x > 0.f ? inv.x : 0.f;
                     inv.y = r2.y > 0.f ? inv.y : 0.f;
                 }
@@ -303,7 +305,14 @@ __device__ __forceinline__ void sym_mixed_chunk(const float4 *xy, const float4 *
     }
 }
 
-template <int I, int T, int TC, int MINB, int U, int NH, int FC>
+// Coincident bodies have to be selected away within the aligned runs of kGuarded bodies, as among the rows of
+// the widest ordered-pair kernel.  With the close-pair check (kCheck) a warp's threshold is at least FLT_MIN,
+// so that a chunk which meets its rows takes the precise path, which guards, also where all its rows lie
+// at the centre.  Without the check, an instance of its own guards the tiles of the rows' run: a guarded
+// fast path beside the precise one, or zeroed remainders there, cost every caller 2 % (N = 262144).
+constexpr int kGuarded = 1024;
+
+template <int I, int T, int TC, int MINB, int U, int NH, int FC, bool kCheck>
 __global__ void __launch_bounds__(T, MINB) force_mixed_sym_kernel(SymKArgs a) {
     using Smem = SymMixedSmem<I, T, TC, NH>;
     constexpr int kWarps = Smem::kWarps, kChunks = Smem::kChunks, kFetch = (TC + T - 1) / T;
@@ -401,7 +410,7 @@ __global__ void __launch_bounds__(T, MINB) force_mixed_sym_kernel(SymKArgs a) {
             const float v6 = warp_maxf(bth);
             if ((t & 31) == 0) {
                 float *b = S.ibox[warp];
-                b[0] = v0; b[1] = v1; b[2] = v2; b[3] = v3; b[4] = v4; b[5] = v5; b[6] = v6;
+                b[0] = v0; b[1] = v1; b[2] = v2; b[3] = v3; b[4] = v4; b[5] = v5; b[6] = fmaxf(v6, FLT_MIN);
             }
         }
         KahanAcc<I, true, T> acc;
@@ -470,13 +479,15 @@ __global__ void __launch_bounds__(T, MINB) force_mixed_sym_kernel(SymKArgs a) {
                     const float g = fmaxf(0.f, fmaxf(lo - iw[3 + d], iw[d] - hi));
                     g2 = fmaf(g, g, g2);
                 }
-                const bool precise = g2 < iw[6];
+                const bool precise = kCheck && g2 < iw[6];
                 const float4 *xy = S.xy[cur] + ch * 64, *zm = S.zm[cur] + ch * 64;
                 const float2 *lx = S.lx[cur] + ch * 32, *ly = S.ly[cur] + ch * 32, *lz = S.lz[cur] + ch * 32;
                 float *col = &S.col[cur][warp][0][0][ch * 64];
                 if (sym) {
                     if (precise)
                         sym_mixed_chunk<I, T, 2, NH, true, true>(xy, zm, lx, ly, lz, S.ilo, nx, ny, nz, mi, fx, fy, fz, col, TC);
+                    else if (!kCheck && jt < (row0 / kGuarded + 1) * (kGuarded / TC))
+                        sym_mixed_chunk<I, T, 2, NH, true, false, true>(xy, zm, lx, ly, lz, S.ilo, nx, ny, nz, mi, fx, fy, fz, col, TC);
                     else
                         sym_mixed_chunk<I, T, U, NH, true, false>(xy, zm, lx, ly, lz, S.ilo, nx, ny, nz, mi, fx, fy, fz, col, TC);
                 } else {
@@ -567,10 +578,13 @@ static const SymShape kSymMixed[] = {{4, 128, 128, 512, 0.3}, {4, 128, 64, 512, 
 SymShape sym_shape(int precision, int kind) { return precision == GTD_PREC_MIXED ? kSymMixed[kind] : kSymF64[kind]; }
 
 template <typename F>
-static void with_sym(int precision, int kind, F &&f) {
+static void with_sym(int precision, int kind, bool check, F &&f) {
     if (precision == GTD_PREC_MIXED) {
-        if (kind == 1) f(force_mixed_sym_kernel<4, 128, 64, 3, 8, 4, 64>, sizeof(SymMixedSmem<4, 128, 64, 4>));
-        else f(force_mixed_sym_kernel<4, 128, 128, 3, 4, 2, 128>, sizeof(SymMixedSmem<4, 128, 128, 2>));
+        constexpr size_t s1 = sizeof(SymMixedSmem<4, 128, 64, 4>), s0 = sizeof(SymMixedSmem<4, 128, 128, 2>);
+        if (kind == 1 && check) f(force_mixed_sym_kernel<4, 128, 64, 3, 8, 4, 64, true>, s1);
+        else if (kind == 1) f(force_mixed_sym_kernel<4, 128, 64, 3, 8, 4, 64, false>, s1);
+        else if (check) f(force_mixed_sym_kernel<4, 128, 128, 3, 4, 2, 128, true>, s0);
+        else f(force_mixed_sym_kernel<4, 128, 128, 3, 4, 2, 128, false>, s0);
     } else {
         if (kind == 1) f(force_f64_sym_kernel<4, 128, 128, 3>, (size_t)0);
         else f(force_f64_sym_kernel<4, 128, 64, 3>, (size_t)0);
@@ -582,7 +596,7 @@ size_t sym_partial_bytes(const ForcePlan &p) { return sym_layout(p.sg, p.sym_byt
 int sym_make_plan(ForcePlan &p, int precision, int kind, int sms) {
     const SymShape sh = sym_shape(precision, kind);
     int per_sm = 1;
-    with_sym(precision, kind, [&](auto k, size_t smem) {
+    with_sym(precision, kind, true, [&](auto k, size_t smem) {
         if (smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, sh.threads, smem);
     });
@@ -649,7 +663,7 @@ int sym_launch_force(int precision, const ForcePlan &p, const double4 *src, doub
         a.queue = reinterpret_cast<unsigned *>(mem) + batch;
         const int grid = (int)std::min<int64_t>(p.grid, a.unit1 - a.unit0);
         cudaError_t e = cudaSuccess;
-        with_sym(precision, p.sym_kind, [&](auto k, size_t smem) {
+        with_sym(precision, p.sym_kind, p.near2 > 0.f, [&](auto k, size_t smem) {
             if (smem > 48 * 1024) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
             if (e == cudaSuccess) launch_chained(chained, k, grid, sym_shape(precision, p.sym_kind).threads, smem, s, a);
         });
