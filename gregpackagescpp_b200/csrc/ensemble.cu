@@ -676,12 +676,12 @@ int ens_smem_bytes(int max_n) { return 4 * ens_stride(max_n) * (int)sizeof(float
 
 using namespace gtd;
 
-static std::vector<HostSpan> ens_spans(const gtd_ensemble *e, const double *m, const double *r, const double *rest,
-                                       const double *x3, const double *v3, const double *a3) {
-    std::vector<HostSpan> o;
+static HostSpans ens_spans(const gtd_ensemble *e, const double *m, const double *r, const double *rest, const double *x3,
+                           const double *v3, const double *a3) {
+    HostSpans o;
     const int64_t nb = e->n_bodies;
     auto add = [&](const double *host, int64_t at, int64_t words) {
-        if (host) o.push_back({const_cast<double *>(host), e->io + at * nb, sizeof(double) * (size_t)(words * nb)});
+        if (host) o.add(host, e->io + at * nb, sizeof(double) * (size_t)(words * nb));
     };
     add(x3, 0, 3);
     add(v3, 3, 3);

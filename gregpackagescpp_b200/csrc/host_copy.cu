@@ -11,57 +11,68 @@
 namespace gtd {
 
 constexpr size_t kSlotBytes = (size_t)512 << 10;
-constexpr int kThreadsMost = 8, kSlotsEach = 2;
+constexpr int kSlots = kRingThreads * kRingSlotsEach;
 constexpr size_t kRingFrom = (size_t)4 << 20;  // smaller copies: starting the threads costs what they save
 // Pinning the ring takes 3.7 ms and the threads save 0.15 ms a MB: a handle's ring is made once the large
 // copies of its life, this one included, come to what that pays for.
 constexpr size_t kRingPays = (size_t)40 << 20;
 
 void release_host_ring(HostRing &ring) {
-    for (cudaEvent_t e : ring.events) cudaEventDestroy(e);
-    ring.events.clear();
+    for (cudaEvent_t &e : ring.events) {
+        if (e) cudaEventDestroy(e);
+        e = nullptr;
+    }
     cudaFreeHost(ring.mem);
     ring.mem = nullptr;
 }
 
-static int ensure_ring(HostRing &ring) {
-    if (ring.mem) return GTD_OK;
-    constexpr int slots = kThreadsMost * kSlotsEach;
-    while ((int)ring.events.size() < slots) {
-        cudaEvent_t e;
-        GTD_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-        ring.events.push_back(e);
-    }
-    GTD_CUDA(cudaMallocHost(&ring.mem, slots * kSlotBytes));
-    return GTD_OK;
+// Whether the ring is there.  Where it cannot be made the copies go on through the driver, and the next
+// attempt waits for as many bytes again.
+static bool ensure_ring(HostRing &ring) {
+    if (ring.mem) return true;
+    bool ok = true;
+    for (cudaEvent_t &e : ring.events) ok = ok && (e || cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess);
+    ok = ok && cudaMallocHost(&ring.mem, kSlots * kSlotBytes) == cudaSuccess;
+    if (ok) return true;
+    cudaGetLastError();
+    ring.mem = nullptr;
+    ring.moved = 0;
+    return false;
 }
 
-// One thread's chunks (every `threads`-th), through its own slots.
-static cudaError_t copy_chunks(HostRing &ring, int device, cudaStream_t stream, const std::vector<HostSpan> &chunks,
+// One thread's chunks (every `threads`-th of the spans in ring_mask), through its own slots.
+static cudaError_t copy_chunks(HostRing &ring, int device, cudaStream_t stream, const HostSpans &spans, unsigned ring_mask,
                                int thread, int threads, bool to_host) {
     cudaError_t e = cudaSetDevice(device);
-    HostSpan held[kSlotsEach] = {};  // to_host: the chunk a slot is being filled with
+    HostSpan held[kRingSlotsEach] = {};  // the chunk a slot is in use for
     auto drain = [&](int s) {
         if (e != cudaSuccess || !held[s].bytes) return;
-        const int slot = thread * kSlotsEach + s;
-        e = cudaEventSynchronize(ring.events[(size_t)slot]);
+        const int slot = thread * kRingSlotsEach + s;
+        e = cudaEventSynchronize(ring.events[slot]);
         if (e == cudaSuccess && to_host) memcpy(held[s].host, ring.mem + slot * kSlotBytes, held[s].bytes);
         held[s].bytes = 0;
     };
-    int s = 0;
-    for (size_t k = (size_t)thread; k < chunks.size() && e == cudaSuccess; k += (size_t)threads, s = (s + 1) % kSlotsEach) {
-        drain(s);
-        if (e != cudaSuccess) break;
-        const HostSpan &c = chunks[k];
-        const int slot = thread * kSlotsEach + s;
-        char *pinned = ring.mem + slot * kSlotBytes;
-        if (!to_host) memcpy(pinned, c.host, c.bytes);
-        e = to_host ? cudaMemcpyAsync(pinned, c.dev, c.bytes, cudaMemcpyDeviceToHost, stream)
-                    : cudaMemcpyAsync(c.dev, pinned, c.bytes, cudaMemcpyHostToDevice, stream);
-        if (e == cudaSuccess) e = cudaEventRecord(ring.events[(size_t)slot], stream);
-        held[s] = c;
+    int s = 0, k = 0;
+    for (int a = 0; a < spans.count; ++a) {
+        if (!(ring_mask >> a & 1u)) continue;
+        const HostSpan &span = spans.span[a];
+        for (size_t at = 0; at < span.bytes && e == cudaSuccess; at += kSlotBytes, ++k) {
+            if (k % threads != thread) continue;
+            drain(s);
+            if (e != cudaSuccess) break;
+            const HostSpan c{static_cast<char *>(span.host) + at, static_cast<char *>(span.dev) + at,
+                             std::min(kSlotBytes, span.bytes - at)};
+            const int slot = thread * kRingSlotsEach + s;
+            char *pinned = ring.mem + slot * kSlotBytes;
+            if (!to_host) memcpy(pinned, c.host, c.bytes);
+            e = to_host ? cudaMemcpyAsync(pinned, c.dev, c.bytes, cudaMemcpyDeviceToHost, stream)
+                        : cudaMemcpyAsync(c.dev, pinned, c.bytes, cudaMemcpyHostToDevice, stream);
+            if (e == cudaSuccess) e = cudaEventRecord(ring.events[slot], stream);
+            held[s] = c;
+            s = (s + 1) % kRingSlotsEach;
+        }
     }
-    for (int q = 0; q < kSlotsEach; ++q) drain((s + q) % kSlotsEach);
+    for (int q = 0; q < kRingSlotsEach; ++q) drain((s + q) % kRingSlotsEach);
     return e;
 }
 
@@ -74,52 +85,53 @@ static bool pageable(const void *p) {
     return at.type == cudaMemoryTypeUnregistered;
 }
 
-static int copy_spans(HostRing &ring, int device, cudaStream_t stream, const std::vector<HostSpan> &spans, bool to_host) {
+static int copy_spans(HostRing &ring, int device, cudaStream_t stream, const HostSpans &spans, bool to_host) {
     size_t total = 0;
-    for (const HostSpan &s : spans) total += s.bytes;
+    for (int a = 0; a < spans.count; ++a) total += spans.span[a].bytes;
     const int cores = (int)std::thread::hardware_concurrency();
     if (total >= kRingFrom && ring.moved < kRingPays) ring.moved += total;
-    const bool threaded = total >= kRingFrom && cores >= 4 && ring.moved >= kRingPays;
-    std::vector<HostSpan> chunks;
-    std::vector<std::thread> pool;
-    for (const HostSpan &s : spans) {
-        if (!threaded || !pageable(s.host)) {
-            GTD_CUDA(to_host ? cudaMemcpyAsync(s.host, s.dev, s.bytes, cudaMemcpyDeviceToHost, stream)
-                             : cudaMemcpyAsync(s.dev, s.host, s.bytes, cudaMemcpyHostToDevice, stream));
-            continue;
-        }
-        for (size_t at = 0; at < s.bytes; at += kSlotBytes)
-            chunks.push_back({static_cast<char *>(s.host) + at, static_cast<char *>(s.dev) + at, std::min(kSlotBytes, s.bytes - at)});
+    unsigned ring_mask = 0;  // the spans that go through the ring
+    if (total >= kRingFrom && cores >= 4 && ring.moved >= kRingPays) {
+        for (int a = 0; a < spans.count; ++a)
+            if (spans.span[a].bytes && pageable(spans.span[a].host)) ring_mask |= 1u << a;
+        if (ring_mask && !ensure_ring(ring)) ring_mask = 0;
     }
-    if (!chunks.empty()) {
-        int rc = ensure_ring(ring);
-        if (rc) return rc;
-        const int threads = std::min(kThreadsMost, cores / 2);
+    for (int a = 0; a < spans.count; ++a) {
+        const HostSpan &s = spans.span[a];
+        if (ring_mask >> a & 1u) continue;
+        GTD_CUDA(to_host ? cudaMemcpyAsync(s.host, s.dev, s.bytes, cudaMemcpyDeviceToHost, stream)
+                         : cudaMemcpyAsync(s.dev, s.host, s.bytes, cudaMemcpyHostToDevice, stream));
+    }
+    if (ring_mask) {
+        const int threads = std::min(kRingThreads, cores / 2);
         std::atomic<int> error{cudaSuccess};
         auto work = [&](int t) {
-            const cudaError_t e = copy_chunks(ring, device, stream, chunks, t, threads, to_host);
+            const cudaError_t e = copy_chunks(ring, device, stream, spans, ring_mask, t, threads, to_host);
             if (e != cudaSuccess) error.store((int)e);
         };
-        pool.reserve((size_t)threads);
+        std::thread pool[kRingThreads];
         int started = 1;  // this thread takes part 0
         try {
-            for (; started < threads; ++started) pool.emplace_back(work, started);
+            for (; started < threads; ++started) pool[started] = std::thread(work, started);
         } catch (...) {  // no more threads: their parts are done here
         }
         work(0);
         for (int t = started; t < threads; ++t) work(t);
-        for (std::thread &t : pool) t.join();
-        GTD_CUDA((cudaError_t)error.load());
+        for (int t = 1; t < started; ++t) pool[t].join();
+        if (error.load() != cudaSuccess) {
+            cudaStreamSynchronize(stream);  // nothing is left in the slots
+            GTD_CUDA((cudaError_t)error.load());
+        }
     }
     if (to_host) GTD_CUDA(cudaStreamSynchronize(stream));
     return GTD_OK;
 }
 
-int copy_to_host(HostRing &ring, int device, cudaStream_t stream, const std::vector<HostSpan> &spans) {
+int copy_to_host(HostRing &ring, int device, cudaStream_t stream, const HostSpans &spans) {
     return copy_spans(ring, device, stream, spans, true);
 }
 
-int copy_to_device(HostRing &ring, int device, cudaStream_t stream, const std::vector<HostSpan> &spans) {
+int copy_to_device(HostRing &ring, int device, cudaStream_t stream, const HostSpans &spans) {
     return copy_spans(ring, device, stream, spans, false);
 }
 

@@ -36,19 +36,16 @@ static IoView io_view(double *base, int64_t n) {
 }
 
 // The caller's arrays beside their staging areas (NULL: not given).
-static std::vector<HostSpan> io_spans(const IoView &io, int64_t n, const double *m, const double *r, const double *rest,
-                                      const double *x3, const double *v3, const double *a3) {
-    std::vector<HostSpan> o;
+static HostSpans io_spans(const IoView &io, int64_t n, const double *m, const double *r, const double *rest, const double *x3,
+                          const double *v3, const double *a3) {
+    HostSpans o;
     const size_t b = sizeof(double) * (size_t)n;
-    auto add = [&](const double *host, double *dev, size_t bytes) {
-        if (host) o.push_back({const_cast<double *>(host), dev, bytes});
-    };
-    add(x3, io.x3, 3 * b);
-    add(v3, io.v3, 3 * b);
-    add(a3, io.a3, 3 * b);
-    add(m, io.m, b);
-    add(r, io.r, b);
-    add(rest, io.rest, b);
+    if (x3) o.add(x3, io.x3, 3 * b);
+    if (v3) o.add(v3, io.v3, 3 * b);
+    if (a3) o.add(a3, io.a3, 3 * b);
+    if (m) o.add(m, io.m, b);
+    if (r) o.add(r, io.r, b);
+    if (rest) o.add(rest, io.rest, b);
     return o;
 }
 
