@@ -13,9 +13,10 @@ namespace gtd {
 constexpr size_t kSlotBytes = (size_t)512 << 10;
 constexpr int kSlots = kRingThreads * kRingSlotsEach;
 constexpr size_t kRingFrom = (size_t)4 << 20;  // smaller copies: starting the threads costs what they save
-// Pinning the ring takes 3.7 ms and the threads save 0.15 ms a MB: a handle's ring is made once the large
-// copies of its life, this one included, come to what that pays for.
-constexpr size_t kRingPays = (size_t)40 << 20;
+// Making the ring takes 4 to 7 ms, and its threads save 0.05 ms a MB of arrays in use and 0.14 of fresh ones
+// (two GPU hosts): what it costs comes back after 50 to 140 MB.  A handle's ring is made once the large
+// copies of its life, this one included, come to about that.
+constexpr size_t kRingPays = (size_t)64 << 20;
 
 void release_host_ring(HostRing &ring) {
     for (cudaEvent_t &e : ring.events) {
