@@ -248,7 +248,7 @@ struct VjpUpdate {
 // Small systems: VJP and update in one launch, as fused_small_kernel (direct.cu) does force and step.
 // kVjpSlices warps share a body, their lanes take the ordered pairs of every 32 kVjpSlices-th partner
 // straight from L1 / L2, and the body's first warp adds the slices in order.  Chained launches: a reverse
-// step of 1000 bodies 8.8 -> 8.1 us, of 2000 16.9 -> 15.2, and with warp_sums 14.8.
+// step of 1000 bodies 8.8 -> 8.1 us (7.2 with two bodies per warp), of 2000 16.9 -> 15.2, with warp_sums 14.8.
 constexpr int kVjpSlices = 4;
 
 template <int I, int GROUPS, int MINB>
@@ -484,8 +484,10 @@ static int adj_vjp(gtd_adjoint *A, const double4 *x, uint64_t k, int &cur, cudaS
     const double4 *w = A->w[cur];
     cur ^= 1;
     if (A->small_vjp) {
-        // bodies per warp, groups per CTA and CTAs per SM as in launch_fused_small
-        if (A->n <= 1000) launch_vjp_small<1, 1, 8>(A->n, x, w, up, st);
+        // bodies per warp, CTAs per SM and the sizes where they change as in launch_fused_small, up to two
+        // bodies.  Us a step both ways with one body per warp and two: 500 bodies 7.49 / 7.82, 592 8.45 /
+        // 8.43, 700 9.14 / 9.18, 800 10.0 / 9.28, 1000 11.8 / 10.9, 1184 13.3 / 13.0, 1480 21.1 / 15.2
+        if (A->n <= 592) launch_vjp_small<1, 1, 8>(A->n, x, w, up, st);
         else if (A->n <= 5 * 148 * 2) launch_vjp_small<2, 1, 5>(A->n, x, w, up, st);
         else launch_vjp_small<2, 1, 4>(A->n, x, w, up, st);
         GTD_CHECK_LAUNCH();
