@@ -1056,12 +1056,14 @@ int enqueue_paired_open(gtd_system *s, const PassHooks &hk) {
     return GTD_OK;
 }
 
-// Two bodies per block from the size where they pay in the fused force kernel.
+// One body per block as far as the blocks fit the GPU at once, 8 on each of 148 SMs; two above.  Us a step
+// with one and with two: 592 bodies 10.8 / 10.9, 727 11.3 / 11.6, 900 13.7 / 14.2, 1000 13.9 / 14.4, 1184
+// 13.84 / 13.85, 1250 16.9 / 14.3, 1480 20.2 / 17.2.
 int enqueue_paired_step(gtd_system *s, int at, const PassHooks &hk, bool closes) {
     CollPtrs p = coll_ptrs(s);
     cudaStream_t st = s->stream;
     double4 *x = s->pm[at], *dst = s->pm[at ^ 1];
-    const int I = s->n <= 900 ? 1 : 2;
+    const int I = s->n <= 8 * 148 ? 1 : 2;
     auto *f = I == 1 ? paired_force_kernel<1> : paired_force_kernel<2>;
     f<<<(unsigned)((s->n + I - 1) / I), (kPairSlices + (hk.for_all ? 1 : 0)) * 32, 0, st>>>(
         s->n, x, dst, s->rad, s->G, s->dt, s->vel, s->acc, s->rest, p.cand, p.count, kMaxCand, hk);
