@@ -444,15 +444,12 @@ int variant_count(int precision) { return precision == GTD_PREC_MIXED ? kNumMixe
 // Variant for a handle nobody tuned: the unordered-pair kernels (direct_sym.cu), per step on B200
 //   mixed   N = 8192 58 us (ordered pairs 75), 16384 160 (192), 65536 1.58 ms (2.32), 262144 21.8 ms (29.3)
 //   FP64    N = 5000 35 us (41), 8192 65 (92), 16384 212 (295), 65536 2.95 ms (4.33)
-// Systems of up to kFusedAutoMaxN bodies take the fused kernel instead; where one was tuned, or for FP64
-// handles' plans, up to 17 rows and tiles of 256 bodies, the 289 ordered tiles all run at once, one per CTA:
-// N = 4200 29 us against 35.
+// Systems of up to kFusedAutoMaxN bodies take the fused kernel instead.
 // From N = 32768 the mixed kernel folds its FP32 sums half as often: 3 % faster, and its rounding
 // (RMS 3.8e-8 of a body's acceleration at N = 262144 against 3.2e-8) is still that of the ordered
 // kernel's fold of 128 (4.0e-8).
 int default_variant(int precision, int64_t n) {
     if (precision == GTD_PREC_MIXED) return n >= 32768 ? 9 : 10;
-    if (n <= 17 * 256) return 1;
     return n <= 32768 ? 5 : 6;
 }
 
@@ -573,27 +570,6 @@ static size_t queue_offset(const ForcePlan &p) {
 size_t partial_bytes(const ForcePlan &p) {
     if (p.sym) return sym_partial_bytes(p);
     return queue_offset(p) + (p.segs > 0 ? 256 : 0);
-}
-
-int fit_plan_partials(ForcePlan &p, size_t max_bytes) {
-    if (p.sym) return sym_fit(p, max_bytes);
-    if (partial_bytes(p) <= max_bytes) return GTD_OK;
-    const size_t per_slot = (size_t)3 * p.bi * sizeof(double);
-    const int64_t max_slots = max_bytes > 512 ? (int64_t)((max_bytes - 512) / per_slot) : 0;
-    if (p.segs > 0) {
-        const int64_t segs = max_slots / std::max<int64_t>(p.rows, 1);
-        if (segs < 1) return fail(GTD_ERR_CAPACITY, "%lld rows need more partial sums than %zu bytes hold",
-                                  (long long)p.rows, max_bytes);
-        set_segments(p, segs);
-        if (p.grid > p.units) p.grid = (int)p.units;
-    } else {
-        const int64_t grid = max_slots - p.rows;
-        if (grid < 1) return fail(GTD_ERR_CAPACITY, "%lld rows need more partial sums than %zu bytes hold",
-                                  (long long)p.rows, max_bytes);
-        if (p.grid > grid) p.grid = (int)grid;
-        p.slots = p.grid + p.rows;
-    }
-    return partial_bytes(p) <= max_bytes ? GTD_OK : fail(GTD_ERR_CAPACITY, "partial sums do not fit %zu bytes", max_bytes);
 }
 
 int launch_force(int precision, const ForcePlan &p, const double4 *src, double G, double *partials,
@@ -838,35 +814,6 @@ int launch_integrate(const ForcePlan &p, const double *partials, int epi, const 
         integrate_warp_kernel<<<(unsigned)((p.n * 32 + threads - 1) / threads), threads, 0, s>>>(a);
     else
         integrate_kernel<<<(unsigned)((p.n + threads - 1) / threads), threads, 0, s>>>(a);
-    GTD_CHECK_LAUNCH();
-    return GTD_OK;
-}
-
-// Thread per body: the summed partials written as a triple (the force alone).
-__global__ void sum_partials_kernel(IntArgs a, double *acc3) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.n) return;
-    const int64_t r = i / a.bi;
-    const int l = (int)(i - r * a.bi);
-    int64_t g0, g1;
-    row_slots(a, r, g0, g1);
-    double ax = 0.0, ay = 0.0, az = 0.0;
-    for (int64_t g = g0; g <= g1; ++g) {
-        const double *slot = a.part + (size_t)g * 3 * a.bi;
-        ax += slot[l];
-        ay += slot[a.bi + l];
-        az += slot[2 * a.bi + l];
-    }
-    acc3[3 * i] = ax;
-    acc3[3 * i + 1] = ay;
-    acc3[3 * i + 2] = az;
-}
-
-int launch_sum_partials(const ForcePlan &p, const double *partials, double *acc3, cudaStream_t s) {
-    if (p.n == 0) return GTD_OK;
-    if (p.sym) return sym_launch_finish(p, partials, EPI_ACC, StepArgs{}, acc3, false, s);
-    IntArgs a{p.n, p.tiles, p.total, p.grid, p.bi, EPI_ACC, partials, StepArgs{}, p.segs};
-    sum_partials_kernel<<<(unsigned)((p.n + 255) / 256), 256, 0, s>>>(a, acc3);
     GTD_CHECK_LAUNCH();
     return GTD_OK;
 }

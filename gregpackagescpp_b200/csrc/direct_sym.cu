@@ -616,6 +616,8 @@ int sym_make_plan(ForcePlan &p, int precision, int kind, int sms) {
     return GTD_OK;
 }
 
+// Shrinks the plan's partial sums to at most max_bytes (more and smaller batches); GTD_ERR_CAPACITY where
+// even one super-group a batch does not fit.
 int sym_fit(ForcePlan &p, size_t max_bytes) {
     SymGeom &g = p.sg;
     // fewer row slots where that saves a batch and leaves some units per CTA

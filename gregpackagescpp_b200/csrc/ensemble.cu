@@ -54,14 +54,13 @@ struct gtd_ensemble {
     double4 *pos = nullptr, *vel = nullptr, *acc = nullptr;
     double *rad = nullptr, *rest = nullptr;
     int32_t *ids = nullptr;
-    unsigned *work = nullptr;         // [2]: unused, merges so far
+    unsigned *merged = nullptr;       // merges so far
     gtd::EnsCand *cand = nullptr;     // [n_sys] rows the separation test flagged
     gtd::EnsInfo *info = nullptr;     // [n_sys] frame of the staged coordinates
     int *arrived = nullptr;           // [n_sys] chunks finished in this launch
     int2 *items = nullptr;            // (system, first row), largest system first
     int64_t n_items = 0;
     int items_for = 0;                // the (threads, ib) the items were made for
-    int *status = nullptr;
     double *io = nullptr;             // host arrays on the device: x3 | v3 | a3 | m | r | rest
     gtd::HostRing host_ring;
     bool begun = false;
@@ -108,7 +107,7 @@ struct EnsArgs {
     int merge;
     int chunk;   // rows per item
     int stride;  // floats per staged coordinate array (largest system, rounded up to even)
-    unsigned *work;
+    unsigned *merged;
 };
 
 __device__ __forceinline__ float ens_rsqrt(float x) {
@@ -617,7 +616,7 @@ __global__ void __launch_bounds__(IB == 1 ? 512 : 256) ensemble_step_kernel(EnsA
         if (left != n) {
             if (t == 0) {
                 a.cnt[s] = left;
-                atomicAdd(&a.work[1], (unsigned)(n - left));
+                atomicAdd(a.merged, (unsigned)(n - left));
             }
             n = left;
             // the force at the merged state, so the next step's first half kick uses a(x) of the bodies
@@ -702,14 +701,14 @@ static void ens_release(gtd_ensemble *e) {
     cudaFree(e->io);
     e->io = nullptr;
     cudaFree(e->off); cudaFree(e->cnt); cudaFree(e->order); cudaFree(e->pos); cudaFree(e->vel); cudaFree(e->acc);
-    cudaFree(e->rad); cudaFree(e->rest); cudaFree(e->ids); cudaFree(e->work); cudaFree(e->status);
+    cudaFree(e->rad); cudaFree(e->rest); cudaFree(e->ids); cudaFree(e->merged);
     e->off = nullptr; e->cnt = nullptr; e->order = nullptr; e->pos = e->vel = e->acc = nullptr;
-    e->rad = e->rest = nullptr; e->ids = nullptr; e->work = nullptr; e->status = nullptr;
+    e->rad = e->rest = nullptr; e->ids = nullptr; e->merged = nullptr;
 }
 
 static EnsArgs ens_args(const gtd_ensemble *e, int kick, int pre) {
     return EnsArgs{e->off, e->cnt, e->order, e->items, e->pos, e->vel, e->acc, e->rad, e->rest, e->ids, e->cand, e->info,
-                   e->arrived, e->G, e->dt, kick, pre, e->merge, e->threads * e->ib, ens_stride(e->max_n), e->work};
+                   e->arrived, e->G, e->dt, kick, pre, e->merge, e->threads * e->ib, ens_stride(e->max_n), e->merged};
 }
 
 static void ens_release_graph(gtd_ensemble *e) {
@@ -913,8 +912,7 @@ int gtd_ensemble_upload(gtd_ensemble *e, int64_t n_systems, const int64_t *offse
     GTD_CUDA(cudaMalloc(&e->rad, sizeof(double) * (size_t)std::max<int64_t>(nb, 1)));
     GTD_CUDA(cudaMalloc(&e->rest, sizeof(double) * (size_t)std::max<int64_t>(nb, 1)));
     GTD_CUDA(cudaMalloc(&e->ids, sizeof(int32_t) * (size_t)std::max<int64_t>(nb, 1)));
-    GTD_CUDA(cudaMalloc(&e->work, 4 * sizeof(unsigned)));
-    GTD_CUDA(cudaMalloc(&e->status, sizeof(int)));
+    GTD_CUDA(cudaMalloc(&e->merged, sizeof(unsigned)));
     const size_t ns = (size_t)std::max<int64_t>(n_systems, 1);
     GTD_CUDA(cudaMalloc(&e->cand, sizeof(EnsCand) * ns));
     GTD_CUDA(cudaMalloc(&e->info, sizeof(EnsInfo) * ns));
@@ -943,8 +941,7 @@ int gtd_ensemble_upload(gtd_ensemble *e, int64_t n_systems, const int64_t *offse
             GTD_CUDA(cudaMemsetAsync(e->rest, 0, sizeof(double) * (size_t)first, st));
         }
     }
-    GTD_CUDA(cudaMemsetAsync(e->work, 0, 4 * sizeof(unsigned), st));
-    GTD_CUDA(cudaMemsetAsync(e->status, 0, sizeof(int), st));
+    GTD_CUDA(cudaMemsetAsync(e->merged, 0, sizeof(unsigned), st));
     GTD_CUDA(cudaStreamSynchronize(st));
     e->begun = false;
     if (!e->configured) ens_default(e);
@@ -977,9 +974,9 @@ int gtd_ensemble_counts(gtd_ensemble *e, int64_t *counts, uint64_t *merges, uint
         for (int64_t s = 0; s < e->n_sys; ++s) counts[s] = c[(size_t)s];
     }
     if (merges) {
-        unsigned w[2] = {0, 0};
-        GTD_CUDA(cudaMemcpy(w, e->work, sizeof(w), cudaMemcpyDeviceToHost));
-        *merges = w[1];
+        unsigned w = 0;
+        GTD_CUDA(cudaMemcpy(&w, e->merged, sizeof w, cudaMemcpyDeviceToHost));
+        *merges = w;
     }
     if (launches) *launches = e->launches;
     return GTD_OK;
@@ -1112,7 +1109,7 @@ int gtd_ensemble_autotune(gtd_ensemble *e, int *best_threads, double *best_ms) {
     e->configured = true;
     e->begun = was_begun;
     GTD_CUDA(cudaStreamSynchronize(e->stream));
-    GTD_CUDA(cudaMemset(e->work, 0, 4 * sizeof(unsigned)));
+    GTD_CUDA(cudaMemset(e->merged, 0, sizeof(unsigned)));
     if (best_threads) *best_threads = best;
     if (best_ms) *best_ms = bestv;
     return GTD_OK;

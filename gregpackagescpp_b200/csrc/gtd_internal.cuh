@@ -135,11 +135,6 @@ int launch_fused_small(int64_t n, const double4 *src, double G, int epi, const S
 void remember_variant(int device, int precision, int64_t n, int variant);
 int tuned_variant(int device, int precision, int64_t n);
 size_t partial_bytes(const ForcePlan &p);
-// Shrinks the plan's partial-sum footprint to at most max_bytes (fewer queue segments, or a smaller
-// stream-K grid); GTD_ERR_CAPACITY when even the smallest split does not fit.
-int fit_plan_partials(ForcePlan &p, size_t max_bytes);
-// acc3[3 i + d] = the summed partials of body i (the force alone, in the bodies' order).
-int launch_sum_partials(const ForcePlan &p, const double *partials, double *acc3, cudaStream_t s);
 // Force on every body of `src` (positions + G-free masses), written as partial sums.  chained: as in
 // launch_chained, for unordered-pair plans.
 int launch_force(int precision, const ForcePlan &p, const double4 *src, double G, double *partials,

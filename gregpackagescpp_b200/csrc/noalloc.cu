@@ -102,10 +102,9 @@ extern "C" int gtd_direct_accelerations_noalloc(int64_t n, const double *pm4, do
     if (rc) return rc;
     // the force is evaluated in as many batches as its partial sums need to fit the fixed scratch
     ForcePlan p = make_plan(n, precision, dev, noalloc_variant(precision, n));
-    rc = fit_plan_partials(p, kNoAllocScratchBytes);
-    if (rc) return rc;
-    if (p.sym && (rc = sym_reset(p, static_cast<double *>(scratch), st))) return rc;
-    rc = launch_force(precision, p, reinterpret_cast<const double4 *>(pm4), G, static_cast<double *>(scratch), st);
-    if (rc) return rc;
-    return launch_sum_partials(p, static_cast<const double *>(scratch), acc3, st);
+    double *partials = static_cast<double *>(scratch);
+    rc = sym_fit(p, kNoAllocScratchBytes);
+    if (!rc) rc = sym_reset(p, partials, st);
+    if (!rc) rc = launch_force(precision, p, reinterpret_cast<const double4 *>(pm4), G, partials, st);
+    return rc ? rc : sym_launch_finish(p, partials, EPI_ACC, StepArgs{}, acc3, false, st);
 }

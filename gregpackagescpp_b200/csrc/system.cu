@@ -786,10 +786,16 @@ int gtd_system_direct_plan_info(gtd_system *s, int64_t *units, int64_t *partial_
     if (!s) return fail(GTD_ERR_INVALID_ARGUMENT, "system is NULL");
     if (s->n == 0) return fail(GTD_ERR_INVALID_ARGUMENT, "no bodies");
     DeviceGuard g(s->device);
-    int rc = ensure_plan(s);
-    if (rc) return rc;
-    if (units) *units = s->plan.units > 0 ? s->plan.units : s->plan.total;
-    if (partial_bytes_out) *partial_bytes_out = (int64_t)partial_bytes(s->plan);
+    ForcePlan p;
+    if (fused_force(s)) {
+        p = make_plan(s->n, s->precision, s->device, tuned_variant(s->device, s->precision, s->n));
+    } else {
+        const int rc = ensure_plan(s);
+        if (rc) return rc;
+        p = s->plan;
+    }
+    if (units) *units = p.units > 0 ? p.units : p.total;
+    if (partial_bytes_out) *partial_bytes_out = (int64_t)partial_bytes(p);
     return GTD_OK;
 }
 

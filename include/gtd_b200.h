@@ -283,7 +283,7 @@ GTD_API int gtd_system_set_mixed_near_factor(gtd_system *sys, double k);
  * one force evaluation (row blocks against runs of columns, taken from a work queue; (row, tile)
  * pairs for the ordered FP64 variants) and the bytes of partial sums they write.  Handles of up to
  * 4736 bodies whose variant is not pinned (FP64: up to 4096 in any case) run one launch
- * without either; the numbers are then the variant's. */
+ * without either; the numbers are then those of the variant it would take. */
 GTD_API int gtd_system_direct_plan_info(gtd_system *sys, int64_t *units, int64_t *partial_bytes);
 /* Measured throughput of a dependent-FMA microkernel on `device` (all SMs): precision
  * GTD_PREC_MIXED gives FP32 FFMA FLOP/s, GTD_PREC_F64 gives FP64 DFMA FLOP/s (2 flops per FMA). */
