@@ -14,10 +14,10 @@
 // system's mean position, with G m; its rows are spread over the threads, IB (1, 2 or 4) each,
 // and each thread sums its rows' forces two j-bodies per packed FP32x2 instruction, folding every
 // 64 j-bodies into FP64.  Alongside the force it keeps the smallest separation to any other body (a
-// 3-input float minimum; the one fold holding the row's own body excludes the self pair by its bit
-// pattern); a body closer to another than its radius plus the system's largest radius, plus a
-// bound on the FP32 staging error, flags the row; only systems with flagged rows run the exact FP64
-// merge scan, over those rows.
+// 3-input float minimum; in the one fold holding the row's own body its j pair is left out by number, not
+// by its value, which coincident bodies share); a body closer to another than its radius plus the system's
+// largest radius, plus a bound on the FP32 staging error, flags the row; only systems with flagged rows run
+// the exact FP64 merge scan, over those rows.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -338,15 +338,14 @@ __device__ __forceinline__ float ens_min3(float a, float b, float c) {
     return d;
 }
 
-// One fold (j pairs q0 .. q1-1) of the force loop for IB rows.  kOwn: the fold holds one of the
-// rows' own bodies, whose self pair (r2 = floor2 exactly) must stay out of the minimum: the
-// separation minimum is then taken on the integer bits offset past floor2 (2 ALU operations per
-// value); every other fold takes a plain 3-input float minimum (1 operation per two values).
+// One fold (j pairs q0 .. q1-1) of the force loop for IB rows, with the smallest r2 to another body.  kOwn:
+// the fold holds one of the rows' own bodies, whose j pair oq[b] stays out of the minimum (its other body is
+// in it from the start).
 template <int IB, bool kOwn>
 __device__ __forceinline__ void ens_fold(int q0, int q1, const float2 *X2, const float2 *Y2, const float2 *Z2,
                                          const float2 *M2, const float2 (&nx)[IB], const float2 (&ny)[IB],
-                                         const float2 (&nz)[IB], float2 fl2, unsigned fbits, float2 (&fx)[IB],
-                                         float2 (&fy)[IB], float2 (&fz)[IB], float (&mnf)[IB], unsigned (&mnr)[IB]) {
+                                         const float2 (&nz)[IB], float2 fl2, const int (&oq)[IB],
+                                         float2 (&fx)[IB], float2 (&fy)[IB], float2 (&fz)[IB], float (&mn)[IB]) {
 #pragma unroll 4
     for (int q = q0; q < q1; ++q) {
         const float2 X = X2[q], Y = Y2[q], Z = Z2[q], M = M2[q];
@@ -356,12 +355,7 @@ __device__ __forceinline__ void ens_fold(int q0, int q1, const float2 *X2, const
             float2 r2 = __ffma2_rn(dx, dx, fl2);
             r2 = __ffma2_rn(dy, dy, r2);
             r2 = __ffma2_rn(dz, dz, r2);
-            if constexpr (kOwn) {
-                mnr[b] = min(mnr[b], (unsigned)__float_as_int(r2.x) - fbits);
-                mnr[b] = min(mnr[b], (unsigned)__float_as_int(r2.y) - fbits);
-            } else {
-                mnf[b] = ens_min3(mnf[b], r2.x, r2.y);
-            }
+            if (!kOwn || q != oq[b]) mn[b] = ens_min3(mn[b], r2.x, r2.y);
             const float2 inv = make_float2(ens_rsqrt(r2.x), ens_rsqrt(r2.y));
             const float2 inv2 = __fmul2_rn(inv, inv);
             float2 sc = __fmul2_rn(M, inv);
@@ -391,9 +385,9 @@ __device__ __forceinline__ int ens_force_rows(int r0, int s, int nc, int npad, c
     const float2 *M2 = reinterpret_cast<const float2 *>(sm);
     float2 nx[IB], ny[IB], nz[IB];
     double ax[IB], ay[IB], az[IB];
-    float mnf[IB];      // min r2 over the folds without the row's own body
-    unsigned mnr[IB];   // min over the own fold's j != i of r2 bits, offset past floor2
-    int own[IB];        // fold of the row's own body
+    float mn[IB];             // smallest r2 to another body
+    int own[IB];              // fold of the row's own body
+    int oq[IB];               // its j pair
 #pragma unroll
     for (int b = 0; b < IB; ++b) {
         const int ic = ens_staged_row(r0 + b * s, r0, nc);
@@ -401,12 +395,12 @@ __device__ __forceinline__ int ens_force_rows(int r0, int s, int nc, int npad, c
         ny[b] = make_float2(-sy[ic], -sy[ic]);
         nz[b] = make_float2(-sz[ic], -sz[ic]);
         ax[b] = ay[b] = az[b] = 0.0;
-        mnf[b] = INFINITY;
-        mnr[b] = 0xffffffffu;
+        const float dx = sx[ic ^ 1] + nx[b].x, dy = sy[ic ^ 1] + ny[b].x, dz = sz[ic ^ 1] + nz[b].x;
+        mn[b] = fmaf(dz, dz, fmaf(dy, dy, fmaf(dx, dx, floor2)));  // padding: infinite
+        oq[b] = ic >> 1;
         own[b] = ens_stand_in(r0 + b * s, r0, nc) / kEnsFold;
     }
     const float2 fl2 = make_float2(floor2, floor2);
-    const unsigned fbits = (unsigned)__float_as_int(floor2) + 1u;
     for (int q0 = 0; q0 < npad / 2; q0 += kEnsFold / 2) {
         const int q1 = min(q0 + kEnsFold / 2, npad / 2);
         const int fold = q0 / (kEnsFold / 2);
@@ -417,9 +411,9 @@ __device__ __forceinline__ int ens_force_rows(int r0, int s, int nc, int npad, c
 #pragma unroll
         for (int b = 0; b < IB; ++b) mine |= own[b] == fold;
         if (__any_sync(0xffffffffu, mine))
-            ens_fold<IB, true>(q0, q1, X2, Y2, Z2, M2, nx, ny, nz, fl2, fbits, fx, fy, fz, mnf, mnr);
+            ens_fold<IB, true>(q0, q1, X2, Y2, Z2, M2, nx, ny, nz, fl2, oq, fx, fy, fz, mn);
         else
-            ens_fold<IB, false>(q0, q1, X2, Y2, Z2, M2, nx, ny, nz, fl2, fbits, fx, fy, fz, mnf, mnr);
+            ens_fold<IB, false>(q0, q1, X2, Y2, Z2, M2, nx, ny, nz, fl2, oq, fx, fy, fz, mn);
 #pragma unroll
         for (int b = 0; b < IB; ++b) {
             ax[b] += (double)fx[b].x + (double)fx[b].y;
@@ -432,8 +426,7 @@ __device__ __forceinline__ int ens_force_rows(int r0, int s, int nc, int npad, c
     for (int b = 0; b < IB; ++b) {
         const int i = r0 + b * s;
         if (i >= nc) continue;
-        float mind2 = mnf[b];
-        if (mnr[b] != 0xffffffffu) mind2 = fminf(mind2, __int_as_float((int)(mnr[b] + fbits)));
+        const float mind2 = mn[b];
         if (mind2 < INFINITY) {  // some other body exists
             const float reach = ((float)rad[i] + rmx) * 1.00001f + slack;
             if (mind2 < reach * reach * 1.0001f + floor2) {
