@@ -815,6 +815,9 @@ static int ens_steps(gtd_ensemble *e, uint64_t steps) {
     return GTD_OK;
 }
 
+static int ens_upload(gtd_ensemble *e, int64_t n_systems, const int64_t *offsets, const double *m, const double *r,
+                      const double *rest, const double *x3, const double *v3);
+
 extern "C" {
 
 int gtd_ensemble_create(gtd_ensemble **out, int device) {
@@ -874,71 +877,18 @@ int gtd_ensemble_upload(gtd_ensemble *e, int64_t n_systems, const int64_t *offse
         return fail(GTD_ERR_INVALID_ARGUMENT, "bad ensemble description");
     cudaSetDevice(e->device);
     ens_release(e);
-    e->n_sys = n_systems;
-    e->off_h.assign(offsets, offsets + n_systems + 1);
-    const int64_t nb = n_systems ? offsets[n_systems] : 0;
-    e->n_bodies = nb;
-    e->max_n = 0;
-    std::vector<int32_t> cnt((size_t)n_systems);
-    std::vector<int32_t> &order = e->order_h;
-    order.assign((size_t)n_systems, 0);
-    for (int64_t s = 0; s < n_systems; ++s) {
-        const int64_t k = offsets[s + 1] - offsets[s];
-        if (k < 0 || offsets[s] < 0) return fail(GTD_ERR_INVALID_ARGUMENT, "offsets must be non-decreasing from 0");
-        if (k > kEnsMaxN) return fail(GTD_ERR_CAPACITY, "system %lld has %lld bodies; the ensemble kernel holds %d",
-                                      (long long)s, (long long)k, kEnsMaxN);
-        cnt[(size_t)s] = (int32_t)k;
-        e->max_n = std::max(e->max_n, (int)k);
+    int rc;
+    try {
+        rc = ens_upload(e, n_systems, offsets, m, r, rest, x3, v3);
+    } catch (const std::bad_alloc &) {
+        rc = fail(GTD_ERR_OUT_OF_MEMORY, "host allocation failed");
     }
-    std::iota(order.begin(), order.end(), 0);
-    std::stable_sort(order.begin(), order.end(), [&](int32_t a, int32_t b) { return cnt[a] > cnt[b]; });
-    const int64_t first = n_systems ? offsets[0] : 0;  // rows before it belong to no system and read as zero
-    for (int64_t i = first; i < nb; ++i)
-        if (m[i] < 0) return fail(GTD_ERR_INVALID_ARGUMENT, "negative mass at body %lld", (long long)i);
-    const size_t b4 = sizeof(double4) * (size_t)std::max<int64_t>(nb, 1);
-    GTD_CUDA(cudaMalloc(&e->off, sizeof(int64_t) * (size_t)(n_systems + 1)));
-    GTD_CUDA(cudaMalloc(&e->cnt, sizeof(int32_t) * (size_t)std::max<int64_t>(n_systems, 1)));
-    GTD_CUDA(cudaMalloc(&e->order, sizeof(int32_t) * (size_t)std::max<int64_t>(n_systems, 1)));
-    GTD_CUDA(cudaMalloc(&e->pos, b4));
-    GTD_CUDA(cudaMalloc(&e->vel, b4));
-    GTD_CUDA(cudaMalloc(&e->acc, b4));
-    GTD_CUDA(cudaMalloc(&e->rad, sizeof(double) * (size_t)std::max<int64_t>(nb, 1)));
-    GTD_CUDA(cudaMalloc(&e->rest, sizeof(double) * (size_t)std::max<int64_t>(nb, 1)));
-    GTD_CUDA(cudaMalloc(&e->ids, sizeof(int32_t) * (size_t)std::max<int64_t>(nb, 1)));
-    GTD_CUDA(cudaMalloc(&e->merged, sizeof(unsigned)));
-    const size_t ns = (size_t)std::max<int64_t>(n_systems, 1);
-    GTD_CUDA(cudaMalloc(&e->cand, sizeof(EnsCand) * ns));
-    GTD_CUDA(cudaMalloc(&e->info, sizeof(EnsInfo) * ns));
-    GTD_CUDA(cudaMalloc(&e->arrived, sizeof(int) * ns));
-    cudaStream_t st = e->stream;
-    GTD_CUDA(cudaMemsetAsync(e->cand, 0, sizeof(EnsCand) * ns, st));
-    GTD_CUDA(cudaMemsetAsync(e->arrived, 0, sizeof(int) * ns, st));
-    GTD_CUDA(cudaMemcpyAsync(e->off, offsets, sizeof(int64_t) * (size_t)(n_systems + 1), cudaMemcpyHostToDevice, st));
-    if (n_systems) {
-        GTD_CUDA(cudaMemcpyAsync(e->cnt, cnt.data(), sizeof(int32_t) * cnt.size(), cudaMemcpyHostToDevice, st));
-        GTD_CUDA(cudaMemcpyAsync(e->order, order.data(), sizeof(int32_t) * order.size(), cudaMemcpyHostToDevice, st));
+    if (rc) {  // what was there is gone: no systems
+        cudaStreamSynchronize(e->stream);
+        ens_release(e);
+        e->n_sys = e->n_bodies = 0;
     }
-    if (nb) {
-        GTD_CUDA(cudaMalloc(&e->io, 12 * sizeof(double) * (size_t)nb));
-        int rc = copy_to_device(e->host_ring, e->device, e->stream, ens_spans(e, m, r, rest, x3, v3, nullptr));
-        if (rc) return rc;
-        ens_pack_kernel<<<(unsigned)n_systems, 256, 0, e->stream>>>(e->off, nb, e->io, v3 != nullptr, r != nullptr,
-                                                                    rest != nullptr, e->pos, e->vel, e->acc, e->rad,
-                                                                    e->rest, e->ids);
-        GTD_CHECK_LAUNCH();
-        if (first > 0) {
-            GTD_CUDA(cudaMemsetAsync(e->pos, 0, sizeof(double4) * (size_t)first, st));
-            GTD_CUDA(cudaMemsetAsync(e->vel, 0, sizeof(double4) * (size_t)first, st));
-            GTD_CUDA(cudaMemsetAsync(e->acc, 0, sizeof(double4) * (size_t)first, st));
-            GTD_CUDA(cudaMemsetAsync(e->rad, 0, sizeof(double) * (size_t)first, st));
-            GTD_CUDA(cudaMemsetAsync(e->rest, 0, sizeof(double) * (size_t)first, st));
-        }
-    }
-    GTD_CUDA(cudaMemsetAsync(e->merged, 0, sizeof(unsigned), st));
-    GTD_CUDA(cudaStreamSynchronize(st));
-    e->begun = false;
-    if (!e->configured) ens_default(e);
-    return GTD_OK;
+    return rc;
 }
 
 int gtd_ensemble_evolve(gtd_ensemble *e, uint64_t steps, int64_t *elapsed_ns) {
@@ -968,7 +918,7 @@ int gtd_ensemble_counts(gtd_ensemble *e, int64_t *counts, uint64_t *merges, uint
     }
     if (merges) {
         unsigned w = 0;
-        GTD_CUDA(cudaMemcpy(&w, e->merged, sizeof w, cudaMemcpyDeviceToHost));
+        if (e->merged) GTD_CUDA(cudaMemcpy(&w, e->merged, sizeof w, cudaMemcpyDeviceToHost));
         *merges = w;
     }
     if (launches) *launches = e->launches;
@@ -1109,3 +1059,75 @@ int gtd_ensemble_autotune(gtd_ensemble *e, int *best_threads, double *best_ms) {
 }
 
 }  // extern "C"
+
+// The systems of an empty handle; after an error some of its buffers may be there.
+static int ens_upload(gtd_ensemble *e, int64_t n_systems, const int64_t *offsets, const double *m, const double *r,
+                      const double *rest, const double *x3, const double *v3) {
+    e->n_sys = n_systems;
+    const int64_t none = 0;
+    if (!n_systems) offsets = &none;
+    e->off_h.assign(offsets, offsets + n_systems + 1);
+    const int64_t nb = offsets[n_systems];
+    e->n_bodies = nb;
+    e->max_n = 0;
+    std::vector<int32_t> cnt((size_t)n_systems);
+    std::vector<int32_t> &order = e->order_h;
+    order.assign((size_t)n_systems, 0);
+    for (int64_t s = 0; s < n_systems; ++s) {
+        const int64_t k = offsets[s + 1] - offsets[s];
+        if (k < 0 || offsets[s] < 0) return fail(GTD_ERR_INVALID_ARGUMENT, "offsets must be non-decreasing from 0");
+        if (k > kEnsMaxN) return fail(GTD_ERR_CAPACITY, "system %lld has %lld bodies; the ensemble kernel holds %d",
+                                      (long long)s, (long long)k, kEnsMaxN);
+        cnt[(size_t)s] = (int32_t)k;
+        e->max_n = std::max(e->max_n, (int)k);
+    }
+    std::iota(order.begin(), order.end(), 0);
+    std::stable_sort(order.begin(), order.end(), [&](int32_t a, int32_t b) { return cnt[a] > cnt[b]; });
+    const int64_t first = offsets[0];  // rows before it belong to no system and read as zero
+    for (int64_t i = first; i < nb; ++i)
+        if (m[i] < 0) return fail(GTD_ERR_INVALID_ARGUMENT, "negative mass at body %lld", (long long)i);
+    const size_t b4 = sizeof(double4) * (size_t)std::max<int64_t>(nb, 1);
+    GTD_CUDA(cudaMalloc(&e->off, sizeof(int64_t) * (size_t)(n_systems + 1)));
+    GTD_CUDA(cudaMalloc(&e->cnt, sizeof(int32_t) * (size_t)std::max<int64_t>(n_systems, 1)));
+    GTD_CUDA(cudaMalloc(&e->order, sizeof(int32_t) * (size_t)std::max<int64_t>(n_systems, 1)));
+    GTD_CUDA(cudaMalloc(&e->pos, b4));
+    GTD_CUDA(cudaMalloc(&e->vel, b4));
+    GTD_CUDA(cudaMalloc(&e->acc, b4));
+    GTD_CUDA(cudaMalloc(&e->rad, sizeof(double) * (size_t)std::max<int64_t>(nb, 1)));
+    GTD_CUDA(cudaMalloc(&e->rest, sizeof(double) * (size_t)std::max<int64_t>(nb, 1)));
+    GTD_CUDA(cudaMalloc(&e->ids, sizeof(int32_t) * (size_t)std::max<int64_t>(nb, 1)));
+    GTD_CUDA(cudaMalloc(&e->merged, sizeof(unsigned)));
+    const size_t ns = (size_t)std::max<int64_t>(n_systems, 1);
+    GTD_CUDA(cudaMalloc(&e->cand, sizeof(EnsCand) * ns));
+    GTD_CUDA(cudaMalloc(&e->info, sizeof(EnsInfo) * ns));
+    GTD_CUDA(cudaMalloc(&e->arrived, sizeof(int) * ns));
+    cudaStream_t st = e->stream;
+    GTD_CUDA(cudaMemsetAsync(e->cand, 0, sizeof(EnsCand) * ns, st));
+    GTD_CUDA(cudaMemsetAsync(e->arrived, 0, sizeof(int) * ns, st));
+    GTD_CUDA(cudaMemcpyAsync(e->off, offsets, sizeof(int64_t) * (size_t)(n_systems + 1), cudaMemcpyHostToDevice, st));
+    if (n_systems) {
+        GTD_CUDA(cudaMemcpyAsync(e->cnt, cnt.data(), sizeof(int32_t) * cnt.size(), cudaMemcpyHostToDevice, st));
+        GTD_CUDA(cudaMemcpyAsync(e->order, order.data(), sizeof(int32_t) * order.size(), cudaMemcpyHostToDevice, st));
+    }
+    if (nb) {
+        GTD_CUDA(cudaMalloc(&e->io, 12 * sizeof(double) * (size_t)nb));
+        int rc = copy_to_device(e->host_ring, e->device, e->stream, ens_spans(e, m, r, rest, x3, v3, nullptr));
+        if (rc) return rc;
+        ens_pack_kernel<<<(unsigned)n_systems, 256, 0, e->stream>>>(e->off, nb, e->io, v3 != nullptr, r != nullptr,
+                                                                    rest != nullptr, e->pos, e->vel, e->acc, e->rad,
+                                                                    e->rest, e->ids);
+        GTD_CHECK_LAUNCH();
+        if (first > 0) {
+            GTD_CUDA(cudaMemsetAsync(e->pos, 0, sizeof(double4) * (size_t)first, st));
+            GTD_CUDA(cudaMemsetAsync(e->vel, 0, sizeof(double4) * (size_t)first, st));
+            GTD_CUDA(cudaMemsetAsync(e->acc, 0, sizeof(double4) * (size_t)first, st));
+            GTD_CUDA(cudaMemsetAsync(e->rad, 0, sizeof(double) * (size_t)first, st));
+            GTD_CUDA(cudaMemsetAsync(e->rest, 0, sizeof(double) * (size_t)first, st));
+        }
+    }
+    GTD_CUDA(cudaMemsetAsync(e->merged, 0, sizeof(unsigned), st));
+    GTD_CUDA(cudaStreamSynchronize(st));
+    e->begun = false;
+    if (!e->configured) ens_default(e);
+    return GTD_OK;
+}
