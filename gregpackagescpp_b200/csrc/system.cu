@@ -33,6 +33,7 @@ int fail(int code, const char *fmt, ...) {
 
 int cuda_fail(cudaError_t e, const char *what, const char *file, int line) {
     set_error("CUDA error %s (%s) in %s at %s:%d", cudaGetErrorName(e), cudaGetErrorString(e), what, file, line);
+    cudaGetLastError();  // reported here: the next launch check is about the next launch
     return e == cudaErrorMemoryAllocation ? GTD_ERR_OUT_OF_MEMORY : GTD_ERR_CUDA;
 }
 
@@ -48,16 +49,21 @@ using namespace gtd;
 static int ensure_capacity(gtd_system *s, int64_t n) {
     if (n <= s->cap) return GTD_OK;
     release_bodies(s);
+    s->n = s->n_uploaded = 0;  // until the caller has put bodies there
     const size_t b4 = sizeof(double4) * (size_t)n;
-    GTD_CUDA(cudaMalloc(&s->pm[0], b4));
-    GTD_CUDA(cudaMalloc(&s->pm[1], b4));
-    GTD_CUDA(cudaMalloc(&s->vel, b4));
-    GTD_CUDA(cudaMalloc(&s->acc, b4));
-    GTD_CUDA(cudaMalloc(&s->rad, sizeof(double) * (size_t)n));
-    GTD_CUDA(cudaMalloc(&s->rest, sizeof(double) * (size_t)n));
-    GTD_CUDA(cudaMalloc(&s->ids, sizeof(int32_t) * (size_t)n));
-    s->cap = n;
-    return GTD_OK;
+    const int rc = [&]() -> int {
+        GTD_CUDA(cudaMalloc(&s->pm[0], b4));
+        GTD_CUDA(cudaMalloc(&s->pm[1], b4));
+        GTD_CUDA(cudaMalloc(&s->vel, b4));
+        GTD_CUDA(cudaMalloc(&s->acc, b4));
+        GTD_CUDA(cudaMalloc(&s->rad, sizeof(double) * (size_t)n));
+        GTD_CUDA(cudaMalloc(&s->rest, sizeof(double) * (size_t)n));
+        GTD_CUDA(cudaMalloc(&s->ids, sizeof(int32_t) * (size_t)n));
+        return GTD_OK;
+    }();
+    if (rc) release_bodies(s);
+    else s->cap = n;
+    return rc;
 }
 
 // Pinned host scratch of at least `bytes`.
