@@ -1448,11 +1448,9 @@ int reorder_bodies(gtd_system *s) {
     int rc = hilbert_sort(s);
     if (rc) return rc;
     cudaStream_t st = s->stream;
-    if (!s->sc4) {
-        GTD_CUDA(cudaMalloc(&s->sc4, sizeof(double4) * (size_t)s->cap));
-        GTD_CUDA(cudaMalloc(&s->sc1, sizeof(double) * (size_t)s->cap));
-        GTD_CUDA(cudaMalloc(&s->sci, sizeof(int32_t) * (size_t)s->cap));
-    }
+    if (!s->sc4) GTD_CUDA(cudaMalloc(&s->sc4, sizeof(double4) * (size_t)s->cap));
+    if (!s->sc1) GTD_CUDA(cudaMalloc(&s->sc1, sizeof(double) * (size_t)s->cap));
+    if (!s->sci) GTD_CUDA(cudaMalloc(&s->sci, sizeof(int32_t) * (size_t)s->cap));
     const unsigned g = blocks_for(n);
     gather_kernel<double4><<<g, kTT, 0, st>>>(n, s->perm, s->pm[s->cur], s->pm[s->cur ^ 1]);
     s->cur ^= 1;

@@ -165,9 +165,8 @@ int ensure_plan(gtd_system *s) {
 }
 
 static int ensure_pred(gtd_system *s) {
-    if (s->pred_pos) return GTD_OK;
-    GTD_CUDA(cudaMalloc(&s->pred_pos, sizeof(double4) * (size_t)s->cap));
-    GTD_CUDA(cudaMalloc(&s->pred_vel, sizeof(double4) * (size_t)s->cap));
+    if (!s->pred_pos) GTD_CUDA(cudaMalloc(&s->pred_pos, sizeof(double4) * (size_t)s->cap));
+    if (!s->pred_vel) GTD_CUDA(cudaMalloc(&s->pred_vel, sizeof(double4) * (size_t)s->cap));
     return GTD_OK;
 }
 
@@ -743,6 +742,7 @@ int gtd_system_energy(gtd_system *s, double *ke, double *pe, double *p3, double 
         if (need > s->escratch_n) {
             cudaFree(s->escratch);
             s->escratch = nullptr;
+            s->escratch_n = 0;
             GTD_CUDA(cudaMalloc(&s->escratch, sizeof(double) * (size_t)need));
             s->escratch_n = need;
         }
