@@ -13,10 +13,11 @@ namespace gtd {
 constexpr size_t kSlotBytes = (size_t)512 << 10;
 constexpr int kSlots = kRingThreads * kRingSlotsEach;
 constexpr size_t kRingFrom = (size_t)4 << 20;  // smaller copies: starting the threads costs what they save
-// Making the ring takes 4 to 7 ms, and its threads save 0.05 ms a MB of arrays in use and 0.14 of fresh ones
-// (two GPU hosts): what it costs comes back after 50 to 140 MB.  A handle's ring is made once the large
-// copies of its life, this one included, come to about that.
-constexpr size_t kRingPays = (size_t)64 << 20;
+// Making the ring takes 4 to 7 ms; its threads save 0.05 ms a MB of arrays in use and 0.14 of fresh ones, 0.1
+// over an upload and a download.  So it pays after 40 to 70 MB, and a handle's ring is made once the large
+// copies of its life, this one included, come to the lower end of that: two calls of 262144 bodies, host
+// arrays in and out, run at 3.03e12 pair-interactions/s with it and at 2.7 to 3.0e12 with 64 MiB.
+constexpr size_t kRingPays = (size_t)40 << 20;
 
 void release_host_ring(HostRing &ring) {
     for (cudaEvent_t &e : ring.events) {
