@@ -340,7 +340,9 @@ __device__ __forceinline__ float ens_min3(float a, float b, float c) {
 
 // One fold (j pairs q0 .. q1-1) of the force loop for IB rows, with the smallest r2 to another body.  kOwn:
 // the fold holds one of the rows' own bodies, whose j pair oq[b] stays out of the minimum (its other body is
-// in it from the start).
+// in it from the start).  Leaving out a vanishing r2 instead leaves out coincident bodies too; us a step so and
+// by number: 4096 systems of up to 64 bodies 52.4 / 52.9, 256 123.5 / 125.2, 512 of 2048 604 / 612, 64 of 8192
+// 1551 / 1492.
 template <int IB, bool kOwn>
 __device__ __forceinline__ void ens_fold(int q0, int q1, const float2 *X2, const float2 *Y2, const float2 *Z2,
                                          const float2 *M2, const float2 (&nx)[IB], const float2 (&ny)[IB],
